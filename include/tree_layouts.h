@@ -265,17 +265,17 @@ int tl_batch_query(const tl_batch_plan *plan, const void *dev_keys, const void *
                    const uint32_t *dev_inst, uint64_t q, uint64_t *dev_answers, void *dev_workspace,
                    uint64_t workspace_bytes, void *stream, float *ms);
 /* Tuning per size class c = floor(log2 n_j), 48 entries each: keys per stream
- * tile (a power of two, 256 .. 96 KB / key_bytes), top levels pinned in shared
- * memory by the query; plus the query work
- * item and the permute block size (256 or 512); 0 / NULL keeps a value.
- * Changing tile sizes rebuilds the plan from dev_offsets. */
+ * tile (a power of two, 256 .. 96 KB / key_bytes); plus the permute block size
+ * (256 or 512); 0 / NULL keeps a value.  pin_levels and query_chunk are kept and
+ * read back, but the queries have nothing to tune.  Changing tile sizes rebuilds
+ * the plan from dev_offsets. */
 int tl_batch_set_tuning(tl_batch_plan *plan, const uint32_t *tile_keys, const uint32_t *pin_levels,
                         uint32_t query_chunk, uint32_t threads, const int64_t *dev_offsets, void *stream);
 int tl_batch_get_tuning(const tl_batch_plan *plan, uint32_t *tile_keys, uint32_t *pin_levels,
                         uint32_t *query_chunk, uint32_t *threads);
-/* Measures and keeps the best tuning (coordinate descent over the block size,
- * per-class tile sizes, the query work item and per-class pinned levels) on the
- * caller's data; dev_keys must hold the sorted instances and is left sorted.
+/* Measures and keeps the best tuning (coordinate descent over the block size and
+ * the per-class tile sizes) on the caller's data; dev_keys must hold the sorted
+ * instances and is left sorted.
  * report (optional) receives a JSON summary. */
 int tl_batch_autotune(tl_batch_plan *plan, const int64_t *dev_offsets, void *dev_keys, const void *dev_queries,
                       const uint32_t *dev_inst, uint64_t q, void *stream, char *report, uint64_t report_len);

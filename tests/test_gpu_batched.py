@@ -186,3 +186,49 @@ def test_batched_default_orders_only_where_it_pays():
     assert plan.ordered()[0] <= forced.ordered()[0]
     plan.permute(keys)
     assert np.array_equal(keys.cpu().numpy().view(np.uint64), ref)
+
+
+@pytest.mark.parametrize("b", [1, 3, 4, 8, 16, 32, 40])
+@pytest.mark.parametrize("kb", [8, 4])
+@pytest.mark.parametrize("num,lo,hi,q,skip", [
+    (5, 0, 6, 1, 0), (40, 2, 12, 1000, 1), (1500, 1, 9, 4097, 3),  # as given; more instances than sort bins
+    (300, 3, 13, (1 << 19) - 1, 2), (300, 3, 13, 1 << 19, 1),        # either side of the sorted form's line
+    (1500, 1, 9, (1 << 19) + 12345, 3),
+])
+def test_batched_queries_over_unaligned_instances(b, kb, num, lo, hi, q, skip):
+    """Exact against a search of the sorted instances: a hit names a position
+    that holds the key, a miss is a key its instance does not hold.  The key
+    array starts `skip` keys into its allocation, so nodes cross 32-byte sectors
+    everywhere and the array's ends do not fall on one; some instance ids are out
+    of range (answer 0)."""
+    import torch
+    dt = torch.int64 if kb == 8 else torch.int32
+    keys, off, sizes = _batch(num, lo, hi, b + num, extra=[0, 1, b, b + 1])
+    n_inst = len(sizes)
+    buf = torch.empty(keys.numel() + skip, dtype=dt, device="cuda")
+    lay = buf[skip:]
+    lay.copy_(keys.to(dt))
+    sizes_t = torch.from_numpy(sizes).cuda()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(q)
+    inst = torch.randint(0, n_inst + 2, (q,), generator=g, device="cuda", dtype=torch.int64)
+    ok = inst < n_inst
+    j = inst.clamp_max(n_inst - 1)
+    n_j, o_j = sizes_t[j], off[j]
+    pos = o_j + (torch.rand(q, generator=g, device="cuda", dtype=torch.float64) * n_j).long().clamp_max_(1 << 40)
+    pos = torch.minimum(pos, (o_j + n_j - 1).clamp_min(0))
+    Q = keys[pos] + torch.randint(0, 3, (q,), generator=g, device="cuda")  # hits, near misses, past the last key
+    plan = TB.BatchPlan(off, b=b, key_bytes=kb)
+    plan.permute(lay)
+    ans = torch.full((q,), -7, dtype=torch.int64, device="cuda")
+    plan.query(lay, Q.to(dt), inst.to(torch.int32), ans)
+    assert bool((ans[~ok] == 0).all())
+    hit = ok & (ans < n_j)
+    assert bool((ans[ok & ~hit] == n_j[ok & ~hit]).all())
+    assert bool((lay[(o_j + ans)[hit]].to(torch.int64) == Q[hit]).all())
+    # present keys, instance by instance in the sorted order: composite (instance, key)
+    comp = torch.repeat_interleave(torch.arange(n_inst, device="cuda"), sizes_t) * (1 << 40) + keys
+    want = j * (1 << 40) + Q
+    at = torch.searchsorted(comp, want).clamp_max(max(comp.numel() - 1, 0))
+    present = ok & (comp[at] == want)
+    assert bool((present == hit).all())

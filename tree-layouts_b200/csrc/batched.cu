@@ -73,14 +73,21 @@ struct BatchTotals {
     uint64_t tiles, chunks, scratch, max_tile;
 };
 
+// What a query needs of its instance, in one 32-byte load: its first key, its
+// keys, and the last node index (plus one) that can have children.
+struct alignas(32) BatchGeo {
+    uint64_t off, n, cmax, pad;
+};
+
 struct tl_batch_plan_impl {
     uint32_t num = 0, key_bytes = 8;
     uint64_t b = 8;
     BatchInst *inst = nullptr;   // device
+    BatchGeo *geo = nullptr;     // device: per instance, for the queries
     BatchTotals tot{};
     uint32_t tile_keys[kMaxClass];
-    uint32_t pin_levels[kMaxClass];  // query: top levels pinned in shared memory per size class
-    uint32_t query_chunk = 2048;     // queries per CTA work item
+    uint32_t pin_levels[kMaxClass];  // kept for tl_batch_get_tuning; the queries do not use it
+    uint32_t query_chunk = 2048;     // likewise
     uint32_t threads = 256;          // permute kernel block size
     uint32_t *owner = nullptr;   // device: owner instance of every tile ticket, then of every copy chunk
     uint32_t *tile = nullptr;    // device: the tile of its owner every tile ticket processes
@@ -91,6 +98,7 @@ struct tl_batch_plan_impl {
     uint64_t ordered_keys = 0;   // their keys
     uint64_t off_flags = 0, off_done = 0, off_ctrl = 0, ws_bytes = 0;
     uint64_t total_keys = 0;
+    uint64_t max_n = 0;          // keys of the largest instance
 };
 
 // ---------------------------------------------------------------- setup
@@ -98,7 +106,8 @@ __global__ void __launch_bounds__(256) batch_setup_kernel(const int64_t *__restr
                                                           uint32_t key_bytes, FastDiv64 fd, FastDiv32 fd32,
                                                           FastDiv32 fd32b, const __grid_constant__ PowDivs pdivs,
                                                           const uint32_t *__restrict__ tile_keys,
-                                                          BatchInst *__restrict__ inst, BatchTotals *__restrict__ tot) {
+                                                          BatchInst *__restrict__ inst, BatchGeo *__restrict__ geo,
+                                                          BatchTotals *__restrict__ tot) {
     // one block: per-instance plans, then exclusive scans in instance order
     __shared__ unsigned long long s_part[3][1024];
     const uint32_t T = blockDim.x;
@@ -135,6 +144,7 @@ __global__ void __launch_bounds__(256) batch_setup_kernel(const int64_t *__restr
         ss += I.S.nscratch ? I.S.nscratch + vec - 1 : 0;  // room to align the base
         sc += I.nchunks;
         inst[j] = I;
+        geo[j] = BatchGeo{I.off, n, (n + 1) / (b + 1), 0};
     }
     s_part[0][threadIdx.x] = st;
     s_part[1][threadIdx.x] = ss;
@@ -338,148 +348,186 @@ batch_permute_kernel(K *__restrict__ keys, K *__restrict__ scr, const BatchInst 
 }
 
 // ---------------------------------------------------------------- queries
-// Queries are grouped by instance (counting sort: histogram, scan, scatter) so
-// that a CTA's work item mostly belongs to one instance; the CTA then pins that
-// instance's top levels in shared memory (depth from the size-class table).
-__global__ void batch_hist_kernel(const uint32_t *__restrict__ qinst, uint64_t q, uint32_t num,
-                                  unsigned int *__restrict__ count) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < q; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t j = qinst[i];
-        if (j < num) atomicAdd(&count[j], 1u);
-    }
-}
+// A query descends its own instance; nothing but the answer is written.  G
+// lanes read a node together: the aligned 32-byte sectors that hold it
+// (instances start anywhere, so a node of B * w bytes spans up to
+// B * w / 32 + 1 of them), lane g the sectors g, g + G, ...  Nodes start at
+// multiples of B keys, so which keys of a lane's sectors belong to the node is
+// the same mask at every level.  As in the single-array query the warp's
+// control flow is uniform, the count is a shuffle sum and an equal key is found
+// by ballot.
+//
+// What bounds it is where the descents go, not how many bytes they read: the
+// instances' upper levels lie all over the key array, so a batch as given
+// touches every 2 MB page of it at every level (measured on B200, 2^24 queries
+// over 1024 arrays of 5.2e8 u64 keys, b = 8: 2.36 ms at a quarter of the DRAM
+// and of the L1 bandwidth; over 32 arrays in 126 MB, 0.9 ms).  So a block
+// takes a chunk of the batch, orders it by instance in shared memory (a
+// counting sort of 16-bit offsets into kBatchBins bins of consecutive
+// instances) and walks the chunk in that order, all blocks through the same
+// instances at about the same time; the answers go to the chunk's own stretch.
+// Same measurement: chunks of 4096 / 8192 / 16384 / 32768 queries 1.77 / 1.16 /
+// 1.14 / 1.25 ms; the previous form (a global counting sort by two atomics a
+// query, then a thread a query over the sorted copy) 4.50 ms.  In this order a
+// thread a query (G = 1) beats groups of lanes (1.14 against 1.54 ms with G =
+// 2, 2.28 with G = 4; b = 16 1.46 against 1.57): more descents in flight, and
+// L1 serves the shared upper nodes.  One block of 1024 threads an SM: 512 x 2
+// 1.24, 256 x 4 1.41 ms (each block has its own window of instances).
+constexpr uint32_t kBatchBins = 1024;
+constexpr int kBatchSortThreads = 1024;
+constexpr uint32_t kBatchSortChunk = 16384;
 
-__global__ void batch_scan_kernel(const unsigned int *__restrict__ count, uint32_t num,
-                                  unsigned long long *__restrict__ start) {
-    __shared__ unsigned long long s_part[1024];
-    const uint32_t T = blockDim.x, per = (num + T - 1) / T;
-    const uint32_t j0 = threadIdx.x * per, j1 = min(num, j0 + per);
-    unsigned long long acc = 0;
-    for (uint32_t j = j0; j < j1; ++j) acc += count[j];
-    s_part[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long a = 0;
-        for (uint32_t t = 0; t < T; ++t) {
-            const unsigned long long x = s_part[t];
-            s_part[t] = a;
-            a += x;
-        }
-        start[num] = a;
+// NB = node bytes (a multiple of 32), or 0 for any b: then the sectors are
+// taken G at a time, their masks computed on the way.  I: an index type that
+// holds every child index of a batch's instances.
+template <typename K, int NB, int G, typename I>
+__device__ __forceinline__ void batch_descend(const K *__restrict__ keys, uint64_t total,
+                                              const BatchGeo *__restrict__ geo, uint32_t num, uint32_t b_rt,
+                                              const K *__restrict__ Q, const uint32_t *__restrict__ qinst,
+                                              uint64_t qi, bool have, uint64_t *__restrict__ ans) {
+    constexpr int KPL = 32 / sizeof(K);                     // keys per sector
+    constexpr int NI = NB ? (NB / 32 + 1 + G - 1) / G : 1;  // sectors per lane
+    const int B = NB ? NB / (int)sizeof(K) : (int)b_rt;
+    const uint32_t lane = threadIdx.x & 31, g = lane % G, gshift = lane - g;
+    const uint32_t j = have ? __ldg(qinst + qi) : num;
+    const K q = have ? __ldg(Q + qi) : K(0);
+    uint64_t rec[4] = {0, 0, 0, 0};  // BatchGeo; an instance id out of range answers 0
+    if (j < num) ldg32(reinterpret_cast<const uint64_t *>(geo + j), rec);
+    const K *A = keys + rec[0];
+    const I n = (I)rec[1], cmax = (I)rec[2];
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(A) & 31) / sizeof(K);
+    const K *A32 = A - off;  // the sector of the instance's first key
+    // an instance whose first or last sector reaches outside the key array is read key by key
+    const bool edge = A32 < keys || A32 + ((uint64_t)n + off + KPL - 1) / KPL * KPL > keys + total;
+    // slots rel .. rel + KPL - 1 against [0, valid)
+    auto mask = [](int rel, int valid) -> uint32_t {
+        return rel >= valid ? 0u : ((1u << KPL) - 1) & (rel < 0 ? ~0u << -rel : ~0u) &
+                                       (valid - rel < KPL ? (1u << (valid - rel)) - 1 : ~0u);
+    };
+    uint32_t vm[NI];
+    if constexpr (NB != 0) {
+#pragma unroll
+        for (int t = 0; t < NI; ++t) vm[t] = mask((int)(g + t * G) * KPL - (int)off, B);
     }
-    __syncthreads();
-    unsigned long long p = s_part[threadIdx.x];
-    for (uint32_t j = j0; j < j1; ++j) {
-        start[j] = p;
-        p += count[j];
-    }
-}
-
-template <typename K>
-__global__ void batch_bucket_kernel(const K *__restrict__ Q, const uint32_t *__restrict__ qinst, uint64_t q,
-                                    uint32_t num, unsigned long long *__restrict__ cursor, K *__restrict__ sq,
-                                    uint32_t *__restrict__ sinst, uint64_t *__restrict__ sidx) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < q; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t j = qinst[i];
-        if (j >= num) continue;
-        const unsigned long long p = atomicAdd(&cursor[j], 1ull);
-        sq[p] = Q[i];
-        sinst[p] = j;
-        sidx[p] = i;
-    }
-}
-
-template <typename K>
-__global__ void __launch_bounds__(kBatchThreads)
-batch_query_kernel(const K *__restrict__ keys, const BatchInst *__restrict__ inst, const K *__restrict__ sq,
-                   const uint32_t *__restrict__ sinst, const uint64_t *__restrict__ sidx,
-                   const unsigned long long *__restrict__ nvalid, uint32_t chunk,
-                   const uint32_t *__restrict__ pin_levels, uint32_t pin_cap, uint64_t *__restrict__ ans) {
-    const uint64_t q = *nvalid;  // queries with a valid instance id (sorted first)
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    K *sm = reinterpret_cast<K *>(smem_raw);
-    __shared__ uint32_t s_j, s_one;
-    __shared__ uint64_t s_P;
-    const uint64_t nchunks = (q + chunk - 1) / chunk;
-    for (uint64_t ck = blockIdx.x; ck < nchunks; ck += gridDim.x) {
-        const uint64_t q0 = ck * chunk, q1 = min(q, q0 + chunk);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            s_j = sinst[q0];
-            s_one = sinst[q1 - 1] == s_j;
-            uint64_t P = 0;
-            if (s_one) {
-                const BtreeStream &S = inst[s_j].S;
-                const uint32_t cls = S.g.n ? bit_length(S.g.n) - 1 : 0;
-                const uint32_t L = pin_levels[cls < kMaxClass ? cls : kMaxClass - 1];
-                const uint32_t LL = L < S.g.h + 1 ? L : S.g.h + 1;
-                P = L ? min(S.g.n, S.g.pw[LL] - 1) : 0;
-                if (P > pin_cap) P = 0;
+    I i = 0, res = n;
+    bool live = n > 0;
+    while (__any_sync(0xFFFFFFFFu, live)) {
+        uint32_t lt = 0, eqm = 0;
+        if (live) {
+            const bool part = n - i < (I)B;  // slots at or past n do not count
+            const int valid = part ? (int)(n - i) : B;
+            uint32_t first = off;  // a node of an odd size starts anywhere in its sector
+            const K *p = A32 + i;
+            if constexpr (NB == 0) {
+                first = (uint32_t)((off + i) % KPL);
+                p = A + i - first;
             }
-            s_P = P;
-        }
-        __syncthreads();
-        const uint64_t P = s_P;
-        if (P) {
-            const K *A = keys + inst[s_j].off;
-            for (uint64_t x = threadIdx.x; x < P; x += blockDim.x) sm[x] = __ldg(A + x);
-            __syncthreads();
-        }
-        for (uint64_t i = q0 + threadIdx.x; i < q1; i += blockDim.x) {
-            const uint32_t j = sinst[i];
-            const BtreeStream &S = inst[j].S;
-            const K *A = keys + inst[j].off;
-            const uint64_t n = S.g.n, b = S.g.b;
-            const uint64_t PP = (s_one && j == s_j) ? P : 0;
-            const K qv = sq[i];
-            uint64_t node = 0, res = n;
-            const uint64_t cmax = (n + 1) / (b + 1);
-            // node rows in 32-byte (or 16-byte) loads where the instance's keys
-            // and its nodes start on such a boundary, else key by key
-            const uintptr_t abase = reinterpret_cast<uintptr_t>(A);
-            const uint32_t vb = (abase & 31) == 0 && (b * sizeof(K)) % 32 == 0   ? 32u
-                                : (abase & 15) == 0 && (b * sizeof(K)) % 16 == 0 ? 16u
-                                                                                  : 0u;
-            while (node < n) {
-                const uint64_t valid = min(b, n - node);
-                uint32_t lt = 0;
-                bool eq = false;
-                if (vb && valid == b && node >= PP) {
-                    const uint32_t kpl = vb / sizeof(K), nl = (uint32_t)(b / kpl);
-#pragma unroll 4
-                    for (uint32_t j = 0; j < nl; ++j) {
-                        K v[32 / sizeof(K)];
-                        if (vb == 32) {
-                            ldg32(A + node + (uint64_t)j * kpl, v);
+            for (int s0 = (int)g; NB ? s0 == (int)g : s0 * KPL - (int)first < valid; s0 += G) {
+                K v[NI][KPL];
+                uint32_t m[NI];
+#pragma unroll
+                for (int t = 0; t < NI; ++t) {
+                    const int s = s0 + t * G;
+                    if constexpr (NB == 0)
+                        m[t] = mask(s * KPL - (int)first, valid);
+                    else
+                        m[t] = part ? vm[t] & mask(s * KPL - (int)first, valid) : vm[t];
+                    if (m[t]) {
+                        if (!edge) {
+                            ldg32(p + s * KPL, v[t]);
                         } else {
-                            const uint4 x = __ldg(reinterpret_cast<const uint4 *>(A + node + (uint64_t)j * kpl));
-                            const K *kx = reinterpret_cast<const K *>(&x);
 #pragma unroll
-                            for (int e = 0; e < (int)(16 / sizeof(K)); ++e) v[e] = kx[e];
+                            for (int e = 0; e < KPL; ++e)
+                                v[t][e] = (m[t] >> e) & 1u ? __ldg(p + s * KPL + e) : K(0);
                         }
+                    }
+                }
 #pragma unroll
-                        for (int e = 0; e < (int)(32 / sizeof(K)); ++e)
-                            if (vb == 32 || e < (int)(16 / sizeof(K))) {
-                                lt += v[e] < qv;
-                                eq |= v[e] == qv;
-                            }
+                for (int t = 0; t < NI; ++t) {
+                    uint32_t l = 0, x = 0;
+#pragma unroll
+                    for (int e = 0; e < KPL; ++e) {
+                        l |= (v[t][e] < q ? 1u : 0u) << e;
+                        x |= (v[t][e] == q ? 1u : 0u) << e;
                     }
-                } else {
-                    for (uint64_t s = 0; s < valid; ++s) {
-                        const uint64_t p = node + s;
-                        const K cur = p < PP ? sm[p] : __ldg(A + p);
-                        lt += cur < qv;
-                        eq |= cur == qv;
-                    }
+                    lt += __popc(l & m[t]);
+                    eqm |= x & m[t];
                 }
-                if (eq) {  // keys are unique: the equal key sits at slot lt
-                    res = node + lt;
-                    break;
-                }
-                if (node + 1 > cmax) break;
-                node = (node + 1) * (b + 1) + (uint64_t)lt * b - 1;
             }
-            ans[sidx[i]] = res;
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) lt += __shfl_xor_sync(0xFFFFFFFFu, lt, o);
+        bool hit = eqm != 0;
+        if constexpr (G > 1) hit = ((__ballot_sync(0xFFFFFFFFu, hit) >> gshift) & ((1u << G) - 1)) != 0;
+        if (live) {
+            if (hit) {  // keys are unique: the equal key sits at slot lt
+                res = i + lt;
+                live = false;
+            } else if (i + 1 > cmax) {  // every child starts past n
+                live = false;
+            } else {
+                i = (i + 1) * (I)(B + 1) + (I)lt * (I)B - 1;
+                live = i < n;
+            }
+        }
+    }
+    if (g == 0 && have) ans[qi] = (uint64_t)res;
+}
+
+// The batch as given, a grid stride (small batches: one launch, no sort).
+template <typename K, int NB, int G, typename I>
+__global__ void __launch_bounds__(kBatchThreads)
+batch_query_kernel(const K *__restrict__ keys, uint64_t total, const BatchGeo *__restrict__ geo, uint32_t num,
+                   uint32_t b, const K *__restrict__ Q, const uint32_t *__restrict__ qinst, uint64_t nq,
+                   uint64_t *__restrict__ ans) {
+    const uint64_t step = (uint64_t)gridDim.x * (blockDim.x / G);
+    const uint64_t first = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * (32 / G);  // the warp's
+    for (uint64_t base = first; base < nq; base += step) {
+        const uint64_t qi = base + (threadIdx.x & 31) / G;
+        batch_descend<K, NB, G, I>(keys, total, geo, num, b, Q, qinst, qi, qi < nq, ans);
+    }
+}
+
+// Chunk by chunk, each in the order of its queries' instances.
+template <typename K, int NB, int G, typename I>
+__global__ void __launch_bounds__(kBatchSortThreads, 1)
+batch_query_sorted_kernel(const K *__restrict__ keys, uint64_t total, const BatchGeo *__restrict__ geo, uint32_t num,
+                          uint32_t b, uint32_t bin_shift, uint32_t chunk, const K *__restrict__ Q,
+                          const uint32_t *__restrict__ qinst, uint64_t nq, uint64_t *__restrict__ ans) {
+    static_assert(kBatchBins == kBatchSortThreads, "one bin a thread in the scan");
+    static_assert(kBatchSortChunk <= 65536, "16-bit offsets into the chunk");
+    extern __shared__ uint16_t order[];  // [chunk]
+    __shared__ uint32_t cnt[kBatchBins], wsum[32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
+        const uint32_t len = (uint32_t)min((uint64_t)chunk, nq - c0);
+        __syncthreads();
+        cnt[threadIdx.x] = 0;
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t x = threadIdx.x; x < len; x += kBatchSortThreads)
+            atomicAdd(&cnt[min(__ldg(qinst + c0 + x) >> bin_shift, kBatchBins - 1)], 1u);
+        __syncthreads();
+        const uint32_t c = cnt[threadIdx.x];
+        uint32_t inc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= (uint32_t)o) inc += y;
+        }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wsum[lane] : 0u);
+        cnt[threadIdx.x] = before + inc - c;
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t x = threadIdx.x; x < len; x += kBatchSortThreads)
+            order[atomicAdd(&cnt[min(__ldg(qinst + c0 + x) >> bin_shift, kBatchBins - 1)], 1u)] = (uint16_t)x;
+        __syncthreads();
+        for (uint32_t base = warp * (32 / G); base < len; base += kBatchSortThreads / G) {
+            const uint32_t at = base + lane / G;
+            const bool have = at < len;
+            batch_descend<K, NB, G, I>(keys, total, geo, num, b, Q, qinst, c0 + (have ? order[at] : 0u), have, ans);
         }
     }
 }
@@ -728,7 +776,7 @@ static int build_plan(tl_batch_plan_impl &P, const int64_t *dev_offsets, cudaStr
     batch_setup_kernel<<<1, 256, 0, st>>>(dev_offsets, P.num, P.b, P.key_bytes, FastDiv64(P.b + 1),
                                            FastDiv32((uint32_t)(P.b + 1)),
                                            P.b >= 2 ? FastDiv32((uint32_t)P.b) : FastDiv32(), make_pow_divs(P.b), d_tk,
-                                           P.inst, d_tot);
+                                           P.inst, P.geo, d_tot);
     TL_CUDA_TRY(cudaGetLastError());
     int64_t last = 0;
     TL_CUDA_TRY(cudaMemcpyAsync(&P.tot, d_tot, sizeof(BatchTotals), cudaMemcpyDeviceToHost, st));
@@ -738,6 +786,8 @@ static int build_plan(tl_batch_plan_impl &P, const int64_t *dev_offsets, cudaStr
     std::vector<int64_t> off(P.num + 1);
     TL_CUDA_TRY(cudaMemcpyAsync(off.data(), dev_offsets, off.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     TL_CUDA_TRY(cudaStreamSynchronize(st));
+    P.max_n = 0;
+    for (uint32_t j = 0; j < P.num; ++j) P.max_n = std::max(P.max_n, (uint64_t)(off[j + 1] - off[j]));
     int rc = order_instances(P, off, st);
     if (rc) return rc;
     std::vector<uint32_t> own, loc;
@@ -781,13 +831,16 @@ int batch_plan_create(const int64_t *dev_offsets, uint32_t num, uint64_t b, uint
     P->b = b;
     P->key_bytes = key_bytes;
     default_tuning(*P);
-    if (cudaMalloc(reinterpret_cast<void **>(&P->inst), (size_t)num * sizeof(BatchInst)) != cudaSuccess) {
+    if (cudaMalloc(reinterpret_cast<void **>(&P->inst), (size_t)num * sizeof(BatchInst)) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void **>(&P->geo), (size_t)num * sizeof(BatchGeo)) != cudaSuccess) {
+        cudaFree(P->inst);
         delete P;
         return TL_ERROR_OUT_OF_MEMORY;
     }
     int rc = build_plan(*P, dev_offsets, st);
     if (rc) {
         cudaFree(P->inst);
+        cudaFree(P->geo);
         if (P->owner) cudaFree(P->owner);
         if (P->tile) cudaFree(P->tile);
         free_order_buffers(*P);
@@ -802,6 +855,7 @@ int batch_plan_destroy(tl_batch_plan *plan) {
     if (!plan) return TL_ERROR_INVALID_VALUE;
     auto *P = reinterpret_cast<tl_batch_plan_impl *>(plan);
     cudaFree(P->inst);
+    cudaFree(P->geo);
     if (P->owner) cudaFree(P->owner);
     if (P->tile) cudaFree(P->tile);
     free_order_buffers(*P);
@@ -876,52 +930,63 @@ int batch_status(const tl_batch_plan *plan, const void *dev_ws, cudaStream_t st)
     return (err & (1u << TL_ERROR_TIMEOUT)) ? TL_ERROR_TIMEOUT : TL_ERROR_UNSUPPORTED;
 }
 
+// The queries need no memory of their own; callers still pass a workspace.
 int batch_query_workspace_bytes(const tl_batch_plan *plan, uint64_t q, uint64_t *bytes) {
+    (void)q;
     if (!plan || !bytes) return TL_ERROR_INVALID_VALUE;
-    const auto &P = *reinterpret_cast<const tl_batch_plan_impl *>(plan);
-    auto al = [](uint64_t x) { return (x + 255) / 256 * 256; };
-    *bytes = al((uint64_t)P.num * 4) + al(((uint64_t)P.num + 1) * 8) + al(q * P.key_bytes) + al(q * 4) + al(q * 8);
+    *bytes = 256;
+    return TL_SUCCESS;
+}
+
+// Batches of kBatchSortMin queries or more go through the sorted form: a block
+// an SM needs some thousands of queries a chunk to pay for its sort.  Measured
+// on B200, 1024 arrays of 5.2e8 u64 keys, as given against sorted: b = 8 2^17
+// queries 30 / 40 us, 2^18 49 / 57, 2^19 85 / 74, 2^20 158 / 83; b = 16 2^18 55 /
+// 74, 2^19 100 / 95.
+constexpr uint64_t kBatchSortMin = 1ull << 19;
+
+template <typename K, int NB, int G1, int GS, typename I>
+static int launch_batch_query_as(const tl_batch_plan_impl &P, const K *keys, const K *Q, const uint32_t *qinst,
+                                 uint64_t q, uint64_t *ans, cudaStream_t st) {
+    const uint64_t sms = (uint64_t)batch_sms();
+    // measurement hooks: variant 30 always sorts, 31 never
+    if (query_variant() == 31 || (query_variant() != 30 && q < kBatchSortMin)) {
+        auto kern = batch_query_kernel<K, NB, G1, I>;
+        int per_sm = 0;
+        TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBatchThreads, 0));
+        const uint64_t grid = std::min<uint64_t>((q * G1 + kBatchThreads - 1) / kBatchThreads,
+                                                 (uint64_t)std::max(per_sm, 1) * sms);
+        kern<<<(unsigned)grid, kBatchThreads, 0, st>>>(keys, P.total_keys, P.geo, P.num, (uint32_t)P.b, Q, qinst, q,
+                                                       ans);
+    } else {
+        // equal chunks, one block an SM: the fewest rounds of at most kBatchSortChunk queries
+        const uint64_t rounds = (q + sms * kBatchSortChunk - 1) / (sms * kBatchSortChunk);
+        const uint64_t chunk = (q + sms * rounds - 1) / (sms * rounds);
+        uint32_t shift = 0;  // bins of 2^shift consecutive instances
+        while (((P.num - 1) >> shift) >= kBatchBins) ++shift;
+        const size_t smem = chunk * sizeof(uint16_t);
+        auto kern = batch_query_sorted_kernel<K, NB, GS, I>;
+        kern<<<(unsigned)std::min<uint64_t>((q + chunk - 1) / chunk, sms), kBatchSortThreads, smem, st>>>(
+            keys, P.total_keys, P.geo, P.num, (uint32_t)P.b, shift, (uint32_t)chunk, Q, qinst, q, ans);
+    }
+    TL_CUDA_TRY(cudaGetLastError());
     return TL_SUCCESS;
 }
 
 template <typename K>
 static int launch_batch_query(const tl_batch_plan_impl &P, const K *keys, const K *Q, const uint32_t *qinst,
-                              uint64_t q, uint64_t *ans, char *ws, cudaStream_t st) {
-    auto al = [](uint64_t x) { return (x + 255) / 256 * 256; };
-    unsigned int *count = reinterpret_cast<unsigned int *>(ws);
-    unsigned long long *start = reinterpret_cast<unsigned long long *>(ws + al((uint64_t)P.num * 4));
-    K *sq = reinterpret_cast<K *>(reinterpret_cast<char *>(start) + al(((uint64_t)P.num + 1) * 8));
-    uint32_t *sinst = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(sq) + al(q * sizeof(K)));
-    uint64_t *sidx = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(sinst) + al(q * 4));
-    const int sms = batch_sms();
-    const unsigned g = (unsigned)std::min<uint64_t>((q + 255) / 256, (uint64_t)sms * 8);
-    TL_CUDA_TRY(cudaMemsetAsync(count, 0, (size_t)P.num * 4, st));
-    // queries whose instance id is out of range answer 0 (their answers are
-    // written here, the valid ones by the query kernel)
-    TL_CUDA_TRY(cudaMemsetAsync(ans, 0, q * 8, st));
-    batch_hist_kernel<<<g, 256, 0, st>>>(qinst, q, P.num, count);
-    batch_scan_kernel<<<1, 1024, 0, st>>>(count, P.num, start);
-    batch_bucket_kernel<K><<<g, 256, 0, st>>>(Q, qinst, q, P.num, start, sq, sinst, sidx);
-    TL_CUDA_TRY(cudaGetLastError());
-    // after the bucket pass start[j] holds the end of bucket j; the query kernel
-    // only needs the sorted arrays.  Valid queries: start[num] (read on device).
-    const uint32_t pin_cap = (uint32_t)(48 * 1024 / sizeof(K));
-    const size_t smem = (size_t)pin_cap * sizeof(K);
-    auto kern = batch_query_kernel<K>;
-    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    uint32_t *d_pin = nullptr;
-    keep_pool_memory();
-    TL_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&d_pin), sizeof(P.pin_levels), st));
-    TL_CUDA_TRY(cudaMemcpyAsync(d_pin, P.pin_levels, sizeof(P.pin_levels), cudaMemcpyHostToDevice, st));
-    int per_sm = 0;
-    TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBatchThreads, smem));
-    const uint64_t chunks = (q + P.query_chunk - 1) / P.query_chunk;
-    const unsigned grid = (unsigned)std::min<uint64_t>(chunks, (uint64_t)std::max(per_sm, 1) * sms);
-    kern<<<grid, kBatchThreads, smem, st>>>(keys, P.inst, sq, sinst, sidx, start + P.num, P.query_chunk, d_pin,
-                                           pin_cap, ans);
-    cudaFreeAsync(d_pin, st);
-    TL_CUDA_TRY(cudaGetLastError());
-    return TL_SUCCESS;
+                              uint64_t q, uint64_t *ans, cudaStream_t st) {
+    // 32-bit node indices: a child index is below n + 2 + b * b
+    if (P.max_n < (1ull << 31) && P.b <= 1024) {
+        switch (P.b * sizeof(K)) {
+            case 32: return launch_batch_query_as<K, 32, 2, 1, uint32_t>(P, keys, Q, qinst, q, ans, st);
+            case 64: return launch_batch_query_as<K, 64, 4, 1, uint32_t>(P, keys, Q, qinst, q, ans, st);
+            case 128: return launch_batch_query_as<K, 128, 4, 1, uint32_t>(P, keys, Q, qinst, q, ans, st);
+            case 256: return launch_batch_query_as<K, 256, 4, 4, uint32_t>(P, keys, Q, qinst, q, ans, st);
+            default: return launch_batch_query_as<K, 0, 4, 1, uint32_t>(P, keys, Q, qinst, q, ans, st);
+        }
+    }
+    return launch_batch_query_as<K, 0, 4, 4, uint64_t>(P, keys, Q, qinst, q, ans, st);
 }
 
 int batch_query(const tl_batch_plan *plan, const void *dev_keys, const void *dev_queries, const uint32_t *dev_inst,
@@ -935,12 +1000,11 @@ int batch_query(const tl_batch_plan *plan, const void *dev_keys, const void *dev
     if (q == 0) return TL_SUCCESS;
     EventTimer timer(ms != nullptr, st);
     timer.start();
-    char *ws = static_cast<char *>(dev_ws);
     int rc = P.key_bytes == 8
                  ? launch_batch_query<uint64_t>(P, static_cast<const uint64_t *>(dev_keys),
-                                                static_cast<const uint64_t *>(dev_queries), dev_inst, q, dev_answers, ws, st)
+                                                static_cast<const uint64_t *>(dev_queries), dev_inst, q, dev_answers, st)
                  : launch_batch_query<uint32_t>(P, static_cast<const uint32_t *>(dev_keys),
-                                                static_cast<const uint32_t *>(dev_queries), dev_inst, q, dev_answers, ws, st);
+                                                static_cast<const uint32_t *>(dev_queries), dev_inst, q, dev_answers, st);
     timer.stop();
     if (rc) return rc;
     if (ms) {
@@ -999,11 +1063,11 @@ static int batch_class_keys(const tl_batch_plan_impl &P, std::vector<uint64_t> &
     return TL_SUCCESS;
 }
 
-// Coordinate-descent autotuner.  Permutation: the block size, then per size class
-// (largest classes first) the tile size, each candidate timed on the whole batch
-// (the sorted input restored from a copy before every trial).  Queries: the
-// work-item size, then per size class the number of top levels pinned in shared
-// memory.  The plan keeps the best values; the keys are left sorted.
+// Coordinate-descent autotuner of the permutation: the block size, then per size
+// class (largest classes first) the tile size, each candidate timed on the whole
+// batch (the sorted input restored from a copy before every trial).  The queries
+// have nothing to tune; a batch of them is timed for the report.  The plan keeps
+// the best values; the keys are left sorted.
 int batch_autotune(tl_batch_plan *plan, const int64_t *dev_offsets, void *dev_keys, const void *dev_queries,
                    const uint32_t *dev_inst, uint64_t q, cudaStream_t st, char *report, size_t report_len) {
     if (!plan || !dev_offsets || !dev_keys) return TL_ERROR_INVALID_VALUE;
@@ -1110,31 +1174,6 @@ int batch_autotune(tl_batch_plan *plan, const int64_t *dev_offsets, void *dev_ke
             return TL_SUCCESS;
         };
         if (!rc) rc = time_query(qcur);
-        for (uint32_t ch : {1024u, 4096u}) {
-            if (rc) break;
-            const uint32_t keep = P.query_chunk;
-            P.query_chunk = ch;
-            float ms = 0.f;
-            rc = time_query(ms);
-            if (!rc && ms < qcur) qcur = ms; else P.query_chunk = keep;
-        }
-        for (int c : order) {
-            if (rc) break;
-            const uint32_t keep = P.pin_levels[c];
-            uint32_t best_l = keep;
-            for (uint32_t L : {0u, 2u, 4u}) {
-                if (L == keep) continue;
-                P.pin_levels[c] = L;
-                float ms = 0.f;
-                rc = time_query(ms);
-                if (rc) break;
-                if (ms < qcur) {
-                    qcur = ms;
-                    best_l = L;
-                }
-            }
-            P.pin_levels[c] = best_l;
-        }
         if (qws) cudaFree(qws);
         if (ans) cudaFree(ans);
     }
