@@ -244,3 +244,66 @@ def test_partitioned_queries_match_unpartitioned(layout, n, kb):
     finally:
         L.tl_debug_set_query_variant(0)
     assert torch.equal(tree[got], Q)
+
+
+def _check_answers(tree, sorted_keys, Q, ans):
+    """Hits name a position that holds the key, misses (answer n) are absent;
+    unsigned values."""
+    import torch
+    n = tree.numel()
+    mask = (1 << (8 * tree.element_size())) - 1 if tree.element_size() == 4 else -1
+    ks, q = sorted_keys.to(torch.int64) & mask, Q.to(torch.int64) & mask
+    at = torch.searchsorted(ks, q).clamp_max(n - 1)
+    present = ks[at] == q
+    hit = ans != n
+    assert torch.equal(hit, present)
+    assert bool(((ans >= 0) & (ans <= n)).all())
+    assert torch.equal(tree[ans[hit]], Q[hit])
+
+
+@pytest.mark.parametrize("layout", ["mveb", "veb"])
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("n,skip", [(1, 0), (2, 1), (15, 3), (16, 5), (31, 0), (255, 1), (256, 7), (4095, 0), (4096, 3),
+                                    (65535, 1), (65536, 6), (1_000_003, 1), (2**22 - 1, 5)])
+def test_veb_pieces_unaligned_layouts(layout, kb, n, skip):
+    """Descents piece by piece: sizes around the recursion's splits, a layout
+    that starts `skip` keys into its allocation (pieces cross 32-byte sectors at
+    every phase and may not be read past either end), batches of one query, of
+    one value, around a block's chunk and over several rounds of chunks."""
+    import torch
+    dt = torch.int64 if kb == 8 else torch.int32
+    keys = data.sorted_keys_torch(n, 1, 3, n + skip, kb)
+    buf = torch.empty(n + skip, dtype=dt, device="cuda")
+    tree = buf[skip:]
+    tree.copy_(keys)
+    T.permute(layout, tree)
+    tabs = T.VebTablesDevice(n, "cuda", standard=layout == "veb")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    top = int(keys[-1].item())
+    for q in [1, 147, 149, 16385, 148 * 16384 + 5]:
+        Q = torch.randint(0, top + 3, (q,), generator=g, device="cuda", dtype=torch.int64).to(dt)
+        ans = torch.full((q,), -7, dtype=torch.int64, device="cuda")
+        T.query(layout, tree, Q, ans, tables=tabs)
+        _check_answers(tree, keys, Q, ans)
+    Q = torch.full((20_000,), top, dtype=dt, device="cuda")
+    Q[::1000] = 0
+    ans = torch.empty(20_000, dtype=torch.int64, device="cuda")
+    T.query(layout, tree, Q, ans, tables=tabs)
+    _check_answers(tree, keys, Q, ans)
+
+
+def test_veb_pieces_with_64_bit_positions():
+    """2^31 + 3 keys: positions and path indices past 32 bits."""
+    import torch
+    n = 2**31 + 3
+    keys = torch.arange(n, device="cuda", dtype=torch.int64).to(torch.int32)  # 0 .. n - 1 as uint32
+    T.permute("mveb", keys)
+    tabs = T.VebTablesDevice(n, "cuda")
+    Q64 = torch.randint(0, n + 1000, (1 << 20,), device="cuda", dtype=torch.int64)
+    Q64[:3] = torch.tensor([0, n - 1, n], device="cuda")
+    ans = torch.empty(1 << 20, dtype=torch.int64, device="cuda")
+    T.query("mveb", keys, Q64.to(torch.int32), ans, tables=tabs)
+    hit = ans != n
+    assert torch.equal(hit, Q64 < n)
+    assert torch.equal(keys[ans[hit]], Q64[hit].to(torch.int32))

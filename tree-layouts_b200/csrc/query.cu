@@ -383,137 +383,352 @@ static int g_query_variant = 0;
 void set_query_variant(int v) { g_query_variant = v; }
 int query_variant() { return g_query_variant; }
 
-// ---------------------------------------------------------------- mvEB
-// searchvEB (gpu/src/query-mveb.cuh:43-66): BFS index i and the table recurrence
-// pos[d] = pos[D_d] + R_d + (i & R_d) * L_d, with pos[] in shared memory, one
-// column per thread (32-bit entries when n < 2^32).  Tables are read through the
-// read-only cache.  A descent past the deepest level ends as "absent" (the
-// reference reads past its table there; it only ever issues hits).
-constexpr int kVebThreads = 128;
-constexpr size_t kVebMinPin = 8 * 1024;
-// A batch grouped by value: neighbouring descents share most deep nodes (L1
-// and L2 hits), so more of them in flight pays where it costs L1 hits on a
-// batch as given.  Measured on B200, 2^27 grouped queries over 2^30 - 1 u32
-// mvEB keys (grouping included): 128 threads and 48 KB a block 20.6 ms,
-// 128 / 24 KB 15.0, 128 / 32 KB 17.7, 256 / 40 KB 14.3, 256 / 48 KB 14.0,
-// 256 / 64 KB 16.0, 384 / 56 KB 13.6, 512 / 72 KB 13.5, 1024 / 136 KB
-// 14.7 ms; shapes with more threads on the batch as given 46.6 to 56.4 ms
-// against 40.0 (128 / 48 KB).
-constexpr int kVebGroupThreads = 512;
-constexpr size_t kVebGroupBudget = 72 * 1024;
+// ---------------------------------------------------------------- chunk order
+// A block takes a chunk of the batch at a time and searches it in value order:
+// a counting sort of 16-bit offsets in shared memory, into kSortBins bins of
+// equal width over the chunk's value range (the order inside a bin does not
+// matter, and a skewed batch only loses locality).  All blocks then sweep the
+// layout from low to high values at about the same time, so a page, a line of an
+// upper subtree and a DRAM row serve many descents while they are hot, and the
+// answers go to the chunk's own stretch of the output.
+constexpr int kSortThreads = 1024;  // one block an SM
+constexpr uint32_t kSortBins = 1024;
+constexpr uint32_t kSortChunk = 16384;
+static_assert(kSortBins == kSortThreads, "one bin a thread in the scan");
+static_assert(kSortChunk <= 65536, "16-bit offsets into the chunk");
 
-// QK descents per thread in lock-step: every step takes all of a thread's
-// unresolved queries one level down, so their key loads are in flight together
-// and each level's table entry is read once for all of them.  A query leaves
-// the step loop when it finds its key (res), falls off the tree (bit in
-// `fell`: absent) or leaves the division [offset, limit) (neither: the caller
-// tries the next division).  pos[] holds QK columns per thread:
-// pos[(cd * QK + k) * T + tid].
-template <typename K, typename PosT, int QK>
-__device__ __forceinline__ void veb_descend_multi(const K *__restrict__ A, const K *sm, uint64_t P,
-                                                  const tl_veb_table *__restrict__ tab, uint32_t d, const K (&q)[QK],
-                                                  uint64_t offset, uint64_t limit, PosT *pos, uint32_t todo,
-                                                  uint64_t (&res)[QK], uint32_t &fell) {
-    const uint32_t T = blockDim.x, tid = threadIdx.x;
-    uint64_t i[QK], index[QK];
-#pragma unroll
-    for (int k = 0; k < QK; ++k) {
-        i[k] = 1;
-        index[k] = 0;
-        pos[k * T + tid] = 1;
+struct ChunkSort {
+    unsigned long long lo, hi;
+    uint32_t cnt[kSortBins], wsum[32];
+};
+
+// order[0, len): the chunk's offsets by value.
+template <typename K>
+__device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t len, uint16_t *order, ChunkSort &cs) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();  // the previous chunk is done with its order
+    if (threadIdx.x == 0) {
+        cs.lo = ~0ull;
+        cs.hi = 0;
     }
-    uint32_t act = todo;
-    uint32_t cd = 0;
-    while (act) {
-        K cur[QK];
+    cs.cnt[threadIdx.x] = 0;
+    __syncthreads();
+    K lo = ~K(0), hi = 0;
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < len; x += kSortThreads) {
+        const K v = __ldg(Q + x);
+        lo = min(lo, v);
+        hi = max(hi, v);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
+    }
+    if (lane == 0 && warp * 32 < len) {
+        atomicMin(&cs.lo, (unsigned long long)lo);
+        atomicMax(&cs.hi, (unsigned long long)hi);
+    }
+    __syncthreads();
+    const K base = (K)cs.lo;
+    const uint32_t span = bit_length(cs.hi - cs.lo), bits = bit_length(kSortBins - 1);
+    const uint32_t shift = span > bits ? span - bits : 0;
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < len; x += kSortThreads)
+        atomicAdd(&cs.cnt[(uint32_t)((__ldg(Q + x) - base) >> shift)], 1u);
+    __syncthreads();
+    const uint32_t c = cs.cnt[threadIdx.x];
+    uint32_t inc = c;
 #pragma unroll
-        for (int k = 0; k < QK; ++k) {
-            cur[k] = K(0);
-            if ((act >> k) & 1u) {
-                if (index[k] + offset < limit)
-                    cur[k] = key_at(A, sm, P, offset + index[k]);
-                else
-                    act &= ~(1u << k);  // left the division: not resolved here
-            }
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+    }
+    if (lane == 31) cs.wsum[warp] = inc;
+    __syncthreads();
+    const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? cs.wsum[lane] : 0u);
+    cs.cnt[threadIdx.x] = before + inc - c;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < len; x += kSortThreads)
+        order[atomicAdd(&cs.cnt[(uint32_t)((__ldg(Q + x) - base) >> shift)], 1u)] = (uint16_t)x;
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------- mvEB
+// searchvEB (gpu/src/query-mveb.cuh:43-66) finds the node at depth c of a path
+// with BFS index i at pos[c] = pos[D_c] + R_c + (i & R_c) * L_c, one dependent
+// key load a level.  A vEB layout stores every subtree of its recursion in one
+// stretch, so here a descent goes down a piece of up to kVebPieceLevels levels
+// at a time: a thread reads the piece's 2^h - 1 keys together (aligned 32-byte
+// sectors), and the number of them below q is q's path through all h levels.
+// The order inside a piece is never looked at, only that it is contiguous: each
+// block works that out from the tables as given (veb_piece_levels), so tables
+// of any split rule do, and a depth where nothing longer is contiguous is a
+// piece of one level.  pos[] needs an entry per piece (8 for the 29 levels of a
+// 3e8-key mvEB), one column per thread in shared memory.  The levels above the
+// first pieces (division 0 only, as many as the budget holds) are gathered into
+// shared memory in BFS order, where a level costs one bank access.
+//
+// What bounds it: a load of a thread's own line is an L1 wavefront, so a level
+// at a time costs 29 a query; a 15-key piece costs at most 3 for 4 levels and a
+// pinned level about a tenth.  ncu, 2^24 queries over 3e8 u32 keys: L1 data pipe
+// 78 %, DRAM 48 %, issue 41 %.  Measured on B200, 2^26 queries over 3e8 u32 mvEB
+// keys: a level at a time over a batch grouped by value in device memory 7.10
+// ms (18.7 as given); pieces over the same grouped batch 6.2, with pinned
+// levels 5.2, over chunks ordered in shared memory 4.24 (over the batch as
+// given 17.1: the descents then share no pages).  Two or four lanes a piece
+// 6.0 and 9.7 ms, four lanes reading each other's pieces 5.5 (half the
+// wavefronts, twice the instructions); 512-thread blocks 5.8; chunks of 4096 /
+// 8192 / 32768 queries 4.76 / 4.46 / 4.62; 64 KB of pinned levels 4.6 (L1 is
+// smaller).  It holds for every batch: 2^10 queries 27 -> 14 us, 2^20 369 -> 95.
+//
+// Tables whose pieces do not chain (not built by buildTable), a piece that
+// reaches past its division, and divisions beyond the first kVebSchedTables
+// take the descent level by level (veb_descend_levels); a descent past the
+// deepest level ends as "absent" (the reference reads past its table there; it
+// only ever issues hits).
+constexpr uint32_t kVebPieceLevels = 4;
+constexpr uint32_t kVebMaxSteps = 16;
+constexpr uint32_t kVebSchedTables = 4;  // divisions with a piece schedule (the rest hold a few keys)
+
+struct VebStep {
+    uint64_t L, R;
+    uint32_t D, h;  // the earlier step the position is relative to; the piece's levels
+    uint32_t c;     // the depth of the piece's root
+};
+struct VebSchedule {
+    VebStep step[kVebMaxSteps];
+    uint32_t steps;  // 0: level by level
+    uint32_t top, ktop;  // levels held in shared memory, and the step that starts below them
+};
+
+// 1-based position of the node at depth c with BFS index i.
+__device__ __forceinline__ uint64_t veb_node_pos(const tl_veb_table *tab, uint32_t c, uint64_t i) {
+    uint64_t p = 1;
+    while (c) {
+        p += tab[c].R + (i & tab[c].R) * tab[c].L;
+        i >>= c - tab[c].D;
+        c = tab[c].D;
+    }
+    return p;
+}
+
+// Whether the table stores the subtree of h levels rooted at depth c in one
+// stretch of 2^h - 1 positions from its root's on: the recursion splits it at
+// some depth e into a top tree and bottoms that are contiguous themselves, the
+// bottoms one after the other behind the top tree.  tab has d entries.
+__device__ __forceinline__ bool veb_splits(const tl_veb_table *tab, uint32_t c, uint32_t e, uint32_t h) {
+    return tab[e].D == c && tab[e].R == low_mask(e - c) && tab[e].L == low_mask(c + h - e);
+}
+__device__ __forceinline__ bool veb_contiguous2(const tl_veb_table *tab, uint32_t d, uint32_t c) {
+    return c + 2 <= d && veb_splits(tab, c, c + 1, 2);
+}
+__device__ __forceinline__ bool veb_contiguous3(const tl_veb_table *tab, uint32_t d, uint32_t c) {
+    return c + 3 <= d && ((veb_splits(tab, c, c + 1, 3) && veb_contiguous2(tab, d, c + 1)) ||
+                          (veb_splits(tab, c, c + 2, 3) && veb_contiguous2(tab, d, c)));
+}
+__device__ __forceinline__ uint32_t veb_piece_levels(const tl_veb_table *tab, uint32_t d, uint32_t c) {
+    const bool c2 = veb_contiguous2(tab, d, c), c3 = veb_contiguous3(tab, d, c);
+    if (c + 4 <= d && ((veb_splits(tab, c, c + 1, 4) && veb_contiguous3(tab, d, c + 1)) ||
+                       (veb_splits(tab, c, c + 2, 4) && c2 && veb_contiguous2(tab, d, c + 2)) ||
+                       (veb_splits(tab, c, c + 3, 4) && c3)))
+        return 4;
+    return c3 ? 3 : c2 ? 2 : 1;
+}
+
+// The piece schedule of a table of d levels, by one warp: tab gets the table,
+// piece is 64 bytes of scratch.  The levels [0, out.top) go to shared memory:
+// down to the start of a piece, at most max_top, all of their keys below
+// position `limit` (the rightmost node of a depth has the largest position).
+__device__ void veb_schedule(const tl_veb_table *__restrict__ gtab, uint32_t d, uint32_t max_steps, uint32_t max_top,
+                             uint64_t limit, VebSchedule &out, tl_veb_table *tab, unsigned char *piece) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t e = lane; e < d; e += 32) tab[e] = gtab[e];
+    __syncwarp();
+    bool bad = false;  // this lane's depth has a key past the limit (max_top <= 32)
+    for (uint32_t c = lane; c < d; c += 32) piece[c] = (unsigned char)veb_piece_levels(tab, d, c);
+    __syncwarp();
+    uint32_t k = 0;
+    if (lane == 0) {
+        unsigned char at[64];  // the step that starts at a depth, or 255
+        for (uint32_t e = 0; e < d; ++e) at[e] = 255;
+        bool ok = true;
+        for (uint32_t c = 0; c < d; ++k) {
+            const uint32_t D = c ? tab[c].D : 0;
+            ok = k < max_steps && (c == 0 || (D < c && at[D] != 255));
+            if (!ok) break;
+            at[c] = (unsigned char)k;
+            VebStep &st = out.step[k];
+            st.L = c ? tab[c].L : 0;
+            st.R = c ? tab[c].R : 0;
+            st.D = at[D];
+            st.h = piece[c];
+            st.c = c;
+            c += piece[c];
         }
-#pragma unroll
-        for (int k = 0; k < QK; ++k)
-            if (((act >> k) & 1u) && q[k] == cur[k]) {
-                res[k] = offset + index[k];
-                act &= ~(1u << k);
-            }
-        if (!act) break;
-        if (cd + 1 >= d) {
-            fell |= act;
-            break;
+        k = ok ? k : 0;
+        out.steps = k;
+    }
+    k = __shfl_sync(0xFFFFFFFFu, k, 0);
+    if (k && lane < max_top) bad = veb_node_pos(tab, lane, (2ull << lane) - 1) > limit;
+    const uint32_t b = __ballot_sync(0xFFFFFFFFu, bad), full = b ? __ffs(b) - 1 : 32;
+    if (lane == 0) {
+        uint32_t kt = 0;
+        while (kt + 1 < k && out.step[kt + 1].c <= min(max_top, full)) ++kt;
+        out.ktop = kt;
+        out.top = k ? out.step[kt].c : 0;
+    }
+}
+
+// One descent level by level.  Returns 1 found (res), 2 absent, 0 left the
+// division [offset, limit) (the caller tries the next one).
+template <typename K>
+__device__ __noinline__ int veb_descend_levels(const K *__restrict__ A, const tl_veb_table *__restrict__ tab, uint32_t d,
+                                               K q, uint64_t offset, uint64_t limit, uint64_t &res) {
+    uint64_t pos[64];
+    uint64_t i = 1, index = 0;
+    pos[0] = 1;
+    for (uint32_t c = 0;;) {
+        if (index + offset >= limit) return 0;
+        const K cur = __ldg(A + offset + index);
+        if (q == cur) {
+            res = offset + index;
+            return 1;
         }
-        ++cd;
-        const uint64_t L = __ldg(&tab[cd].L), R = __ldg(&tab[cd].R);
-        const uint32_t D = __ldg(&tab[cd].D);
-        if (D >= cd) {  // not a table built by buildTable: stop instead of reading outside pos[]
-            fell |= act;
-            break;
-        }
-#pragma unroll
-        for (int k = 0; k < QK; ++k)
-            if ((act >> k) & 1u) {
-                i[k] = 2 * i[k] + (q[k] > cur[k]);
-                const uint64_t p = (uint64_t)pos[(D * QK + k) * T + tid] + R + (i[k] & R) * L;
-                pos[(cd * QK + k) * T + tid] = (PosT)p;
-                index[k] = p - 1;
-            }
+        if (++c >= d) return 2;
+        const uint64_t L = __ldg(&tab[c].L), R = __ldg(&tab[c].R);
+        const uint32_t D = __ldg(&tab[c].D);
+        if (D >= c) return 2;  // not a table built by buildTable: stop instead of reading outside pos[]
+        i = 2 * i + (q > cur);
+        pos[c] = pos[D] + R + (i & R) * L;
+        index = pos[c] - 1;
     }
 }
 
 // idx == nullptr: perfect layout, one table (timeQueryvEB); otherwise the
 // non-perfect table set (timeQueryvEB_nonperfect): the divisions in order, each
-// query until it is resolved.  A block takes QK * T consecutive queries at a
-// time, thread t the queries t, t + T, ...
-template <typename K, typename PosT, int QK, int kThreads>
-__global__ void __launch_bounds__(kThreads)
-veb_query_kernel(const K *__restrict__ A, uint64_t n, uint64_t P, uint32_t dmax,
+// query until it is resolved.  A division's path is followed to its end on
+// counts alone; an equal key is then where the path last went left, one chain of
+// the recurrence and one load.  I: index type (32 bits when n < 2^31).
+template <typename K, typename I>
+__global__ void __launch_bounds__(kSortThreads, 1)
+veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t max_top, uint32_t chunk,
                  const tl_veb_table *__restrict__ tables, const uint64_t *__restrict__ idx,
-                 const uint32_t *__restrict__ table_idx, uint32_t num_tables, const K *__restrict__ Q,
-                 uint64_t nq, const uint32_t *__restrict__ perm, uint64_t *__restrict__ ans) {
+                 const uint32_t *__restrict__ table_idx, uint32_t num_tables, const K *__restrict__ Q, uint64_t nq,
+                 uint64_t *__restrict__ ans) {
+    constexpr uint32_t KPL = 32 / sizeof(K);             // keys per sector
+    constexpr uint32_t M = (1u << kVebPieceLevels) - 1;  // keys of the longest piece
+    constexpr int NS = (M + KPL - 1 + KPL - 1) / KPL;    // sectors it may span
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PosT *pos = reinterpret_cast<PosT *>(smem_raw);
-    K *sm = reinterpret_cast<K *>(smem_raw + ((size_t)dmax * QK * blockDim.x * sizeof(PosT) + 15) / 16 * 16);
-    pin_prefix(A, P, sm);
-    const uint64_t T = blockDim.x;
-    for (uint64_t base = (uint64_t)blockIdx.x * QK * T; base < nq; base += (uint64_t)gridDim.x * QK * T) {
-        K q[QK];
-        uint64_t res[QK];
-        uint32_t todo = 0, fell = 0;
+    I *pos = reinterpret_cast<I *>(smem_raw) + threadIdx.x;  // [cols][kSortThreads], this thread's column
+    K *tree = reinterpret_cast<K *>(smem_raw + (size_t)cols * kSortThreads * sizeof(I));  // [2^max_top], from 1
+    uint16_t *order = reinterpret_cast<uint16_t *>(tree + (1ull << max_top));             // [chunk]
+    __shared__ ChunkSort cs;
+    __shared__ VebSchedule sched[kVebSchedTables];
+    __shared__ tl_veb_table s_tabs[kVebSchedTables][64];
+    __shared__ unsigned char s_piece[kVebSchedTables][64];
+    const tl_veb_table *s_tab = s_tabs[0];
+    const I n = (I)n64;
+    static_assert(kSortThreads / 32 >= kVebSchedTables, "a warp a division");
+    if (const uint32_t j = threadIdx.x / 32; j < min(num_tables, kVebSchedTables)) {
+        const uint64_t first = idx && j ? __ldg(idx + j - 1) : 0;
+        veb_schedule(idx ? tables + __ldg(table_idx + j) : tables, bit_length(n64 - first), cols, j == 0 ? max_top : 0,
+                     idx ? __ldg(idx + j) : n64, sched[j], s_tabs[j], s_piece[j]);
+    }
+    __syncthreads();
+    const uint32_t top = sched[0].top;
+    for (uint32_t x = threadIdx.x + 1; x < (1u << top); x += kSortThreads) {
+        const uint64_t p = veb_node_pos(s_tab, 31 - __clz(x), x) - 1;
+        tree[x] = p < n64 ? __ldg(A + p) : K(0);
+    }
+    __syncthreads();
+    const uint32_t a_off = (uint32_t)(reinterpret_cast<uintptr_t>(A) & 31) / sizeof(K);
+    const I low = a_off ? KPL : 0;  // a piece from here on can be read in whole sectors
+    for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
+        const uint32_t len = (uint32_t)min((uint64_t)chunk, nq - c0);
+        chunk_order(Q + c0, len, order, cs);
+        for (uint32_t slot = threadIdx.x; slot < len; slot += kSortThreads) {
+            const uint64_t qi = c0 + order[slot];
+            const K q = __ldg(Q + qi);
+            I res = n, offset = 0;
+            for (uint32_t j = 0; j < num_tables; ++j) {
+                const uint64_t lim64 = idx ? __ldg(idx + j) : n64;
+                const I limit = (I)lim64;
+                const uint32_t steps = j < kVebSchedTables ? sched[j].steps : 0;
+                bool slow = steps == 0, left = false;
+                I i = 1;
+                uint32_t c = 0, k = 0;
+                if (j == 0 && top) {
+                    uint32_t x = 1;
+                    for (; c < top; ++c) x = 2 * x + (tree[x] < q);
+                    i = x;
+                    for (; k < sched[0].ktop; ++k) {
+                        const VebStep &st = sched[0].step[k];
+                        const I b = i >> (top - st.c);
+                        pos[k * kSortThreads] =
+                            k ? (I)(pos[st.D * kSortThreads] + (I)st.R + (b & (I)st.R) * (I)st.L) : (I)1;
+                    }
+                }
+                for (; k < steps; ++k) {
+                    const VebStep &st = sched[j].step[k];
+                    const uint32_t h = st.h, m = (1u << h) - 1;
+                    const I p = k ? (I)(pos[st.D * kSortThreads] + (I)st.R + (i & (I)st.R) * (I)st.L) : (I)1;
+                    pos[k * kSortThreads] = p;
+                    const I s = offset + p - 1;
+                    if (s >= limit || limit - s < (I)m) {
+                        slow = s < limit;  // a piece across the division's end; else left the division
+                        left = true;
+                        break;
+                    }
+                    const uint32_t o = (uint32_t)((s + a_off) % KPL);  // the piece's first slot in its sector
+                    K v[NS][KPL];
+                    if (s >= low && n - s >= (I)(M + KPL)) {
+                        const K *at = A + s - o;
 #pragma unroll
-        for (int k = 0; k < QK; ++k) {
-            const uint64_t qi = base + k * T + threadIdx.x;
-            res[k] = n;
-            q[k] = K(0);
-            if (qi < nq) {
-                q[k] = __ldcs(Q + qi);
-                todo |= 1u << k;
+                        for (int t = 0; t < NS; ++t)
+                            if (t * KPL < o + m) ldg32(at + t * KPL, v[t]);
+                    } else {
+#pragma unroll
+                        for (int t = 0; t < NS; ++t)
+#pragma unroll
+                            for (uint32_t e = 0; e < KPL; ++e) {
+                                const uint32_t sl = t * KPL + e;
+                                v[t][e] = sl >= o && sl < o + m ? __ldg(A + s + (sl - o)) : K(0);
+                            }
+                    }
+                    uint32_t l = 0;
+#pragma unroll
+                    for (int t = 0; t < NS; ++t)
+#pragma unroll
+                        for (uint32_t e = 0; e < KPL; ++e) l |= (v[t][e] < q ? 1u : 0u) << (t * KPL + e);
+                    i = (i << h) + (I)__popc((l >> o) & ((1u << m) - 1));
+                    c += h;
+                }
+                const tl_veb_table *tab = idx ? tables + __ldg(table_idx + j) : tables;
+                if (slow) {
+                    uint64_t r = 0;
+                    const int rc = veb_descend_levels(A, tab, bit_length(n64 - (uint64_t)offset), q, (uint64_t)offset,
+                                                      lim64, r);
+                    if (rc == 1) res = (I)r;
+                    if (rc) break;
+                } else {
+                    // the smallest key of the path at or above q: above the path's trailing right turns
+                    const I right = ~i;
+                    const uint32_t up = sizeof(I) == 8 ? __ffsll((long long)right) : __ffs((int)right);
+                    const I node = up ? (i >> (up - 1)) >> 1 : 0;
+                    if (node) {
+                        const tl_veb_table *t = j < kVebSchedTables ? s_tabs[j] : tab;
+                    const I at = offset + (I)(veb_node_pos(t, c - up, node) - 1);
+                        if (at < limit && __ldg(A + at) == q) {
+                            res = at;
+                            break;
+                        }
+                    }
+                    if (!left) break;  // past the deepest level: absent
+                }
+                offset = limit;
             }
-        }
-        if (!idx) {
-            veb_descend_multi<K, PosT, QK>(A, sm, P, tables, bit_length(n), q, 0, n, pos, todo, res, fell);
-        } else {
-            uint64_t offset = 0;
-            for (uint32_t j = 0; j < num_tables && todo; ++j) {
-                const uint64_t lim = __ldg(idx + j);
-                veb_descend_multi<K, PosT, QK>(A, sm, P, tables + __ldg(table_idx + j), bit_length(n - offset), q,
-                                               offset, lim, pos, todo, res, fell);
-#pragma unroll
-                for (int k = 0; k < QK; ++k)
-                    if (res[k] != n) todo &= ~(1u << k);  // found
-                todo &= ~fell;                             // absent
-                offset = lim;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < QK; ++k) {
-            const uint64_t qi = base + k * T + threadIdx.x;
-            const uint64_t out = qi < nq ? (perm ? (uint64_t)__ldg(perm + qi) : qi) : nq;
-            if (out < nq) __stcs(ans + out, res[k]);
+            ans[qi] = (uint64_t)res;
         }
     }
 }
@@ -904,20 +1119,18 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
     const K *Q = static_cast<const K *>(a.queries);
     uint64_t P = std::min<uint64_t>(a.n, kPinBytes / sizeof(K));
     unsigned grid = 1;
-    // BST and vEB descents search a batch of 2^21 queries or more grouped by
-    // value, over a vEB layout of 4 MB or more and a BST of 64 MB or more.
-    // Measured on B200, as given against grouped (grouping included): mvEB
-    // 2^30 - 1 u32, 2^27 queries 39.8 / 13.5 ms; mvEB 2^20 - 1 u32, 2^22
-    // queries 0.49 / 0.32 ms, 2^20 queries 0.14 / 0.14; BST 2^23 - 1 u64 (64
-    // MB), 2^22 queries 0.39 / 0.31 ms, 2^20 queries 0.11 / 0.13; BST 2^22 - 1
-    // u64 (32 MB) 0.30 / 0.29 at 2^22 and 9.2 / 11.4 ms at 2^27 queries.
-    // B-tree nodes gain little even sorted (9.45 against 8.28 ms) and keep the
-    // batch's order.  Measurement hooks: variant 19 never groups, 20 always.
+    // BST descents search a batch of 2^21 queries or more grouped by value, over
+    // a layout of 64 MB or more.  Measured on B200, as given against grouped
+    // (grouping included): 2^23 - 1 u64 keys (64 MB), 2^22 queries 0.39 / 0.31
+    // ms, 2^20 queries 0.11 / 0.13; 2^22 - 1 u64 (32 MB) 0.30 / 0.29 at 2^22 and
+    // 9.2 / 11.4 ms at 2^27 queries.  B-tree nodes gain little even sorted (9.45
+    // against 8.28 ms) and keep the batch's order; vEB descents order chunks of
+    // it in shared memory.  Measurement hooks: variant 19 never groups, 20 always.
     QueryPartition part;
     const uint32_t *perm = nullptr;
     const uint64_t tree_bytes = a.n * sizeof(K);
-    const bool large = a.layout == Q_BST ? tree_bytes >= (64ull << 20) : tree_bytes >= (4ull << 20);
-    if ((a.layout == Q_BST || a.layout == Q_VEB || a.layout == Q_VEB_NP) && g_query_variant != 19 &&
+    const bool large = tree_bytes >= (64ull << 20);
+    if (a.layout == Q_BST && g_query_variant != 19 &&
         a.q < (1ull << 32) && (g_query_variant == 20 || (a.q >= (1ull << 21) && large))) {
         const int rc = partition_queries<K>(Q, a.q, st, part);
         if (rc == TL_SUCCESS) {
@@ -1060,43 +1273,29 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         const uint32_t dmax = bit_length(a.n);
         if (dmax > 63) return TL_ERROR_UNSUPPORTED;
         const bool np = a.layout == Q_VEB_NP;
-        const bool narrow = a.n < (1ull << 32);
-        // QK columns of pos[] per thread; the layout's first positions pinned
-        // in what is left of the block's shared-memory budget
-        // one descent per thread: measured faster on B200 than two or four in
-        // lock-step (2^27 queries over 2^30 - 1 u32 keys: 40.5 ms against 55.5
-        // and 55.6; over 3e8 keys 36.6 against 49.0 and 49.3)
-        const int qk = g_query_variant == 3 ? 2 : g_query_variant == 4 ? 4 : 1;
-        const bool grouped = perm != nullptr && qk == 1;
-        const int threads = grouped ? kVebGroupThreads : kVebThreads;
-        const size_t budget = grouped ? kVebGroupBudget : qk == 1 ? 48 * 1024 : qk == 2 ? 72 * 1024 : 110 * 1024;
-        const size_t pos_bytes = (size_t)dmax * qk * threads * (narrow ? 4 : 8);
-        const size_t pin_budget = pos_bytes + kVebMinPin <= budget ? budget - pos_bytes : kVebMinPin;
-        P = std::min<uint64_t>(a.n, pin_budget / sizeof(K));
-        const size_t smem = (pos_bytes + 15) / 16 * 16 + P * sizeof(K);
-        if (smem > 227 * 1024) return TL_ERROR_UNSUPPORTED;  // pos[] of a tree deeper than about 50 levels
-        auto launch = [&](auto kern, int qpt) -> int {
+        const bool narrow = a.n < (1ull << 31);
+        // pieces are 2.5 levels long on average at worst (heights 2, 3, 2, 3, ...)
+        const uint32_t cols = std::min<uint32_t>(kVebMaxSteps, (2 * dmax + 4) / 5 + 1);
+        // pinned levels: at most 32 KB from 2^20 queries, else 16 KB (a block
+        // gathers them; 2^18 queries over 3e8 u32 keys 41 against 44 us, 2^20 97
+        // against 94)
+        const size_t top_bytes = a.q >= (1ull << 20) ? 32 * 1024 : 16 * 1024;
+        uint32_t max_top = 0;
+        while (max_top + 1 < dmax && (sizeof(K) << (max_top + 1)) <= top_bytes) ++max_top;
+        auto launch = [&](auto kern) -> int {
+            const uint64_t slots = query_sm_count();
+            const uint64_t rounds = (a.q + slots * kSortChunk - 1) / (slots * kSortChunk);
+            const uint64_t chunk = (a.q + slots * rounds - 1) / (slots * rounds);  // equal chunks, the fewest rounds
+            const size_t smem = (size_t)cols * kSortThreads * (narrow ? 4 : 8) + (sizeof(K) << max_top) +
+                                chunk * sizeof(uint16_t);
             TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            int per_sm = 0;
-            TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-            uint64_t g = (uint64_t)std::max(per_sm, 1) * query_sm_count();
-            uint64_t need = (a.q + (uint64_t)qpt * threads - 1) / ((uint64_t)qpt * threads);
-            unsigned gr = (unsigned)std::max<uint64_t>(1, std::min(g, need));
-            kern<<<gr, threads, smem, st>>>(A, a.n, P, dmax, a.tables, np ? a.idx : nullptr,
-                                                np ? a.table_idx : nullptr, np ? a.num_tables : 1u, Q, a.q, perm,
-                                                a.answers);
+            const uint64_t blocks = std::min(slots, (a.q + chunk - 1) / chunk);
+            kern<<<(unsigned)blocks, kSortThreads, smem, st>>>(A, a.n, cols, max_top, (uint32_t)chunk, a.tables,
+                                                              np ? a.idx : nullptr, np ? a.table_idx : nullptr,
+                                                              np ? a.num_tables : 1u, Q, a.q, a.answers);
             return TL_SUCCESS;
         };
-        int rc;
-        constexpr int T1 = kVebThreads, TG = kVebGroupThreads;
-        if (grouped)
-            rc = narrow ? launch(veb_query_kernel<K, uint32_t, 1, TG>, 1) : launch(veb_query_kernel<K, uint64_t, 1, TG>, 1);
-        else if (qk == 1)
-            rc = narrow ? launch(veb_query_kernel<K, uint32_t, 1, T1>, 1) : launch(veb_query_kernel<K, uint64_t, 1, T1>, 1);
-        else if (qk == 2)
-            rc = narrow ? launch(veb_query_kernel<K, uint32_t, 2, T1>, 2) : launch(veb_query_kernel<K, uint64_t, 2, T1>, 2);
-        else
-            rc = narrow ? launch(veb_query_kernel<K, uint32_t, 4, T1>, 4) : launch(veb_query_kernel<K, uint64_t, 4, T1>, 4);
+        const int rc = narrow ? launch(veb_query_kernel<K, uint32_t>) : launch(veb_query_kernel<K, uint64_t>);
         if (rc) return rc;
     }
     TL_CUDA_TRY(cudaGetLastError());
