@@ -162,3 +162,37 @@ def test_learned_kernel_forms_equal_plain_answers(variant):
     finally:
         L.tl_debug_set_query_variant(0)
     assert torch.equal(plain, learned)
+
+
+@pytest.mark.parametrize("n,b", [(2, 16), (15, 16), (17, 8), (288, 16), (4913, 16), (100_003, 8), (1_000_003, 32),
+                                 (2_000_017, 16)])
+@pytest.mark.parametrize("variant", [0, 8])
+def test_learned_index_widths_equal_plain_answers(n, b, variant):
+    """The 32-bit index form (the default below 2^31 keys) and the 64-bit one
+    (variant 8) give the plain query's answers, past both ends included, for a
+    model of the keys and for one of other keys (windows that are wrong only
+    cost restarts)."""
+    import ctypes as C
+
+    import torch
+    L = T.lib()
+    L.tl_debug_set_query_variant.argtypes = [C.c_int]
+    keys = _keys(n, seed=3) if n > 1000 else torch.arange(n, device="cuda", dtype=torch.int64) * 977 + 5
+    tree = keys.clone()
+    T.permute("btree", tree, b)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    Q = torch.cat([keys[torch.randint(0, n, (20_000,), generator=g, device="cuda")],
+                   torch.randint(0, 2**62, (20_000,), generator=g, device="cuda"), keys[:1] - 1, keys[-1:] + 1,
+                   torch.tensor([0, 1, 2**62], device="cuda")])
+    plain = torch.empty(Q.numel(), dtype=torch.int64, device="cuda")
+    T.query("btree", tree, Q, plain, b)
+    for fit in (keys, torch.arange(n, device="cuda", dtype=torch.int64) * 3 + 1):
+        model, leaves = LL.train(fit, num_leaves=256, steps=50, batch=4096)
+        learned = torch.full((Q.numel(),), -7, dtype=torch.int64, device="cuda")
+        L.tl_debug_set_query_variant(variant)
+        try:
+            LL.query(tree, model, leaves, Q, learned, b)
+        finally:
+            L.tl_debug_set_query_variant(0)
+        assert torch.equal(plain, learned), (n, b, variant)

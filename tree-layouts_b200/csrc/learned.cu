@@ -249,6 +249,14 @@ __device__ __forceinline__ tl_rank_leaf load_leaf(const tl_rank_leaf *__restrict
     return leaf_from_words(w);
 }
 
+// leaf_predict for n < 2^31.
+__device__ __forceinline__ uint32_t leaf_predict32(const tl_rank_leaf &lf, uint64_t key, uint32_t n) {
+    const float off = key > lf.kmin ? (float)(key - lf.kmin) : 0.f;
+    const float d = lf.slope * off;  // >= 0: slopes are non-negative
+    const uint32_t ri = (uint32_t)lf.base + (d > 0.f ? (uint32_t)fminf(d + 0.5f, 2147483648.f) : 0u);
+    return ri < n ? ri : n - 1;
+}
+
 // Rank prediction of a segment, clamped to [0, n).
 // The segment's base rank stays an integer and only the offset within the
 // segment is FP32 (the base itself in FP32 would round to 64 ranks near 2^30,
@@ -594,6 +602,7 @@ __global__ void rmi_predict_kernel(const __grid_constant__ ModelParams p, bool u
 struct LearnedGeom {
     BtreeGeom g;
     FastDiv64 fd;
+    FastDiv32 fd32;
     uint64_t cmax;  // (n + 1) / (b + 1): nodes below it have a child inside the layout
 };
 
@@ -692,6 +701,41 @@ __device__ __forceinline__ uint64_t learned_start_at(const LearnedGeom &G, const
         --k;
     }
     const uint64_t i = g.pw[k] - 1 + glo * B;
+    if (i >= n) return 0;
+    flags = kSubtree;
+    depth = k;
+    return i;
+}
+
+// learned_start_at with 32-bit ranks, gaps and node indices (n < 2^31).
+template <uint32_t B>
+__device__ __forceinline__ uint32_t learned_start_at32(const LearnedGeom &G, const tl_rank_leaf &lf, uint64_t q,
+                                                       uint32_t &flags, uint32_t &depth) {
+    const BtreeGeom &g = G.g;
+    const uint32_t n = (uint32_t)g.n, li = (uint32_t)(g.l + g.i), lir = (uint32_t)g.lir, lr = (uint32_t)(g.l + g.r);
+    const uint32_t gi = (uint32_t)g.i;
+    flags = 0;
+    depth = 0;
+    if (g.h == 0) return 0;
+    const uint32_t pr = leaf_predict32(lf, q, n);
+    const uint32_t rlo = pr > lf.eps_lo ? pr - lf.eps_lo : 0;
+    const uint32_t rhi = lf.eps_hi < n - pr ? pr + lf.eps_hi : n - 1;
+    // the gap below rlo and the gap above rhi (rank_gaps)
+    const uint32_t qlo = G.fd32.div(rlo), qhi = G.fd32.div(rhi);
+    uint32_t glo = rlo < li ? qlo : rlo < lir ? gi : rlo - lr;
+    uint32_t ghi = rhi < li ? qhi + (rhi - qhi * (B + 1) < B ? 0u : 1u) : rhi < lir ? gi : rhi - lr + 1;
+    uint32_t k = g.h;  // depth of the subtree root (h = a last-level node)
+    while (glo != ghi) {
+        glo = G.fd32.div(glo);
+        ghi = G.fd32.div(ghi);
+        --k;
+    }
+    // a last-level node that does not exist: start one level up
+    if (k == g.h && !(glo < gi || (glo == gi && g.r > 0))) {
+        glo = G.fd32.div(glo);
+        --k;
+    }
+    const uint32_t i = (uint32_t)g.pw[k] - 1 + glo * B;
     if (i >= n) return 0;
     flags = kSubtree;
     depth = k;
@@ -855,22 +899,29 @@ learned_query_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, const 
 // of GL sectors, one L1 wavefront each (the plain B-tree query's node read).
 // Idle groups take the prepared starts in group order; the group adds its
 // lanes' counts with full-warp shuffles and learns of an equal key by ballot.
-template <int NB, int GL, bool kStats>
+// I: ranks, gaps and node indices, 32 bits when n < 2^31.  The kernel is bound
+// by instruction issue (ncu: 71 % at 2^24 Zipf queries over 2^26 skewed keys with
+// 64-bit indices), and 64-bit divisions, products and shuffles of indices were
+// a quarter of its instructions.  Measured on B200, b = 16, 64 -> 32 bits: 2^26
+// queries over 2^27 keys 3.19 -> 2.51 ms, 2^24 over 2^26 keys (2^16 segments)
+// 875 -> 682 us.  512 x 3 blocks 2.60, 1024 x 1 2.93, 1024 x 2 (spills) 3.20 ms.
+template <int NB, int GL, bool kStats, typename I>
 __global__ void __launch_bounds__(kLearnedGroupThreads, TL_LEARNED_GROUP_MIN_BLOCKS)
 learned_query_group_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, const __grid_constant__ ModelParams p,
                            int use_net, const tl_rank_leaf *__restrict__ leaves, const uint64_t *__restrict__ Q,
                            uint64_t nq, uint64_t *__restrict__ ans, unsigned long long *__restrict__ stats) {
-    constexpr uint64_t B = NB / 8;
+    constexpr I B = NB / 8;
     constexpr int KPL = 4;               // keys per 32-byte load
     constexpr int NL = NB / (32 * GL);   // loads per lane and node
     static_assert((GL == 2 || GL == 4 || GL == 8) && NL >= 1 && NL * GL * 32 == NB, "2, 4 or 8 lanes per node");
     constexpr unsigned kLeaders = GL == 2 ? 0x55555555u : GL == 4 ? 0x11111111u : 0x01010101u;
-    constexpr uint64_t kFlagShift = 61, kNodeMask = (1ull << kFlagShift) - 1;
+    constexpr I kNone = ~I(0);                     // an idle group
+    constexpr I kStart = I(1) << (sizeof(I) * 8 - 1);  // a prepared start below the root (kSubtree)
     __shared__ PiecesSmem sp;
     if (use_net) stage_pieces(p, sp);
     const bool leaves32 = (reinterpret_cast<uintptr_t>(leaves) & 31) == 0;
-    const uint64_t n = G.g.n;
-    const uint64_t cmax = G.cmax;
+    const I n = (I)G.g.n;
+    const I cmax = (I)G.cmax;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t g = lane % GL, lead = lane - g;
     const unsigned below = (1u << lane) - 1u, below_lead = (1u << lead) - 1u;
@@ -880,13 +931,16 @@ learned_query_group_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, 
     const uint64_t q0 = min(nq, w * per);
     const uint32_t cnt = (uint32_t)(min(nq, q0 + per) - q0);
     uint32_t n_fallback = 0, depth_sum = 0;
-    uint64_t cur = kIdle, key = 0;  // this group's descent: node | flags << kFlagShift
+    I cur = kNone;  // this group's descent: its node and flags
+    uint32_t fl = 0;
+    uint64_t key = 0;
     uint32_t qoff = 0;
-    uint64_t e_cur = 0, e_key = 0;  // this lane's prepared entry of the current batch
+    I e_cur = 0;  // this lane's prepared entry of the current batch
+    uint64_t e_key = 0;
     uint32_t next = 0, batch0 = 0, bn = 0, bpos = 0;
     (void)below;
     for (;;) {
-        unsigned need = __ballot_sync(0xFFFFFFFFu, cur == kIdle) & kLeaders;
+        unsigned need = __ballot_sync(0xFFFFFFFFu, cur == kNone) & kLeaders;
         while (need) {
             if (bpos == bn) {
                 if (next >= cnt) break;
@@ -897,8 +951,13 @@ learned_query_group_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, 
                 if (lane < bn) {
                     e_key = __ldcs(Q + q0 + batch0 + lane);
                     uint32_t f, d;
-                    const uint64_t nd = learned_start<B>(G, p, sp, use_net, leaves, leaves32, e_key, f, d);
-                    e_cur = nd | ((uint64_t)f << kFlagShift);
+                    const tl_rank_leaf lf = load_leaf(leaves, learned_segment(p, sp, use_net, e_key), leaves32);
+                    I nd;
+                    if constexpr (sizeof(I) == 4)
+                        nd = learned_start_at32<B>(G, lf, e_key, f, d);
+                    else
+                        nd = learned_start_at<B>(G, lf, e_key, f, d);
+                    e_cur = nd | (f ? kStart : I(0));
                     if (kStats) {
                         if (f) depth_sum += d; else ++n_fallback;
                     }
@@ -918,26 +977,27 @@ learned_query_group_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, 
             const bool mine = (take >> lead) & 1u;
             const uint32_t src = bpos + __popc(take & below_lead);
             const uint64_t k2 = __shfl_sync(0xFFFFFFFFu, e_key, mine ? src : 0);
-            const uint64_t c2 = __shfl_sync(0xFFFFFFFFu, e_cur, mine ? src : 0);
+            const I c2 = __shfl_sync(0xFFFFFFFFu, e_cur, mine ? src : 0);
             if (mine) {
                 key = k2;
-                cur = c2;
+                cur = c2 & ~kStart;
+                fl = c2 & kStart ? kSubtree : 0;
                 qoff = batch0 + src;
             }
             bpos += __popc(take);
             need &= ~take;
         }
-        if (!__any_sync(0xFFFFFFFFu, cur != kIdle)) break;
-        const bool live = cur != kIdle;
-        const uint64_t node = cur & kNodeMask;
+        if (!__any_sync(0xFFFFFFFFu, cur != kNone)) break;
+        const bool live = cur != kNone;
+        const I node = cur;
         uint32_t lt = 0;
         bool eq = false;
         if (live) {
-            const uint64_t s0 = node + (uint64_t)g * KPL;
-            if (node + B <= n) {
+            const I s0 = node + (I)(g * KPL);
+            if (n - node >= B) {
                 uint64_t v[NL][KPL];
 #pragma unroll
-                for (int j = 0; j < NL; ++j) ldg32(A + s0 + (uint64_t)j * GL * KPL, v[j]);
+                for (int j = 0; j < NL; ++j) ldg32(A + s0 + j * GL * KPL, v[j]);
 #pragma unroll
                 for (int j = 0; j < NL; ++j)
 #pragma unroll
@@ -950,7 +1010,7 @@ learned_query_group_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, 
                 for (int j = 0; j < NL; ++j)
 #pragma unroll
                     for (int e = 0; e < KPL; ++e) {
-                        const uint64_t pos = s0 + (uint64_t)j * GL * KPL + e;
+                        const I pos = s0 + (I)(j * GL * KPL + e);
                         if (pos < n) {
                             const uint64_t c = __ldg(A + pos);
                             lt += c < key;
@@ -963,26 +1023,26 @@ learned_query_group_kernel(const uint64_t *__restrict__ A, const LearnedGeom G, 
         for (int off = GL / 2; off > 0; off >>= 1) lt += __shfl_xor_sync(0xFFFFFFFFu, lt, off);
         const bool hit = ((__ballot_sync(0xFFFFFFFFu, eq) >> lead) & ((1u << GL) - 1)) != 0;
         if (live) {
-            const uint32_t valid = node + B <= n ? (uint32_t)B : (uint32_t)(n - node);
-            uint32_t fl = (uint32_t)(cur >> kFlagShift);
-            uint64_t res = kIdle;
+            const uint32_t valid = n - node >= B ? (uint32_t)B : (uint32_t)(n - node);
+            I res = kNone;
             if (hit) {
                 res = node + lt;
             } else {
                 fl |= (lt > 0 ? kSeenLess : 0u) | (lt < valid ? kSeenGreater : 0u);
-                const uint64_t nx = node + 1 <= cmax ? (node + 1) * (B + 1) + (uint64_t)lt * B - 1 : n;
+                const I nx = node + 1 <= cmax ? (node + 1) * (B + 1) + (I)lt * B - 1 : n;
                 if (nx < n) {
-                    cur = nx | ((uint64_t)fl << kFlagShift);
+                    cur = nx;
                 } else if (!(fl & kSubtree) || ((fl & kSeenLess) && (fl & kSeenGreater))) {
                     res = n;  // absent (from the root; or the subtree straddles the query)
                 } else {      // the window could not decide: plain search from the root
                     if (kStats && g == 0) ++n_fallback;
                     cur = 0;
+                    fl = 0;
                 }
             }
-            if (res != kIdle) {
-                if (g == 0) __stcs(ans + q0 + qoff, res);
-                cur = kIdle;
+            if (res != kNone) {
+                if (g == 0) __stcs(ans + q0 + qoff, (uint64_t)res);
+                cur = kNone;
             }
         }
     }
@@ -1191,6 +1251,7 @@ int query_btree_learned(const uint64_t *A, uint64_t n, uint64_t b, const tl_rank
     LearnedGeom G;
     G.g = make_btree_geom(n, b);
     G.fd = FastDiv64(b + 1);
+    G.fd32 = FastDiv32((uint32_t)(b + 1));
     G.cmax = (n + 1) / (b + 1);
     EventTimer timer(ms != nullptr, st);
     int dev = 0, sms = 148;
@@ -1210,39 +1271,46 @@ int query_btree_learned(const uint64_t *A, uint64_t n, uint64_t b, const tl_rank
         return TL_SUCCESS;
     };
     auto launch = [&](auto kern) -> int { return launch_with(kern, kLearnedThreads); };
-    auto launch_group = [&](auto kern) -> int { return launch_with(kern, kLearnedGroupThreads); };
+    auto launch_group = [&](bool narrow, auto k32, auto k64) -> int {
+        return narrow ? launch_with(k32, kLearnedGroupThreads) : launch_with(k64, kLearnedGroupThreads);
+    };
     // 64-, 128- and 256-byte nodes on a 32-byte aligned layout: a group of
     // lanes per descent; else one lane per descent with 32-byte node loads
     // (32-byte aligned layout, node bytes a multiple of 32) or 16-byte ones
     const bool v32 = (reinterpret_cast<uintptr_t>(A) & 31) == 0 && (b * 8) % 32 == 0;
     const bool grp = v32 && query_variant() != 6;
+    // 32-bit node indices with a flag bit (variant 8: the 64-bit form at any size)
+    const bool narrow = n < (1ull << 31) && query_variant() != 8;
+#define TL_GROUP(NB, GL, ST) \
+    narrow, learned_query_group_kernel<NB, GL, ST, uint32_t>, learned_query_group_kernel<NB, GL, ST, uint64_t>
     int rc;
     switch (b * 8) {
         case 16: rc = launch(learned_query_kernel<16, 16>); break;
         case 32: rc = v32 ? launch(learned_query_kernel<32, 32>) : launch(learned_query_kernel<32, 16>); break;
         case 64:
-            rc = grp   ? (stats ? launch_group(learned_query_group_kernel<64, 2, true>)
-                                : launch_group(learned_query_group_kernel<64, 2, false>))
+            rc = grp   ? (stats ? launch_group(TL_GROUP(64, 2, true))
+                                : launch_group(TL_GROUP(64, 2, false)))
                  : v32 ? launch(learned_query_kernel<64, 32>)
                        : launch(learned_query_kernel<64, 16>);
             break;
         case 128:
             rc = grp && query_variant() == 7
-                     ? (stats ? launch_group(learned_query_group_kernel<128, 4, true>)
-                              : launch_group(learned_query_group_kernel<128, 4, false>))
-                 : grp   ? (stats ? launch_group(learned_query_group_kernel<128, 2, true>)
-                                  : launch_group(learned_query_group_kernel<128, 2, false>))
+                     ? (stats ? launch_group(TL_GROUP(128, 4, true))
+                              : launch_group(TL_GROUP(128, 4, false)))
+                 : grp   ? (stats ? launch_group(TL_GROUP(128, 2, true))
+                                  : launch_group(TL_GROUP(128, 2, false)))
                  : v32 ? launch(learned_query_kernel<128, 32>)
                        : launch(learned_query_kernel<128, 16>);
             break;
         case 256:
-            rc = grp   ? (stats ? launch_group(learned_query_group_kernel<256, 4, true>)
-                                : launch_group(learned_query_group_kernel<256, 4, false>))
+            rc = grp   ? (stats ? launch_group(TL_GROUP(256, 4, true))
+                                : launch_group(TL_GROUP(256, 4, false)))
                  : v32 ? launch(learned_query_kernel<256, 32>)
                        : launch(learned_query_kernel<256, 16>);
             break;
         default: return TL_ERROR_UNSUPPORTED;
     }
+#undef TL_GROUP
     if (rc) return rc;
     timer.stop();
     TL_CUDA_TRY(cudaGetLastError());
