@@ -307,3 +307,44 @@ def test_veb_pieces_with_64_bit_positions():
     hit = ans != n
     assert torch.equal(hit, Q64 < n)
     assert torch.equal(keys[ans[hit]], Q64[hit].to(torch.int32))
+
+
+@pytest.mark.parametrize("kb,b", [(8, 8), (8, 16), (8, 32), (4, 16), (4, 32), (4, 64)])
+def test_btree_top_levels_in_shared_memory(kb, b):
+    """The B-tree form with its top levels in shared memory (variant 9 at any
+    size; the default from 2^20 queries): trees with one level up to several
+    below the top, a partial last leaf, evenly spread and skewed keys (most top
+    keys in one bin), all keys equal in their high bits, queries for every key
+    of the top, below the first, past the last."""
+    import ctypes as C
+
+    import torch
+    L = T.lib()
+    L.tl_debug_set_query_variant.argtypes = [C.c_int]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(b + kb)
+    dt = torch.int64 if kb == 8 else torch.int32
+    for n in [b, b + 1, (b + 1) ** 2 - 1, (b + 1) ** 2 + b // 2, 50_021, 1_000_003]:
+        even = data.sorted_keys_torch(n, 1, 3, n, kb).to(torch.int64)
+        rank = torch.arange(n, device="cuda", dtype=torch.float64)
+        skew = even + (torch.exp2(rank / n * 24 + 6)).to(torch.int64) if kb == 4 else \
+            even + (torch.exp2(rank / n * 60)).to(torch.int64)
+        for keys in (even, skew.clamp_max(2**31 - n) + torch.arange(n, device="cuda") if kb == 4 else skew):
+            tree = keys.to(dt).clone()
+            T.permute("btree", tree, b)
+            Q = torch.cat([tree[:min(n, 5000)].to(torch.int64), keys[torch.randint(0, n, (20_000,), generator=g,
+                                                                                   device="cuda")],
+                           keys[torch.randint(0, n, (20_000,), generator=g, device="cuda")] + 1, keys[:1] - 1,
+                           keys[-1:] + 1, torch.zeros(1, dtype=torch.int64, device="cuda")]).to(dt)
+            got = torch.full((Q.numel(),), -7, dtype=torch.int64, device="cuda")
+            L.tl_debug_set_query_variant(9)
+            try:
+                T.query("btree", tree, Q, got, b)
+            finally:
+                L.tl_debug_set_query_variant(0)
+            _check_answers(tree, keys.to(dt), Q, got)
+    q = (1 << 20) + 77  # the default route
+    Q = keys[torch.randint(0, n, (q,), generator=g, device="cuda")].to(dt) + 1
+    got = torch.full((q,), -7, dtype=torch.int64, device="cuda")
+    T.query("btree", tree, Q, got, b)
+    _check_answers(tree, keys.to(dt), Q, got)

@@ -379,6 +379,146 @@ btree_query_group32_kernel(const K *__restrict__ A, uint64_t n, const K *__restr
     }
 }
 
+// The same read of a node by G lanes, below a top of T whole levels searched in
+// shared memory: their m = (b + 1)^T - 1 keys in sorted order, and kTopBins bins
+// of equal width over their value range holding the first rank of each, so a
+// query finds its rank among them with a bin and a binary search inside it (one
+// or two probes where keys are spread evenly, log2(m) at worst) and starts at
+// the node of level T with that number.
+// What bounds it: each level read from global memory costs a query NL L1
+// wavefronts (two for 128-byte nodes; ncu, 2^24 queries over 1e8 u64 keys, b =
+// 16: L1 data pipe 92 % before and after), a probe of shared memory about a
+// fifth of one, and three of the seven levels there fit 40 KB.  Measured on
+// B200, without and with the top: b = 16 u64, 2^24 queries over 1e8 keys 1068 ->
+// 704 us, over 2^20 keys 751 -> 408, 2^27 over 5e8 9.43 -> 7.5 to 8.4 ms (there
+// the three levels in DRAM, 400 bytes a query, are 8.2 ms of the copy
+// bandwidth); b = 32 u64 over 2^28 keys 1866 -> 1262; b = 8 u64 1024 -> 921; b =
+// 16 u32 over 5e8 keys 899 -> 740.  Ordering the batch by value in chunks first
+// gains nothing here (a level's wavefronts stay, 704 -> 820 us), nor does a
+// thread a query whose nodes four lanes read together (half the wavefronts, 48
+// warps' registers: 1028).  Two blocks of 1024 threads an SM at 32 registers;
+// the wide form of I would not fit, so layouts of 2^31 keys or more keep the
+// kernel above.
+constexpr uint32_t kTopBins = 4096;
+constexpr int kTopThreads = 1024;
+constexpr uint64_t kTopBytes = 40 * 1024;
+
+template <typename K, int NB, int G>
+__global__ void __launch_bounds__(kTopThreads, 2)
+btree_query_top_kernel(const K *__restrict__ A, uint32_t n, uint32_t m, const K *__restrict__ Q, uint64_t nq,
+                       uint64_t *__restrict__ ans) {
+    constexpr uint32_t KPL = 32 / sizeof(K);  // keys per 32-byte load
+    constexpr int NL = NB / 32 / G;           // 32-byte loads per lane and node
+    constexpr uint32_t B = NB / sizeof(K);    // == b
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    K *top = reinterpret_cast<K *>(smem_raw);               // [m]
+    uint16_t *bin = reinterpret_cast<uint16_t *>(top + m);  // [kTopBins + 1]
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t g = lane % G;
+    const uint32_t gshift = lane - g;
+    const uint32_t cmax = (uint32_t)(((uint64_t)n + 1) / (B + 1));
+    // position p of the top: the x-th multiple of mult (x not a multiple of b + 1) on its level
+    for (uint32_t p = threadIdx.x; p < m; p += kTopThreads) {
+        uint32_t end = B + 1, mult = (m + 1) / (B + 1);  // the level's end + 1, its keys' spacing
+        while (p + 1 >= end) {
+            end *= B + 1;
+            mult /= B + 1;
+        }
+        const uint32_t t = p + 1 - end / (B + 1);
+        top[(t + 1 + t / B) * mult - 1] = __ldg(A + p);
+    }
+    __syncthreads();
+    const K first = top[0];
+    const uint32_t span = bit_length((uint64_t)(top[m - 1] - first)), bits = bit_length(kTopBins - 1);
+    const uint32_t shift = span > bits ? span - bits : 0;
+    for (uint32_t r = threadIdx.x; r <= m; r += kTopThreads) {
+        const uint32_t hi = r < m ? (uint32_t)((top[r] - first) >> shift) : kTopBins;
+        for (uint32_t k = r ? (uint32_t)((top[r - 1] - first) >> shift) + 1 : 0; k <= hi; ++k) bin[k] = (uint16_t)r;
+    }
+    __syncthreads();
+    const uint64_t warps = (uint64_t)gridDim.x * (kTopThreads / 32);
+    const uint64_t wid = ((uint64_t)blockIdx.x * kTopThreads + threadIdx.x) / 32;
+    for (uint64_t base = wid * (32 / G); base < nq; base += warps * (32 / G)) {
+        const uint64_t qi = base + lane / G;
+        const bool have = qi < nq;
+        const K q = have ? __ldcs(Q + qi) : K(0);
+        uint32_t r = 0;  // top keys below q
+        if (q >= first) {
+            const K k = (K)(q - first) >> shift;
+            uint32_t r1 = m;
+            r = m;
+            if (k < kTopBins) {
+                r = bin[k];
+                r1 = bin[k + 1];
+            }
+            while (r < r1) {
+                const uint32_t mid = (r + r1) >> 1;
+                if (top[mid] < q)
+                    r = mid + 1;
+                else
+                    r1 = mid;
+            }
+        }
+        uint32_t i = m + r * B, res = n;
+        bool live = have && i < n;
+        if (r < m && top[r] == q) {  // a key of the top: its position there
+            uint32_t x = r + 1, end = m + 1;
+            while (x % (B + 1) == 0) {
+                x /= B + 1;
+                end /= B + 1;
+            }
+            res = end / (B + 1) - 1 + (x - x / (B + 1) - 1);
+            live = false;
+        }
+        while (__any_sync(0xFFFFFFFFu, live)) {
+            uint32_t lt = 0;
+            bool eq = false;
+            if (live) {
+                const uint32_t s0 = i + g * KPL;  // lane g: slots s0 + j * G * KPL + e
+                if (n - i >= B) {
+                    K v[NL][KPL];
+#pragma unroll
+                    for (int j = 0; j < NL; ++j) ldg32(A + s0 + j * G * KPL, v[j]);
+#pragma unroll
+                    for (int j = 0; j < NL; ++j)
+#pragma unroll
+                        for (uint32_t e = 0; e < KPL; ++e) {
+                            lt += v[j][e] < q;
+                            eq |= v[j][e] == q;
+                        }
+                } else {  // the partial last leaf: slots at or past n do not count
+#pragma unroll
+                    for (int j = 0; j < NL; ++j)
+#pragma unroll
+                        for (uint32_t e = 0; e < KPL; ++e) {
+                            const uint32_t p = s0 + j * G * KPL + e;
+                            if (p < n) {
+                                const K cur = __ldg(A + p);
+                                lt += cur < q;
+                                eq |= cur == q;
+                            }
+                        }
+                }
+            }
+#pragma unroll
+            for (int off = G / 2; off > 0; off >>= 1) lt += __shfl_xor_sync(0xFFFFFFFFu, lt, off);
+            const bool hit = ((__ballot_sync(0xFFFFFFFFu, eq) >> gshift) & ((1u << G) - 1)) != 0;
+            if (live) {
+                if (hit) {
+                    res = i + lt;
+                    live = false;
+                } else if (i + 1 > cmax) {
+                    live = false;
+                } else {
+                    i = (i + 1) * (B + 1) + lt * B - 1;
+                    live = i < n;
+                }
+            }
+        }
+        if (g == 0 && have) __stcs(ans + qi, (uint64_t)res);
+    }
+}
+
 static int g_query_variant = 0;
 void set_query_variant(int v) { g_query_variant = v; }
 int query_variant() { return g_query_variant; }
@@ -1209,7 +1349,32 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         // - against 6.54e9; b = 32 u64 over 2^28 keys 8.33e9 / 9.08e9 / 6.06e9
         // against 4.28e9; b = 16 u32 over 2^30 keys 17.7e9 against 11.7e9;
         // b = 8 u64 over 2^30 keys 12.7e9 against 8.56e9
-        if ((base & 31) == 0 && g_query_variant != 2 && g_query_variant != 5 && g_query_variant != 6) {
+        // from 2^20 queries (a block gathers and indexes its top first: over 5e8
+        // u64 keys 2^18 queries 32 / 32 us, 2^19 50 / 49, 2^20 88 / 83; over 2^20
+        // keys 20 / 23, 32 / 31, 54 / 42) the whole top levels that 40 KB hold are
+        // searched in shared memory (10 KB, two levels at b = 16: 838 against 702
+        // us over 1e8 keys).  Variant 9 takes this form at any size.
+        uint64_t m = 0;
+        for (uint64_t t = a.b; t <= a.n && t * sizeof(K) <= kTopBytes; t = t * (a.b + 1) + a.b) m = t;
+        auto topped = [&](auto kern, uint64_t lanes_per_query) -> int {
+            const size_t bytes = m * sizeof(K) + (kTopBins + 1) * sizeof(uint16_t);
+            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+            const uint64_t need = (a.q * lanes_per_query + kTopThreads - 1) / kTopThreads;
+            kern<<<(unsigned)std::min<uint64_t>(2 * (uint64_t)query_sm_count(), need), kTopThreads, bytes, st>>>(
+                A, (uint32_t)a.n, (uint32_t)m, Q, a.q, a.answers);
+            done = true;
+            return TL_SUCCESS;
+        };
+        if ((base & 31) == 0 && m && a.n < (1ull << 31) &&
+            (g_query_variant == 9 || (g_query_variant == 0 && a.q >= (1ull << 20)))) {
+            switch (node_bytes) {
+                case 64: rc = topped(btree_query_top_kernel<K, 64, 2>, 2); break;
+                case 128: rc = topped(btree_query_top_kernel<K, 128, 2>, 2); break;
+                case 256: rc = topped(btree_query_top_kernel<K, 256, 4>, 4); break;
+                default: break;
+            }
+        }
+        if (!done && (base & 31) == 0 && g_query_variant != 2 && g_query_variant != 5 && g_query_variant != 6) {
             if (g_query_variant == 7) {  // one 32-byte load per lane
                 switch (node_bytes) {
                     case 128: rc = grp(btree_query_group32_kernel<K, 128, 4>, 4); break;
