@@ -64,3 +64,43 @@ def test_full_size_round_trip(layout, b, n, kb, gap):
     assert not torch.equal(t, keys)
     T.unpermute(layout, t, b)
     assert torch.equal(t, keys)
+
+
+@pytest.mark.parametrize("layout,b,n,kb,skip", [
+    # either side of each form's line (8, 32, 192 MB), ragged sizes, arrays that
+    # start off a 16- or 128-byte boundary (no vector stores, shifted stretches)
+    ("btree", 16, (8 << 17) - 1, 8, 1), ("btree", 16, (8 << 17) + 1, 8, 0), ("btree", 3, 2_100_001, 4, 3),
+    ("btree", 16, 25_165_824, 8, 0), ("btree", 16, 25_165_825, 8, 1), ("btree", 2, 60_000_001, 4, 5),
+    ("btree", 1000, 30_000_001, 8, 3), ("btree", 100_000, 50_331_777, 4, 1),
+    ("bst", 1, 2**25 + 5, 8, 1), ("bst", 1, 2**26 - 1, 8, 0), ("bst", 1, 3 * 2**25 + 1, 8, 1),
+    ("mveb", 0, 2**22, 8, 1), ("mveb", 0, 2**22 + 1, 8, 0), ("mveb", 0, 2**23 - 1, 8, 1), ("mveb", 0, 2**24 + 7, 4, 3),
+    ("veb", 0, 2**23 + 1, 4, 1), ("veb", 0, 2**19 - 1, 8, 1), ("veb", 0, 12_345_679, 8, 1), ("veb", 0, 2**25 - 1, 4, 0),
+])
+def test_reverse_forms_round_trip(layout, b, n, kb, skip):
+    import torch
+    keys = data.sorted_keys_torch(n, 1, 3, 5, kb)
+    buf = torch.full((n + skip + 64,), -1, dtype=keys.dtype, device="cuda")
+    t = buf[skip:skip + n]
+    t.copy_(keys)
+    T.permute(layout, t, b or 16)
+    T.unpermute(layout, t, b or 16)
+    assert torch.equal(t, keys)
+    assert bool((buf[:skip] == -1).all()) and bool((buf[skip + n:] == -1).all())
+
+
+def test_expired_reverse_wait_reports_timeout_and_context_survives():
+    import torch
+    n = 30_000_001
+    keys = data.sorted_keys_torch(n, 1, 16, 9, 8)
+    t = keys.clone()
+    T.permute("btree", t, 16)
+    lay = t.clone()
+    T.set_wait(spin_limit=64, force_timeout=True)
+    try:
+        with pytest.raises(T.TreeLayoutError) as e:
+            T.unpermute("btree", t, 16)
+        assert e.value.status == T.ERROR_TIMEOUT
+    finally:
+        T.set_wait(0, False)
+    T.unpermute("btree", lay, 16)
+    assert torch.equal(lay, keys)

@@ -89,56 +89,6 @@ btree_fix_kernel(K *__restrict__ A, const K *__restrict__ scr, const FixSeg *__r
     }
 }
 
-// One copy range for the bulk engine: its 16-byte-aligned interior in
-// kBulkChunk pieces, its ragged keys apart.  The scratch shares A's offset
-// within 16 bytes at both range bases, so the interiors line up.
-template <typename K>
-static int add_bulk_range(const K *A, const K *scr, const CopyRange &r, BulkPlan &P) {
-    if (P.nr == kMaxBulkRanges) return TL_ERROR_UNSUPPORTED;
-    const uintptr_t da = reinterpret_cast<uintptr_t>(A + r.dst), sa = reinterpret_cast<uintptr_t>(scr + r.src);
-    if ((da ^ sa) & 15) return TL_ERROR_INVALID_VALUE;
-    BulkRange R{};
-    R.key_dst = r.dst;
-    R.key_src = r.src;
-    R.len = r.len;
-    const uint64_t head = std::min<uint64_t>(((16 - (da & 15)) & 15) / sizeof(K), r.len);
-    const uint64_t body = ((r.len - head) * sizeof(K)) & ~15ull;
-    R.head = (uint32_t)head;
-    R.tail = (uint32_t)(r.len - head - body / sizeof(K));
-    R.dst = (r.dst + head) * sizeof(K);
-    R.src = (r.src + head) * sizeof(K);
-    R.bytes = body;
-    R.chunk0 = P.nchunks;
-    P.nchunks += (body + kBulkChunk - 1) / kBulkChunk;
-    P.r[P.nr++] = R;
-    return TL_SUCCESS;
-}
-
-// The copy ranges of a plan: per level (plans R, L), or the runs of whole
-// scratch tiles (plan O: tiles [x, y) from scratch slot z on).
-template <typename K>
-static int make_bulk_plan(const BtreeStream &S, const OrderTables &ot, const K *A, const K *scr, BulkPlan &P) {
-    P.nr = 0;
-    P.nchunks = 0;
-    if (S.plan == PLAN_O) {
-        for (uint64_t i = 0; i < ot.nranges; ++i) {
-            const uint64_t u0 = ot.ranges[i].x, u1 = ot.ranges[i].y;
-            const uint64_t d0 = u0 << S.tile_shift, d1 = std::min<uint64_t>(u1 << S.tile_shift, S.g.n);
-            const uint64_t s0 = (uint64_t)ot.ranges[i].z << S.tile_shift;  // host data: S.tab may be device memory
-            const int rc = add_bulk_range(A, scr, CopyRange{d0, s0, d1 - d0}, P);
-            if (rc) return rc;
-        }
-        return TL_SUCCESS;
-    }
-    for (int j = 0; j < btree_copy_range_count(S); ++j) {
-        CopyRange r;
-        if (!btree_copy_range(S, j, r)) continue;
-        const int rc = add_bulk_range(A, scr, r, P);
-        if (rc) return rc;
-    }
-    return TL_SUCCESS;
-}
-
 // ---------------------------------------------------------------- mvEB stream
 template <typename K>
 __global__ void __launch_bounds__(kStreamThreads, kStreamBlocksPerSM)
@@ -250,18 +200,6 @@ mveb_scatter_kernel(K *__restrict__ A, const K *__restrict__ scr, const __grid_c
 }
 
 // ---------------------------------------------------------------- host side
-struct PermutePlan {
-    int layout = 0;
-    uint32_t key_bytes = 8;
-    uint64_t n = 0, b = 1;
-    uint64_t tile_keys = 0, ntiles = 0, scratch_keys = 0;
-    bool ordered = false;  // B-tree plan O, with these tables (host, then device pointers)
-    OrderTables ot;
-    BtreeStream bs;
-    MvebParams mp;
-    uint64_t off_flags = 0, off_ctrl = 0, bytes = 0;
-};
-
 // When a B-tree permutation takes plan O: ORDER_AUTO from kOrderMinTiles tiles
 // up (below that a tile order has too few tiles to pay for its second pass),
 // for a BST from kOrderMinTilesBst (measured on B200, u64 keys: at 2^20 - 1
@@ -465,20 +403,6 @@ int stream_blocks_per_sm(int layout, uint32_t key_bytes) {
               : blocks_per_sm_of(btree_stream_kernel<uint32_t, false>, smem);
 }
 
-int permute_geometry(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, PermuteGeometry &geo) {
-    PermutePlan pl;
-    const int rc = make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
-    if (rc) return rc;
-    geo.layout = pl.layout;
-    geo.key_bytes = pl.key_bytes;
-    geo.n = pl.n;
-    geo.tile_keys = pl.tile_keys;
-    geo.ntiles = pl.ntiles;
-    geo.bs = pl.bs;
-    geo.mp = pl.mp;
-    return TL_SUCCESS;
-}
-
 int permute_plan_of(int layout, uint64_t n, uint64_t b, uint32_t key_bytes) {
     PermutePlan pl;
     const int rc = make_plan(layout, n, b, key_bytes, pl);
@@ -533,13 +457,8 @@ int permute_workspace_bytes_fixed(int layout, uint64_t n, uint64_t b, uint32_t k
     return TL_SUCCESS;
 }
 
-int permute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes, void *dev_ws,
-            uint64_t ws_bytes, cudaStream_t st, float *ms, float *phase_ms, bool allow_ordered) {
-    if (n > 0 && !dev_A) return TL_ERROR_INVALID_VALUE;
-    if (reinterpret_cast<uintptr_t>(dev_A) % (key_bytes ? key_bytes : 1)) return TL_ERROR_INVALID_VALUE;
-    if (dev_ws && reinterpret_cast<uintptr_t>(dev_ws) % 256) return TL_ERROR_INVALID_VALUE;
-    PermutePlan pl;
-    if (allow_ordered && n > 1 && !is_veb_layout(layout)) {
+int permute_plan_device(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, cudaStream_t st, PermutePlan &pl) {
+    if (n > 1 && !is_veb_layout(layout)) {
         // a geometry not seen before: its ordered-tile tables with kernels on
         // st (make_plan below finds them cached; if this cannot be done it
         // computes them on the host)
@@ -547,24 +466,47 @@ int permute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes,
         if (make_plan(layout, n, b, key_bytes, fx, ORDER_NEVER) == TL_SUCCESS && order_wanted(fx, ORDER_AUTO))
             btree_order_prepare(fx.bs, st);
     }
-    int rc = make_plan(layout, n, b, key_bytes, pl, allow_ordered ? ORDER_AUTO : ORDER_NEVER);
+    const int rc = make_plan(layout, n, b, key_bytes, pl, ORDER_AUTO);
+    if (rc || n <= 1 || !pl.ordered) return rc;
+    // plan O needs its tile tables on the device; without them, the
+    // fixed-direction plan
+    OrderTables dt;
+    if (!btree_order_device(pl.bs, st, dt)) {
+        pl = PermutePlan{};
+        return make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
+    }
+    pl.ot = dt;
+    pl.bs.tab = dt.tab;
+    pl.bs.order = dt.order;
+    return TL_SUCCESS;
+}
+
+int permute_plan_replay(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, bool ordered, OrderVectors &ov,
+                        PermutePlan &pl) {
+    const int rc = make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
+    if (rc || !ordered || is_veb_layout(layout)) return rc;
+    btree_compute_order(pl.bs, ov);  // computed here, not taken from the library's cache
+    const OrderTables ot = ov.tables();
+    return make_plan(layout, n, b, key_bytes, pl, ORDER_ALWAYS, &ot);
+}
+
+int permute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes, void *dev_ws,
+            uint64_t ws_bytes, cudaStream_t st, float *ms, float *phase_ms, bool allow_ordered) {
+    if (n > 0 && !dev_A) return TL_ERROR_INVALID_VALUE;
+    if (reinterpret_cast<uintptr_t>(dev_A) % (key_bytes ? key_bytes : 1)) return TL_ERROR_INVALID_VALUE;
+    if (dev_ws && reinterpret_cast<uintptr_t>(dev_ws) % 256) return TL_ERROR_INVALID_VALUE;
+    PermutePlan pl;
+    int rc = allow_ordered ? permute_plan_device(layout, n, b, key_bytes, st, pl)
+                           : make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
     if (rc) return rc;
     if (n <= 1) {
         if (ms) *ms = 0.f;
         return TL_SUCCESS;
     }
-    // plan O needs its tile tables on the device and a scratch over every
-    // position; without either, the fixed-direction plan
-    if (pl.ordered) {
-        OrderTables dt;
-        if ((dev_ws && ws_bytes < pl.bytes) || !btree_order_device(pl.bs, st, dt)) {
-            rc = make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
-            if (rc) return rc;
-        } else {
-            pl.ot = dt;
-            pl.bs.tab = dt.tab;
-            pl.bs.order = dt.order;
-        }
+    if (pl.ordered && dev_ws && ws_bytes < pl.bytes) {  // the fixed-direction plan may fit
+        pl = PermutePlan{};
+        rc = make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
+        if (rc) return rc;
     }
     if (dev_ws && ws_bytes < pl.bytes) return TL_ERROR_WORKSPACE_TOO_SMALL;
     EventTimer timer(ms != nullptr || phase_ms != nullptr, st);
@@ -648,15 +590,9 @@ int debug_order_tables_match(int layout, uint64_t n, uint64_t b, uint32_t key_by
 static int emulate_permute_kb(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, uint64_t *A,
                               uint64_t *violations, int order_mode) {
     PermutePlan pl;
-    int rc = make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
+    OrderVectors ov;
+    const int rc = permute_plan_replay(layout, n, b, key_bytes, order_mode != ORDER_NEVER, ov, pl);
     if (rc) return rc;
-    OrderVectors ov;  // computed here, not taken from the library's cache
-    if (order_mode != ORDER_NEVER && !is_veb_layout(layout)) {
-        btree_compute_order(pl.bs, ov);
-        const OrderTables ot = ov.tables();
-        rc = make_plan(layout, n, b, key_bytes, pl, order_mode, &ot);
-        if (rc) return rc;
-    }
     // tile kk's ticket precedes (or is) tile k's
     auto earlier = [&](uint64_t kk, uint64_t k) {
         if (pl.ordered) return btree_o_rank(pl.bs, kk) <= btree_o_rank(pl.bs, k);
