@@ -139,3 +139,26 @@ def test_ordered_tables_gpu_build_equals_host_build(layout, b, n, kb):
     L = T.lib()
     L.tl_debug_order_tables_match.argtypes = [C.c_int, C.c_uint64, C.c_uint64, C.c_uint32, C.c_void_p]
     assert L.tl_debug_order_tables_match(T.LAYOUTS[layout], n, b, kb, None) == 1, (layout, b, n, kb)
+
+
+@pytest.mark.parametrize("layout,b", [("bst", 1), ("btree", 2), ("btree", 8), ("btree", 16), ("btree", 5000)])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+def test_small_arrays_key_by_key_and_by_tiles(layout, b, dtype):
+    """B-trees and BSTs of up to 12 MB are moved key by key; with a caller's
+    workspace too small for a copy of the array they keep the tiled form.  Both
+    equal the oracle, on either side of the line and off 16-byte boundaries."""
+    import torch
+    kb = np.dtype(dtype).itemsize
+    line = (12 << 20) // kb
+    for n in [2, 3, 255, 4097, 100_003, 1_000_003, line, line + 1]:
+        keys = data.sorted_keys_np(n, 1, 3, n, dtype)
+        exp = O.permute(layout, keys, b)
+        for skip in (0, 1, 3):
+            buf = to_dev(np.concatenate([np.zeros(skip, dtype), keys]))
+            T.permute(layout, buf[skip:], b)
+            assert np.array_equal(from_dev(buf)[skip:], exp), (layout, b, n, skip)
+        need = T.workspace_bytes(layout, n, b, kb)
+        if need < n * kb:
+            t = to_dev(keys)
+            T.permute(layout, t, b, workspace=torch.empty(need, dtype=torch.uint8, device="cuda"))
+            assert np.array_equal(from_dev(t), exp), (layout, b, n, "tiles")

@@ -37,13 +37,17 @@ int read_error_word(const unsigned int *dev_word, unsigned int *out, cudaStream_
 // Wait statistics of the last permutation (test and profiling hook).
 static std::atomic<unsigned long long> g_stalled_waits{0}, g_stall_polls{0};
 
-void record_wait_stats(const Ctrl *ctrl, cudaStream_t st) {
-    unsigned long long v[2] = {0, 0};
-    if (cudaMemcpyAsync(v, &ctrl->stalled_waits, sizeof v, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return;
-    g_stalled_waits = v[0];
-    g_stall_polls = v[1];
+int read_ctrl(const Ctrl *dev_ctrl, unsigned int *error, cudaStream_t st) {
+    Ctrl c{};
+    if (dev_ctrl) {
+        // pageable destination: the copy has completed when cudaMemcpyAsync returns
+        TL_CUDA_TRY(cudaMemcpyAsync(&c, dev_ctrl, sizeof c, cudaMemcpyDeviceToHost, st));
+        TL_CUDA_TRY(cudaStreamSynchronize(st));
+    }
+    *error = c.error;
+    g_stalled_waits = c.stalled_waits;
+    g_stall_polls = c.stall_polls;
+    return TL_SUCCESS;
 }
 
 int sync_and_check(cudaStream_t st) {

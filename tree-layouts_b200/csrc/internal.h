@@ -91,8 +91,10 @@ void workspace_release(void *p);
 void keep_pool_memory();
 int sync_and_check(cudaStream_t st);
 struct Ctrl;
-// Keeps the wait statistics of a permutation's control block (tl_debug_wait_stats).
-void record_wait_stats(const Ctrl *ctrl, cudaStream_t st);
+// Reads back a permutation's control block in one copy (blocks the host): its
+// error word, and its wait statistics for tl_debug_wait_stats.  Without one (a
+// permutation that never waits) the statistics are zero.
+int read_ctrl(const Ctrl *dev_ctrl, unsigned int *error, cudaStream_t st);
 
 int permute_workspace_bytes(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, uint64_t *bytes);
 // The workspace of the fixed-direction schedules (what permute needs when told

@@ -89,6 +89,14 @@ btree_fix_kernel(K *__restrict__ A, const K *__restrict__ scr, const FixSeg *__r
     }
 }
 
+// Small arrays (permute_by_keys): every key of the copy C to its position.
+template <typename K>
+__global__ void __launch_bounds__(256)
+btree_scatter_keys_kernel(K *__restrict__ A, const K *__restrict__ C, uint64_t n, const __grid_constant__ KeysGeometry kg) {
+    const uint64_t x = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    if (x < n) A[btree_pos(kg.g, kg.fd, x)] = C[x];
+}
+
 // ---------------------------------------------------------------- mvEB stream
 template <typename K>
 __global__ void __launch_bounds__(kStreamThreads, kStreamBlocksPerSM)
@@ -490,14 +498,38 @@ int permute_plan_replay(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, 
     return make_plan(layout, n, b, key_bytes, pl, ORDER_ALWAYS, &ot);
 }
 
+bool permute_by_keys(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, KeysGeometry &kg) {
+    if (layout == TL_LAYOUT_BST) b = 1;
+    else if (layout != TL_LAYOUT_BTREE) return false;
+    if ((key_bytes != 4 && key_bytes != 8) || b == 0 || b >= (1ull << 31)) return false;  // make_plan's refusals
+    if (n <= 1 || n > kKeysBytes / key_bytes) return false;
+    kg.g = make_btree_geom(n, b);
+    kg.fd = FastDiv64(b + 1);
+    return true;
+}
+
+template <typename K>
+static int launch_by_keys(const KeysGeometry &kg, K *A, char *ws, uint64_t n, cudaStream_t st, EventTimer &timer) {
+    K *C = reinterpret_cast<K *>(ws);
+    TL_CUDA_TRY(cudaMemcpyAsync(C, A, n * sizeof(K), cudaMemcpyDeviceToDevice, st));
+    timer.mid();
+    btree_scatter_keys_kernel<K><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, C, n, kg);
+    TL_CUDA_TRY(cudaGetLastError());
+    g_last_launches = 1;
+    return TL_SUCCESS;
+}
+
 int permute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes, void *dev_ws,
             uint64_t ws_bytes, cudaStream_t st, float *ms, float *phase_ms, bool allow_ordered) {
     if (n > 0 && !dev_A) return TL_ERROR_INVALID_VALUE;
     if (reinterpret_cast<uintptr_t>(dev_A) % (key_bytes ? key_bytes : 1)) return TL_ERROR_INVALID_VALUE;
     if (dev_ws && reinterpret_cast<uintptr_t>(dev_ws) % 256) return TL_ERROR_INVALID_VALUE;
+    KeysGeometry kg;
+    const bool by_keys = permute_by_keys(layout, n, b, key_bytes, kg) && (!dev_ws || ws_bytes >= n * key_bytes);
     PermutePlan pl;
-    int rc = allow_ordered ? permute_plan_device(layout, n, b, key_bytes, st, pl)
-                           : make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
+    int rc = by_keys         ? TL_SUCCESS
+             : allow_ordered ? permute_plan_device(layout, n, b, key_bytes, st, pl)
+                             : make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
     if (rc) return rc;
     if (n <= 1) {
         if (ms) *ms = 0.f;
@@ -508,18 +540,19 @@ int permute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes,
         rc = make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
         if (rc) return rc;
     }
-    if (dev_ws && ws_bytes < pl.bytes) return TL_ERROR_WORKSPACE_TOO_SMALL;
+    const uint64_t need = by_keys ? n * key_bytes : pl.bytes;
+    if (dev_ws && ws_bytes < need) return TL_ERROR_WORKSPACE_TOO_SMALL;
     EventTimer timer(ms != nullptr || phase_ms != nullptr, st);
     char *ws = static_cast<char *>(dev_ws);
     bool owned = false;
     bool pooled = false;
     if (!ws) {
-        ws = static_cast<char *>(workspace_acquire(pl.bytes));
+        ws = static_cast<char *>(workspace_acquire(need));
         if (ws) {
             owned = true;
         } else {  // the cache could not help: a stream-ordered allocation
             keep_pool_memory();
-            if (cudaMallocAsync(reinterpret_cast<void **>(&ws), pl.bytes, st) != cudaSuccess) {
+            if (cudaMallocAsync(reinterpret_cast<void **>(&ws), need, st) != cudaSuccess) {
                 record_cuda_error(cudaGetLastError());
                 return TL_ERROR_OUT_OF_MEMORY;
             }
@@ -527,15 +560,16 @@ int permute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes,
         }
     }
     timer.start();
-    rc = key_bytes == 8 ? launch_permute<uint64_t>(pl, static_cast<uint64_t *>(dev_A), ws, st, timer)
-                        : launch_permute<uint32_t>(pl, static_cast<uint32_t *>(dev_A), ws, st, timer);
+    if (by_keys)
+        rc = key_bytes == 8 ? launch_by_keys(kg, static_cast<uint64_t *>(dev_A), ws, n, st, timer)
+                            : launch_by_keys(kg, static_cast<uint32_t *>(dev_A), ws, n, st, timer);
+    else
+        rc = key_bytes == 8 ? launch_permute<uint64_t>(pl, static_cast<uint64_t *>(dev_A), ws, st, timer)
+                            : launch_permute<uint32_t>(pl, static_cast<uint32_t *>(dev_A), ws, st, timer);
     timer.stop();
     unsigned int err = 0;
-    if (rc == TL_SUCCESS) {
-        Ctrl *ctrl = reinterpret_cast<Ctrl *>(ws + pl.off_ctrl);
-        rc = read_error_word(&ctrl->error, &err, st);
-        if (rc == TL_SUCCESS) record_wait_stats(ctrl, st);
-    }
+    if (rc == TL_SUCCESS)
+        rc = read_ctrl(by_keys ? nullptr : reinterpret_cast<const Ctrl *>(ws + pl.off_ctrl), &err, st);
     if (owned && pooled) cudaFreeAsync(ws, st);
     if (rc == TL_SUCCESS) rc = sync_and_check(st);
     if (owned && !pooled) {

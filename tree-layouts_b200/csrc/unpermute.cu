@@ -22,7 +22,7 @@
 // Traffic is 2 n w (1 + f), f the forward scratch fraction, where a copy of the
 // layout and a gather from the copy take 4 n w.  Measured on B200, copy and gather
 // as it was (one load a thread at a time) against this: B-tree b = 8 over 6e7 u64
-// keys 371 -> 231 us, b = 16 over 5e8 2.97 -> 1.41 ms (5.66 TB/s of 2 n w), mvEB
+// keys 371 -> 220 us, b = 16 over 5e8 2.97 -> 1.41 ms (5.66 TB/s of 2 n w), mvEB
 // over 3e8 u32 keys 969 -> 468 us, over 2^30 - 1 3.37 -> 1.70 ms, standard vEB
 // over 3e8 984 -> 517 us, BST over 2^28 - 1 u64 1.87 -> 1.13 ms.  Smaller arrays,
 // which stay in L2, go back from a copy in two launches without waits
@@ -237,6 +237,51 @@ static inline uint64_t btree_gather_keys(uint64_t tile_keys, uint64_t b, uint32_
     return std::max(bulk + tops + tops / 32 + 2, tile_keys + tile_keys / 32 + 2);
 }
 
+// The bulk keys of a boundary tile into the tile buffer, by warps 1..: four a
+// thread at a time; a load has returned once its key is in shared memory, and a
+// warp then takes off the layout keys it read, a subtraction a tile.  (Out of
+// line: its state would spill the common path's registers; 1.41 -> 1.67 ms on
+// the 5e8-key B-tree.)
+template <typename K, bool kCopy>
+static __device__ __noinline__ void gather_boundary(const BtreeStream &S, const K *src, const K *scr, K *sm, uint64_t p0,
+                                                    uint32_t cnt, Ctrl *ctrl, unsigned int *rem, int *ok) {
+    const uint32_t tb = threadIdx.x - 32, nb = blockDim.x - 32, lane = tb & 31u;
+    for (uint32_t b0 = tb & ~31u; b0 < cnt; b0 += 4 * nb) {
+        uint64_t idx[4];
+        K v[4];
+        uint32_t how[4];  // 1 layout, 2 scratch
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const uint32_t o = b0 + x * nb + lane;
+            how[x] = 0;
+            if (o >= cnt || btree_is_top(S, p0 + o)) continue;
+            if (kCopy) {
+                how[x] = 1;
+                v[x] = src[btree_pos(S.g, S.fd, p0 + o)];
+            } else {
+                how[x] = btree_place(S, p0 + o, idx[x]) ? 1 : 2;
+                if (how[x] == 2 && idx[x] >= S.nscratch) {
+                    btree_o_bad(ctrl);
+                    *ok = 0;
+                    how[x] = 0;
+                }
+                if (how[x]) v[x] = (how[x] == 1 ? src : scr)[idx[x]];
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            if (how[x]) sm[gskew(b0 + x * nb + lane)] = v[x];
+            if (kCopy) continue;
+            const unsigned act = __ballot_sync(0xFFFFFFFFu, how[x] == 1);
+            if (how[x] == 1) {
+                const uint32_t u = (uint32_t)(idx[x] >> S.tile_shift);
+                const unsigned same = __match_any_sync(act, u);
+                if ((int)lane == __ffs(same) - 1) atomicSub(&rem[u], (unsigned)__popc(same));
+            }
+        }
+    }
+}
+
 // The tile loop: tickets, or (kCopy) a grid stride.
 template <bool kCopy>
 __device__ __forceinline__ unsigned long long first_tile(Ctrl *ctrl, unsigned long long *s_ticket) {
@@ -259,16 +304,21 @@ __device__ __forceinline__ unsigned long long next_tile(unsigned long long t, co
 // while the top keys come run by run into slots of their own; the tile is put
 // together as it is written, 16 bytes a thread.  Boundary tiles and the tail
 // under the right-to-left schedule are gathered in order, key by key.
-// kCopy: every key comes from a copy of the layout (src == scr, the
+// kCopy: every key comes from a copy of the layout (scr, under the
 // left-to-right schedule with every scratch slot at its final position), in any
 // tile order, with nothing to count or wait for.
-template <typename K, bool kCopy>
-__global__ void __launch_bounds__(kGatherThreads, kGatherBlocksPerSM)
-btree_unstream_kernel(K *A, const K *src, const K *__restrict__ scr, const __grid_constant__ BtreeStream S,
+// kTops: top keys a thread loads at a time.  Where they are a ninth of the keys or
+// more (b <= 8), four at 5 blocks an SM (48 registers): b = 8 over 6e7 u64 keys 220
+// us against 226 with one at 6 blocks, b = 3 over 2^27 509 / 528, BST over 2^28 - 1
+// 1126 / 1214; above, one at 6 blocks: b = 16 over 5e8 1403 against 1491 us.
+template <typename K, bool kCopy, int kTops>
+__global__ void __launch_bounds__(kGatherThreads, kTops == 1 ? kGatherBlocksPerSM : kGatherBlocksPerSM - 1)
+btree_unstream_kernel(K *__restrict__ A, const K *__restrict__ scr, const __grid_constant__ BtreeStream S,
                       uint32_t top_at, Ctrl *ctrl, WaitCfg wc, unsigned int *rem) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K *sm = tile_smem<K>(smem_raw);
     K *top = sm + top_at;
+    const K *src = kCopy ? scr : A;  // where the layout is read
     __shared__ unsigned long long s_ticket;
     __shared__ GatherShared gs;
     __shared__ uint32_t s_stage[2];  // the staged stretch: its offset in the buffer, its first index - dbase
@@ -328,45 +378,7 @@ btree_unstream_kernel(K *A, const K *src, const K *__restrict__ scr, const __gri
                 }
             } else {
                 if (tb == 0) gs.bulk = ReadPart{0, 0, 0};
-                if (R.kind == 0) {
-                    // key by key, four a thread at a time; a load has returned
-                    // once its key is in shared memory, and a warp then takes
-                    // off the layout keys it read, a subtraction a tile
-                    for (uint32_t b0 = tb & ~31u; b0 < cnt; b0 += 4 * nb) {
-                        uint64_t idx[4];
-                        K v[4];
-                        uint32_t how[4];  // 1 layout, 2 scratch
-#pragma unroll
-                        for (int x = 0; x < 4; ++x) {
-                            const uint32_t o = b0 + x * nb + (tb & 31u);
-                            how[x] = 0;
-                            if (kCopy) {
-                                if (o < cnt && !btree_is_top(S, p0 + o)) {
-                                    how[x] = 1;
-                                    v[x] = src[btree_pos(S.g, S.fd, p0 + o)];
-                                }
-                            } else if (o < cnt && !btree_is_top(S, p0 + o)) {
-                                how[x] = btree_place(S, p0 + o, idx[x]) ? 1 : 2;
-                                if (how[x] == 2 && idx[x] >= S.nscratch) {
-                                    btree_o_bad(ctrl);
-                                    gs.ok1 = 0;
-                                    how[x] = 0;
-                                }
-                                if (how[x]) v[x] = (how[x] == 1 ? src : scr)[idx[x]];
-                            }
-                        }
-#pragma unroll
-                        for (int x = 0; x < 4; ++x) {
-                            if (how[x]) sm[gskew(b0 + x * nb + (tb & 31u))] = v[x];
-                            const unsigned act = __ballot_sync(0xFFFFFFFFu, how[x] == 1);
-                            if (!kCopy && how[x] == 1) {
-                                const uint32_t u = (uint32_t)(idx[x] >> S.tile_shift);
-                                const unsigned same = __match_any_sync(act, u);
-                                if ((int)(tb & 31u) == __ffs(same) - 1) atomicSub(&rem[u], (unsigned)__popc(same));
-                            }
-                        }
-                    }
-                }
+                if (R.kind == 0) gather_boundary<K, kCopy>(S, src, scr, sm, p0, cnt, ctrl, rem, &gs.ok1);
             }
         }
         __syncthreads();  // the runs and the regime are known
@@ -376,12 +388,11 @@ btree_unstream_kernel(K *A, const K *src, const K *__restrict__ scr, const __gri
         if (gs.ok && gs.ok1) {
             const uint32_t total = gs.cum[gs.nslots];
             uint32_t r = 0;  // the run of gi only moves forward as gi grows
-            for (uint32_t g0 = threadIdx.x; g0 < total; g0 += 2 * kGatherThreads) {
-                // two keys a thread at a time: their loads in flight together
-                K v[2];
-                uint32_t at[2];
+            for (uint32_t g0 = threadIdx.x; g0 < total; g0 += kTops * kGatherThreads) {
+                K v[kTops];
+                uint32_t at[kTops];
 #pragma unroll
-                for (int x = 0; x < 2; ++x) {
+                for (int x = 0; x < kTops; ++x) {
                     const uint32_t gi = g0 + x * kGatherThreads;
                     if (gi < total) {
                         while (gi >= gs.cum[r + 1]) ++r;
@@ -393,7 +404,7 @@ btree_unstream_kernel(K *A, const K *src, const K *__restrict__ scr, const __gri
                     }
                 }
 #pragma unroll
-                for (int x = 0; x < 2; ++x)
+                for (int x = 0; x < kTops; ++x)
                     if (g0 + x * kGatherThreads < total) sm[at[x]] = v[x];
             }
         }
@@ -471,10 +482,11 @@ static inline uint64_t mveb_gather_keys(uint64_t tile_keys) {
 
 template <typename K, bool kCopy>
 __global__ void __launch_bounds__(kGatherThreads, kGatherBlocksPerSM)
-mveb_unstream_kernel(K *A, const K *src, const K *__restrict__ scr, const __grid_constant__ MvebParams prm, Ctrl *ctrl,
+mveb_unstream_kernel(K *__restrict__ A, const K *__restrict__ scr, const __grid_constant__ MvebParams prm, Ctrl *ctrl,
                      WaitCfg wc, unsigned int *rem) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K *sm = tile_smem<K>(smem_raw);
+    const K *src = kCopy ? scr : A;  // where the layout is read
     __shared__ unsigned long long s_ticket;
     __shared__ unsigned long long s_from[kGatherStretches];
     __shared__ uint32_t s_at[kGatherStretches], s_len[kGatherStretches], s_n;
@@ -613,9 +625,9 @@ mveb_unstream_kernel(K *A, const K *src, const K *__restrict__ scr, const __grid
 // B-trees and BSTs of a few megabytes: a thread a key from the copy.
 template <typename K>
 __global__ void __launch_bounds__(kGatherThreads)
-btree_gather_keys_kernel(K *__restrict__ A, const K *__restrict__ C, uint64_t n, const __grid_constant__ BtreeStream S) {
+btree_gather_keys_kernel(K *__restrict__ A, const K *__restrict__ C, uint64_t n, const __grid_constant__ KeysGeometry kg) {
     const uint64_t x = (uint64_t)blockIdx.x * kGatherThreads + threadIdx.x;
-    if (x < n) A[x] = __ldg(C + btree_pos(S.g, S.fd, x));
+    if (x < n) A[x] = __ldg(C + btree_pos(kg.g, kg.fd, x));
 }
 
 // ---------------------------------------------------------------- host side
@@ -629,6 +641,7 @@ static inline uint64_t align256(uint64_t x) { return (x + 255) / 256 * 256; }
 // 252 / 214 / 219 on the fixed directions (39 % of its keys take scratch), 2 GB
 // on the ordered schedule 1129 in place; mvEB u64 from a copy / in place: 16 MB 23
 // / 26, 32 MB 35 / 33, 64 MB 55 / 44, 128 MB 95 / 64.
+// (Key by key: permute_by_keys, decided before there is a plan.)
 enum ReverseForm { REVERSE_KEYS, REVERSE_COPY, REVERSE_IN_PLACE };
 // Workspace of the in-place form: the scratch (starting at the array's own offset
 // within a line), the tiles' counts, the control block.
@@ -647,7 +660,7 @@ static ReverseForm reverse_form(const PermutePlan &pl) {
     const uint64_t bytes = pl.n * pl.key_bytes;
     if (is_veb_layout(pl.layout) ? bytes <= (32ull << 20)
                                  : pl.b == 1 ? !pl.ordered : bytes <= (192ull << 20))
-        return !is_veb_layout(pl.layout) && bytes <= (8ull << 20) ? REVERSE_KEYS : REVERSE_COPY;
+        return REVERSE_COPY;
     // (a schedule whose scratch is about as large as the array gains nothing in place)
     return reverse_space(pl).bytes <= align256(bytes) ? REVERSE_IN_PLACE : REVERSE_COPY;
 }
@@ -685,31 +698,32 @@ static int gather_grid(Kern kern, size_t smem, uint64_t ntiles, unsigned *grid) 
 }
 
 template <typename K>
-static int launch_from_copy(const PermutePlan &pl, ReverseForm form, K *A, char *ws, cudaStream_t st) {
+static int launch_from_copy(const PermutePlan &pl, const KeysGeometry &kg, ReverseForm form, uint64_t n, K *A,
+                            char *ws, cudaStream_t st) {
     K *C = reinterpret_cast<K *>(ws);
-    TL_CUDA_TRY(cudaMemcpyAsync(C, A, pl.n * sizeof(K), cudaMemcpyDeviceToDevice, st));
+    TL_CUDA_TRY(cudaMemcpyAsync(C, A, n * sizeof(K), cudaMemcpyDeviceToDevice, st));
     unsigned grid = 1;
     int rc = TL_SUCCESS;
     if (form == REVERSE_KEYS) {
-        grid = (unsigned)((pl.n + kGatherThreads - 1) / kGatherThreads);
-        btree_gather_keys_kernel<K><<<grid, kGatherThreads, 0, st>>>(A, C, pl.n, pl.bs);
+        grid = (unsigned)((n + kGatherThreads - 1) / kGatherThreads);
+        btree_gather_keys_kernel<K><<<grid, kGatherThreads, 0, st>>>(A, C, n, kg);
     } else if (is_veb_layout(pl.layout)) {
         auto kern = mveb_unstream_kernel<K, true>;
         const size_t smem = mveb_gather_keys<K>(pl.tile_keys) * sizeof(K) + 128;
         rc = gather_grid(kern, smem, pl.ntiles, &grid);
         if (rc) return rc;
-        kern<<<grid, kGatherThreads, smem, st>>>(A, C, C, pl.mp, nullptr, WaitCfg{}, nullptr);
+        kern<<<grid, kGatherThreads, smem, st>>>(A, C, pl.mp, nullptr, WaitCfg{}, nullptr);
     } else {
         uint32_t top_at = 0;
         const size_t smem = btree_gather_keys(pl.tile_keys, pl.b, sizeof(K), &top_at) * sizeof(K) + 128;
-        auto kern = btree_unstream_kernel<K, true>;
+        auto kern = pl.b <= 8 ? btree_unstream_kernel<K, true, 4> : btree_unstream_kernel<K, true, 1>;
         rc = gather_grid(kern, smem, pl.ntiles, &grid);
         if (rc) return rc;
         BtreeStream S = pl.bs;  // left to right with slots at their positions: last-level and tail tiles are staged
         S.plan = PLAN_L;
         S.seg1 = S.g.ni;
         S.nscratch = pl.n;
-        kern<<<grid, kGatherThreads, smem, st>>>(A, C, C, S, top_at, nullptr, WaitCfg{}, nullptr);
+        kern<<<grid, kGatherThreads, smem, st>>>(A, C, S, top_at, nullptr, WaitCfg{}, nullptr);
     }
     TL_CUDA_TRY(cudaGetLastError());
     return TL_SUCCESS;
@@ -739,7 +753,7 @@ static int launch_in_place(const PermutePlan &pl, K *A, char *ws, cudaStream_t s
         const size_t smem = mveb_gather_keys<K>(pl.tile_keys) * sizeof(K) + 128;
         const int rc = gather_grid(kern, smem, pl.ntiles, &grid);
         if (rc) return rc;
-        kern<<<grid, kGatherThreads, smem, st>>>(A, A, scr, pl.mp, ctrl, wc, rem);
+        kern<<<grid, kGatherThreads, smem, st>>>(A, scr, pl.mp, ctrl, wc, rem);
     } else {
         BulkPlan bp;
         int rc = make_bulk_plan(pl.bs, pl.ot, A, scr, bp);
@@ -770,10 +784,10 @@ static int launch_in_place(const PermutePlan &pl, K *A, char *ws, cudaStream_t s
         }
         uint32_t top_at = 0;
         const size_t smem = btree_gather_keys(pl.tile_keys, pl.b, sizeof(K), &top_at) * sizeof(K) + 128;
-        auto kern = btree_unstream_kernel<K, false>;
+        auto kern = pl.b <= 8 ? btree_unstream_kernel<K, false, 4> : btree_unstream_kernel<K, false, 1>;
         rc = gather_grid(kern, smem, pl.ntiles, &grid);
         if (rc) return rc;
-        kern<<<grid, kGatherThreads, smem, st>>>(A, A, scr, pl.bs, top_at, ctrl, wc, rem);
+        kern<<<grid, kGatherThreads, smem, st>>>(A, scr, pl.bs, top_at, ctrl, wc, rem);
     }
     TL_CUDA_TRY(cudaGetLastError());
     return TL_SUCCESS;
@@ -784,14 +798,16 @@ int unpermute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_byte
     if (n > 0 && !dev_A) return TL_ERROR_INVALID_VALUE;
     if (reinterpret_cast<uintptr_t>(dev_A) % (key_bytes ? key_bytes : 1)) return TL_ERROR_INVALID_VALUE;
     if (dev_ws && reinterpret_cast<uintptr_t>(dev_ws) % 256) return TL_ERROR_INVALID_VALUE;
+    KeysGeometry kg;
+    const bool by_keys = permute_by_keys(layout, n, b, key_bytes, kg);
     PermutePlan pl;
-    int rc = permute_plan_device(layout, n, b, key_bytes, st, pl);
+    int rc = by_keys ? TL_SUCCESS : permute_plan_device(layout, n, b, key_bytes, st, pl);
     if (rc) return rc;
     if (n <= 1) {
         if (ms) *ms = 0.f;
         return TL_SUCCESS;
     }
-    const ReverseForm form = reverse_form(pl);
+    const ReverseForm form = by_keys ? REVERSE_KEYS : reverse_form(pl);
     const bool in_place = form == REVERSE_IN_PLACE;
     if (dev_ws && ws_bytes < align256(n * key_bytes)) return TL_ERROR_WORKSPACE_TOO_SMALL;
     const uint64_t need = in_place ? reverse_space(pl).bytes : align256(n * key_bytes);
@@ -814,17 +830,15 @@ int unpermute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_byte
     }
     timer.start();
     if (!in_place)
-        rc = key_bytes == 8 ? launch_from_copy<uint64_t>(pl, form, static_cast<uint64_t *>(dev_A), ws, st)
-                            : launch_from_copy<uint32_t>(pl, form, static_cast<uint32_t *>(dev_A), ws, st);
+        rc = key_bytes == 8 ? launch_from_copy<uint64_t>(pl, kg, form, n, static_cast<uint64_t *>(dev_A), ws, st)
+                            : launch_from_copy<uint32_t>(pl, kg, form, n, static_cast<uint32_t *>(dev_A), ws, st);
     else
         rc = key_bytes == 8 ? launch_in_place<uint64_t>(pl, static_cast<uint64_t *>(dev_A), ws, st)
                             : launch_in_place<uint32_t>(pl, static_cast<uint32_t *>(dev_A), ws, st);
     timer.stop();
     unsigned int err = 0;
-    if (rc == TL_SUCCESS && in_place) {
-        const Ctrl *ctrl = reinterpret_cast<const Ctrl *>(ws + reverse_space(pl).off_ctrl);
-        rc = read_error_word(&ctrl->error, &err, st);
-    }
+    if (rc == TL_SUCCESS && in_place)
+        rc = read_ctrl(reinterpret_cast<const Ctrl *>(ws + reverse_space(pl).off_ctrl), &err, st);
     if (owned && pooled) cudaFreeAsync(ws, st);
     if (rc == TL_SUCCESS) rc = sync_and_check(st);
     if (owned && !pooled) {

@@ -35,6 +35,20 @@ int permute_plan_device(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, 
 int permute_plan_replay(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, bool ordered, OrderVectors &ov,
                         PermutePlan &pl);
 
+// Arrays of up to kKeysBytes in a B-tree or BST layout are moved key by key
+// through a copy, either way: two launches, no tiles, no waits.  False (rc 0)
+// when the layout or the size asks for a plan; the argument checks are make_plan's.
+// Measured on B200, one call's wall time by tiles / key by key (us): 2^10 to 2^17
+// keys 50 to 66 / 18 to 22, BST of 2^20 - 1 u64 61 / 26, b = 16 3 * 2^18 u64 68 / 29, b =
+// 2 2^21 u32 76 / 37; back from the layout 23 to 40 / 18 to 37 (from a copy tile by
+// tile).  At 16 MB both ways are even for narrow nodes.
+constexpr uint64_t kKeysBytes = 12ull << 20;
+struct KeysGeometry {
+    BtreeGeom g;
+    FastDiv64 fd;
+};
+bool permute_by_keys(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, KeysGeometry &kg);
+
 // One copy range for the bulk engine: its 16-byte-aligned interior in
 // kBulkChunk pieces, its ragged keys apart.  The scratch shares A's offset
 // within 16 bytes at both range bases, so the interiors line up.
