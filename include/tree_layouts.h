@@ -197,7 +197,7 @@ int tl_query_sorted_u32(const uint32_t *dev_sorted, uint64_t n, const uint32_t *
                         uint64_t q, uint64_t *dev_answers, void *stream, float *ms);
 int tl_query_sorted_u64(const uint64_t *dev_sorted, uint64_t n, const uint64_t *dev_queries,
                         uint64_t q, uint64_t *dev_answers, void *stream, float *ms);
-/* BST queries: a batch of 2^21 queries or more over a layout of at least 64 MB
+/* BST queries: a batch of more than 2^22 queries over a layout of 1 GB or more
  * is first grouped by value, in stream-ordered temporary device memory of about
  * q * (2 w + 8) bytes plus up to 16 MB (w the key width), so that queries close
  * in value share the deep nodes they fetch; the answers keep the batch's order.

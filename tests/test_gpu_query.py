@@ -348,3 +348,58 @@ def test_btree_top_levels_in_shared_memory(kb, b):
     got = torch.full((q,), -7, dtype=torch.int64, device="cuda")
     T.query("btree", tree, Q, got, b)
     _check_answers(tree, keys.to(dt), Q, got)
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("n,skip", [(1, 0), (2, 1), (3, 0), (4094, 1), (4095, 0), (4096, 3), (8191, 0), (8192, 1),
+                                    (65_537, 1), (2**20 - 1, 0), (2_000_003, 3)])
+def test_bst_ordered_chunks(kb, n, skip):
+    """BST descents over chunks ordered by value: trees within, just past and well
+    past the levels in shared memory, unaligned layouts, batches of one query, of
+    one value, around a block's chunk and over several rounds; the grouped route
+    (variant 20) on the same batches."""
+    import ctypes as C
+
+    import torch
+    L = T.lib()
+    L.tl_debug_set_query_variant.argtypes = [C.c_int]
+    dt = torch.int64 if kb == 8 else torch.int32
+    keys = data.sorted_keys_torch(n, 1, 3, n + skip, kb)
+    buf = torch.empty(n + skip, dtype=dt, device="cuda")
+    tree = buf[skip:]
+    tree.copy_(keys)
+    T.permute("bst", tree)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    top = int(keys[-1].item())
+    for q in [1, 295, 297, 4097, 296 * 4096 + 5]:
+        Q = torch.randint(0, top + 3, (q,), generator=g, device="cuda", dtype=torch.int64).to(dt)
+        for variant in (0, 20):
+            ans = torch.full((q,), -7, dtype=torch.int64, device="cuda")
+            L.tl_debug_set_query_variant(variant)
+            try:
+                T.query("bst", tree, Q, ans)
+            finally:
+                L.tl_debug_set_query_variant(0)
+            _check_answers(tree, keys, Q, ans)
+    Q = torch.full((20_000,), top, dtype=dt, device="cuda")
+    Q[::1000] = 0
+    ans = torch.empty(20_000, dtype=torch.int64, device="cuda")
+    T.query("bst", tree, Q, ans)
+    _check_answers(tree, keys, Q, ans)
+
+
+def test_bst_with_64_bit_nodes():
+    """2^31 + 3 keys: node numbers past 32 bits, in chunks and grouped."""
+    import torch
+    n = 2**31 + 3
+    keys = torch.arange(n, device="cuda", dtype=torch.int64).to(torch.int32)  # 0 .. n - 1 as uint32
+    T.permute("bst", keys)
+    for q in (1 << 20, (1 << 22) + 1):
+        Q64 = torch.randint(0, n + 1000, (q,), device="cuda", dtype=torch.int64)
+        Q64[:3] = torch.tensor([0, n - 1, n], device="cuda")
+        ans = torch.empty(q, dtype=torch.int64, device="cuda")
+        T.query("bst", keys, Q64.to(torch.int32), ans)
+        hit = ans != n
+        assert torch.equal(hit, Q64 < n)
+        assert torch.equal(keys[ans[hit]], Q64[hit].to(torch.int32))

@@ -18,10 +18,10 @@ namespace tl {
 
 constexpr int kQueryThreads = 256;
 constexpr uint32_t kPinBytes = 48 * 1024;
-// A grouped batch over a BST of 256 MB or more pins fewer top levels, leaving
-// room for 8 blocks an SM: measured on B200, 2^27 grouped queries, 2^30 - 1 u64
-// keys 13.25 -> 12.14 ms, 2^27 - 1 u32 10.23 -> 9.79 ms (8 KB: the same); over
-// a 128 MB tree 11.0 -> 11.6 ms, so not there
+// The search of a grouped batch over a large BST pins 16 KB of top levels,
+// leaving room for 8 blocks an SM: measured on B200, 2^27 grouped queries, 2^30 -
+// 1 u64 keys 13.25 -> 12.14 ms against 32 KB, 2^27 - 1 u32 10.23 -> 9.79 ms (8
+// KB: the same)
 constexpr uint32_t kBstGroupPinBytes = 16 * 1024;
 
 template <typename K>
@@ -36,7 +36,8 @@ __device__ __forceinline__ K key_at(const K *__restrict__ A, const K *sm, uint64
 }
 
 // ---------------------------------------------------------------- BST
-// searchBST (gpu/src/query-bst.cuh:31-42): i = 2i + 1 + (q > A[i]).
+// searchBST (gpu/src/query-bst.cuh:31-42): i = 2i + 1 + (q > A[i]).  The batch
+// grouped by value (partition_queries), answers through the carried index.
 template <typename K>
 __global__ void __launch_bounds__(kQueryThreads)
 bst_query_kernel(const K *__restrict__ A, uint64_t n, uint64_t P, const K *__restrict__ Q, uint64_t nq,
@@ -56,7 +57,7 @@ bst_query_kernel(const K *__restrict__ A, uint64_t n, uint64_t P, const K *__res
             }
             i = 2 * i + 1 + (q > cur);
         }
-        const uint64_t out = perm ? (uint64_t)__ldg(perm + qi) : qi;
+        const uint64_t out = __ldg(perm + qi);
         if (out < nq) __stcs(ans + out, res);
     }
 }
@@ -542,10 +543,33 @@ struct ChunkSort {
     uint32_t cnt[kSortBins], wsum[32];
 };
 
-// order[0, len): the chunk's offsets by value.
-template <typename K>
+// order[0, len): the chunk's offsets by value.  With kPer > 0 the chunk is read
+// once, kPer keys a thread (kPer * kSortThreads >= len), and stays in registers;
+// with 0 it is read at each of the three steps (16 keys a thread would spill:
+// the vEB search over 3e8 u64 keys 7.1 -> 7.6 ms).
+template <int kPer, typename K>
 __device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t len, uint16_t *order, ChunkSort &cs) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    K v[kPer ? kPer : 1];
+    K lo = ~K(0), hi = 0;
+    // f(x, key) for this thread's entries of the chunk
+    auto each = [&](auto f) {
+        if constexpr (kPer > 0) {
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+                const uint32_t x = threadIdx.x + i * kSortThreads;
+                if (x < len) f(x, v[i]);
+            }
+        } else {
+#pragma unroll 4
+            for (uint32_t x = threadIdx.x; x < len; x += kSortThreads) f(x, __ldg(Q + x));
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const uint32_t x = threadIdx.x + i * kSortThreads;
+        if (x < len) v[i] = __ldg(Q + x);
+    }
     __syncthreads();  // the previous chunk is done with its order
     if (threadIdx.x == 0) {
         cs.lo = ~0ull;
@@ -553,13 +577,10 @@ __device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t le
     }
     cs.cnt[threadIdx.x] = 0;
     __syncthreads();
-    K lo = ~K(0), hi = 0;
-#pragma unroll 4
-    for (uint32_t x = threadIdx.x; x < len; x += kSortThreads) {
-        const K v = __ldg(Q + x);
-        lo = min(lo, v);
-        hi = max(hi, v);
-    }
+    each([&](uint32_t, K k) {
+        lo = min(lo, k);
+        hi = max(hi, k);
+    });
     for (int o = 16; o > 0; o >>= 1) {
         lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
         hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
@@ -572,9 +593,7 @@ __device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t le
     const K base = (K)cs.lo;
     const uint32_t span = bit_length(cs.hi - cs.lo), bits = bit_length(kSortBins - 1);
     const uint32_t shift = span > bits ? span - bits : 0;
-#pragma unroll 4
-    for (uint32_t x = threadIdx.x; x < len; x += kSortThreads)
-        atomicAdd(&cs.cnt[(uint32_t)((__ldg(Q + x) - base) >> shift)], 1u);
+    each([&](uint32_t, K k) { atomicAdd(&cs.cnt[(uint32_t)((K)(k - base) >> shift)], 1u); });
     __syncthreads();
     const uint32_t c = cs.cnt[threadIdx.x];
     uint32_t inc = c;
@@ -588,10 +607,60 @@ __device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t le
     const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? cs.wsum[lane] : 0u);
     cs.cnt[threadIdx.x] = before + inc - c;
     __syncthreads();
-#pragma unroll 4
-    for (uint32_t x = threadIdx.x; x < len; x += kSortThreads)
-        order[atomicAdd(&cs.cnt[(uint32_t)((__ldg(Q + x) - base) >> shift)], 1u)] = (uint16_t)x;
+    each([&](uint32_t x, K k) { order[atomicAdd(&cs.cnt[(uint32_t)((K)(k - base) >> shift)], 1u)] = (uint16_t)x; });
     __syncthreads();
+}
+
+// ---------------------------------------------------------------- BST, ordered chunks
+// Chunks of the batch in value order, the top P = 2^T - 1 keys (as they lie) in
+// shared memory.  With 1-based nodes x the children are 2x and 2x + 1; the top is
+// walked without tests for equality, and an equal key there is where the path
+// last went left.  Neighbours in the order share their nodes far down (a level of
+// 2^k nodes is 2^k consecutive keys), so a level's loads fall into a few lines.
+// Measured on B200, before (as given below 2^21 queries or 64 MB, else grouped in
+// device memory) -> now: 2^24 queries over 2^27 - 1 u32 keys 1118 -> 1054 us, over
+// 2^26 - 1 1181 -> 844, over 2^24 - 1 1574 -> 660; 2^20 over 2^27 - 1 keys 265 -> 87, over
+// 2^20 - 1 62 -> 31.  Chunks of 8192 or 16384, or 64 KB of top levels, take L1 from
+// the descents (1205, 1193, 1471 us); one block an SM 1.5 times the time.
+constexpr uint32_t kBstChunk = 4096;
+constexpr int kBstBlocksPerSM = 2;
+
+template <typename K, typename I>
+__global__ void __launch_bounds__(kSortThreads, kBstBlocksPerSM)
+bst_query_sorted_kernel(const K *__restrict__ A, uint64_t n64, uint32_t P, uint32_t chunk, const K *__restrict__ Q,
+                        uint64_t nq, uint64_t *__restrict__ ans) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    K *sm = reinterpret_cast<K *>(smem_raw);                     // [P + 1], from 1
+    uint16_t *order = reinterpret_cast<uint16_t *>(sm + P + 1);  // [chunk]
+    __shared__ ChunkSort cs;
+    const I n = (I)n64;
+    for (uint32_t x = threadIdx.x; x < P; x += kSortThreads) sm[x + 1] = __ldg(A + x);
+    const uint32_t levels = bit_length((uint64_t)P);
+    for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
+        const uint32_t len = (uint32_t)min((uint64_t)chunk, nq - c0);
+        chunk_order<kBstChunk / kSortThreads>(Q + c0, len, order, cs);  // its barriers also cover the top
+        for (uint32_t slot = threadIdx.x; slot < len; slot += kSortThreads) {
+            const uint64_t qi = c0 + order[slot];
+            const K q = __ldg(Q + qi);
+            uint32_t y = 1;
+            for (uint32_t c = 0; c < levels; ++c) y = 2 * y + (sm[y] < q);
+            const uint32_t at = y >> __ffs(~y);
+            I x = y, res = n;
+            if (at && sm[at] == q) {
+                res = at - 1;
+                x = n + 1;
+            }
+            while (x <= n) {
+                const K cur = __ldg(A + (x - 1));
+                if (cur == q) {
+                    res = x - 1;
+                    break;
+                }
+                x = 2 * x + (cur < q);
+            }
+            ans[qi] = (uint64_t)res;
+        }
+    }
 }
 
 // ---------------------------------------------------------------- mvEB
@@ -786,7 +855,7 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
     const I low = a_off ? KPL : 0;  // a piece from here on can be read in whole sectors
     for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
         const uint32_t len = (uint32_t)min((uint64_t)chunk, nq - c0);
-        chunk_order(Q + c0, len, order, cs);
+        chunk_order<0>(Q + c0, len, order, cs);
         for (uint32_t slot = threadIdx.x; slot < len; slot += kSortThreads) {
             const uint64_t qi = c0 + order[slot];
             const K q = __ldg(Q + qi);
@@ -1259,19 +1328,20 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
     const K *Q = static_cast<const K *>(a.queries);
     uint64_t P = std::min<uint64_t>(a.n, kPinBytes / sizeof(K));
     unsigned grid = 1;
-    // BST descents search a batch of 2^21 queries or more grouped by value, over
-    // a layout of 64 MB or more.  Measured on B200, as given against grouped
-    // (grouping included): 2^23 - 1 u64 keys (64 MB), 2^22 queries 0.39 / 0.31
-    // ms, 2^20 queries 0.11 / 0.13; 2^22 - 1 u64 (32 MB) 0.30 / 0.29 at 2^22 and
-    // 9.2 / 11.4 ms at 2^27 queries.  B-tree nodes gain little even sorted (9.45
-    // against 8.28 ms) and keep the batch's order; vEB descents order chunks of
-    // it in shared memory.  Measurement hooks: variant 19 never groups, 20 always.
+    // A large batch over a large BST is grouped by value in device memory: its
+    // warps then share nodes much further down than a chunk's do, for two passes
+    // over the batch per 4 bits and answers written to random places.  Measured on
+    // B200, grouped / in ordered chunks (us): 2^27 - 1 u32 keys (512 MB) 2^24
+    // queries 1129 / 1063, 2^27 9617 / 8487; 2^28 - 1 u32 (1 GB) 2^21 230 / 188, 2^22
+    // 370 / 355, 2^23 650 / 702, 2^24 1196 / 1371; 2^30 - 1 u32 2^21 297 / 274, 2^22
+    // 513 / 553, 2^24 1458 / 2455; u64 of 512 MB 2^24 1265 / 1136, of 2 GB 1442 / 2086.
+    // Measurement hooks: variant 19 never groups, 20 always.
     QueryPartition part;
     const uint32_t *perm = nullptr;
     const uint64_t tree_bytes = a.n * sizeof(K);
-    const bool large = tree_bytes >= (64ull << 20);
-    if (a.layout == Q_BST && g_query_variant != 19 &&
-        a.q < (1ull << 32) && (g_query_variant == 20 || (a.q >= (1ull << 21) && large))) {
+    const bool large = tree_bytes >= (1ull << 30) - 1024;  // 2^28 - 1 u32 keys included
+    if (a.layout == Q_BST && g_query_variant != 19 && a.q < (1ull << 32) &&
+        (g_query_variant == 20 || (a.q > (1ull << 22) && large))) {
         const int rc = partition_queries<K>(Q, a.q, st, part);
         if (rc == TL_SUCCESS) {
             Q = static_cast<const K *>(part.qs);
@@ -1290,18 +1360,31 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         int rc = persistent_grid(kern, smem, a.q, &grid);
         if (rc) return rc;
         kern<<<grid, kQueryThreads, smem, st>>>(A, a.n, L, Q, a.q, a.answers);
-    } else if (a.layout == Q_BST) {
-        // whole top levels: 2^T - 1 keys (a grouped batch over a large tree:
-        // at most kBstGroupPinBytes of them, leaving room for more blocks)
-        if (perm && tree_bytes >= (256ull << 20)) P = std::min<uint64_t>(P, kBstGroupPinBytes / sizeof(K));
-        uint64_t top = 1;
-        while (top * 2 + 1 <= P) top = top * 2 + 1;
+    } else if (a.layout == Q_BST && perm) {
+        uint64_t top = 1;  // whole top levels: 2^T - 1 keys
+        while ((top * 2 + 1) * sizeof(K) <= kBstGroupPinBytes) top = top * 2 + 1;
         P = std::min<uint64_t>(top, a.n);
         size_t smem = P * sizeof(K);
         auto kern = bst_query_kernel<K>;
         int rc = persistent_grid(kern, smem, a.q, &grid);
         if (rc) return rc;
         kern<<<grid, kQueryThreads, smem, st>>>(A, a.n, P, Q, a.q, perm, a.answers);
+    } else if (a.layout == Q_BST) {
+        uint64_t top = 1;  // whole top levels, at most 32 KB with the unused slot 0
+        while (top * 2 + 1 <= a.n && (top * 2 + 2) * sizeof(K) <= 32768) top = top * 2 + 1;
+        const uint64_t slots = (uint64_t)query_sm_count() * kBstBlocksPerSM;
+        const uint64_t rounds = (a.q + slots * kBstChunk - 1) / (slots * kBstChunk);
+        const uint64_t chunk = (a.q + slots * rounds - 1) / (slots * rounds);  // equal chunks, the fewest rounds
+        const size_t smem = (top + 1) * sizeof(K) + chunk * sizeof(uint16_t);
+        auto launch = [&](auto kern) -> int {
+            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kern<<<(unsigned)std::min(slots, (a.q + chunk - 1) / chunk), kSortThreads, smem, st>>>(
+                A, a.n, (uint32_t)top, (uint32_t)chunk, Q, a.q, a.answers);
+            return TL_SUCCESS;
+        };
+        const int rc = a.n < (1ull << 31) ? launch(bst_query_sorted_kernel<K, uint32_t>)
+                                          : launch(bst_query_sorted_kernel<K, uint64_t>);
+        if (rc) return rc;
     } else if (a.layout == Q_BTREE) {
         uint64_t top = 0, lvl = a.b;
         while (top + lvl <= P) {  // whole top levels: (b+1)^L - 1 keys
