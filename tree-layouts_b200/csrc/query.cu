@@ -1311,11 +1311,42 @@ static int query_sm_count() {
     return g_qsm;
 }
 
+constexpr size_t kSmemLimit = 64 * 1024;
+
+// Resident blocks per SM of a kernel, asked of the runtime once per thread, device
+// and shape (the question and the attribute cost a small batch's call a
+// microsecond of its four).
+static int resident_blocks(const void *kern, size_t smem, int *per_sm) {
+    struct Known {
+        const void *kern;
+        size_t smem;
+        int dev, per_sm;
+    };
+    constexpr int kKnown = 32;
+    static thread_local Known known[kKnown];
+    static thread_local int count = 0;
+    int dev = 0;
+    TL_CUDA_TRY(cudaGetDevice(&dev));
+    for (int i = 0; i < std::min(count, kKnown); ++i)
+        if (known[i].kern == kern && known[i].smem == smem && known[i].dev == dev) {
+            *per_sm = known[i].per_sm;
+            return TL_SUCCESS;
+        }
+    // one limit for every shape (a later smaller one must not lower it); all ask for at most kPinBytes
+    static_assert(kPinBytes <= kSmemLimit, "the pinned prefix fits the limit");
+    if (smem > kSmemLimit) return TL_ERROR_UNSUPPORTED;
+    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+    TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, kQueryThreads, smem));
+    known[count++ % kKnown] = Known{kern, smem, dev, *per_sm};  // the oldest goes first
+    if (count == 2 * kKnown) count = kKnown;
+    return TL_SUCCESS;
+}
+
 template <typename Kern>
 static int persistent_grid(Kern kern, size_t smem, uint64_t work_threads, unsigned *grid) {
-    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kQueryThreads, smem));
+    const int rc = resident_blocks(reinterpret_cast<const void *>(kern), smem, &per_sm);
+    if (rc) return rc;
     uint64_t g = (uint64_t)std::max(per_sm, 1) * query_sm_count();
     uint64_t need = (work_threads + kQueryThreads - 1) / kQueryThreads;
     *grid = (unsigned)std::max<uint64_t>(1, std::min(g, need));

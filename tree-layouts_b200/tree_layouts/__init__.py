@@ -96,11 +96,22 @@ def _check(rc: int, what: str) -> None:
         raise TreeLayoutError(rc, what)
 
 
+_raw_stream = None  # (current device, raw current stream) getters
+
+
 def _stream_ptr(stream) -> int:
-    if stream is None:
+    if stream is not None:
+        return getattr(stream, "cuda_stream", stream)
+    global _raw_stream
+    if _raw_stream is None:
         import torch
-        return torch.cuda.current_stream().cuda_stream
-    return getattr(stream, "cuda_stream", stream)
+        torch.cuda.current_stream()  # CUDA initialised
+        # the raw handle where torch has a getter for it: building a Stream object
+        # takes 3 us, a third of a small query's call
+        get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        _raw_stream = (torch.cuda.current_device, get or (lambda dev: torch.cuda.current_stream(dev).cuda_stream))
+    device, raw = _raw_stream
+    return raw(device())
 
 
 def _key_bytes(t) -> int:
