@@ -403,3 +403,29 @@ def test_bst_with_64_bit_nodes():
         hit = ans != n
         assert torch.equal(hit, Q64 < n)
         assert torch.equal(keys[ans[hit]], Q64[hit].to(torch.int32))
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("n,skip", [(1, 0), (2, 1), (3, 0), (31, 3), (4096, 1), (4097, 0), (8193, 1), (1_000_003, 5)])
+def test_sorted_array_ordered_chunks(kb, n, skip):
+    """Binary search over chunks ordered by value: arrays within and past the
+    pinned probes, unaligned arrays, batches on either side of the form's line and
+    over several rounds of chunks, a batch of one value."""
+    import torch
+    dt = torch.int64 if kb == 8 else torch.int32
+    keys = data.sorted_keys_torch(n, 1, 3, n + skip, kb)
+    buf = torch.empty(n + skip, dtype=dt, device="cuda")
+    arr = buf[skip:]
+    arr.copy_(keys)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    top = int(keys[-1].item())
+    for q in [1, (1 << 16) - 1, 1 << 16, 296 * 4096 + 5]:
+        Q = torch.randint(0, top + 3, (q,), generator=g, device="cuda", dtype=torch.int64).to(dt)
+        ans = torch.full((q,), -7, dtype=torch.int64, device="cuda")
+        T.query("sorted", arr, Q, ans)
+        _check_answers(arr, keys, Q, ans)
+    Q = torch.full((70_000,), top, dtype=dt, device="cuda")
+    ans = torch.empty(70_000, dtype=torch.int64, device="cuda")
+    T.query("sorted", arr, Q, ans)
+    _check_answers(arr, keys, Q, ans)
