@@ -162,3 +162,33 @@ def test_small_arrays_key_by_key_and_by_tiles(layout, b, dtype):
             t = to_dev(keys)
             T.permute(layout, t, b, workspace=torch.empty(need, dtype=torch.uint8, device="cuda"))
             assert np.array_equal(from_dev(t), exp), (layout, b, n, "tiles")
+
+
+@pytest.mark.parametrize("layout", ["mveb", "veb"])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+@pytest.mark.parametrize("tiles", [2, 295, 297, 593, 900])
+def test_veb_stream_ring_of_stages(layout, dtype, tiles):
+    """Fewer tiles than blocks, one to four a block (a stage used again, and never), the last one ragged and
+    the array off the 16-byte boundary at both ends."""
+    n = tiles * 32768 // np.dtype(dtype).itemsize - 37
+    keys = data.sorted_keys_np(n, 1, 5, n, dtype)
+    buf = to_dev(np.concatenate([np.zeros(1, dtype), keys, np.zeros(1, dtype)]))
+    T.permute(layout, buf[1:1 + n])
+    out = from_dev(buf)
+    assert np.array_equal(out[1:1 + n], O.permute(layout, keys, 16))
+    assert out[0] == 0 and out[-1] == 0
+
+
+def test_veb_stream_expired_wait_reports_timeout():
+    keys = data.sorted_keys_np(8_000_003, 1, 16, 1, np.uint32)
+    t = to_dev(keys)
+    T.set_wait(spin_limit=64, force_timeout=True)
+    try:
+        with pytest.raises(T.TreeLayoutError) as ei:
+            T.permute("mveb", t)
+        assert ei.value.status == T.ERROR_TIMEOUT
+    finally:
+        T.set_wait(0, False)
+    t = to_dev(keys)
+    T.permute("mveb", t)
+    assert np.array_equal(from_dev(t), O.permute("mveb", keys, 16))

@@ -62,13 +62,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // Bounded wait for phase `parity` of an mbarrier.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-    for (unsigned int it = 0; it <= kBulkSpinLimit; ++it) {
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned int limit = kBulkSpinLimit) {
+    for (unsigned int it = 0; it <= limit; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         __nanosleep(64);
     }
     return false;
+}
+
+// For a phase that another warp's read-flag wait may hold up (about a second):
+// the bound lies several times above that wait's.
+__device__ __forceinline__ bool mbar_wait_long(uint64_t *bar, uint32_t parity) {
+    return mbar_wait(bar, parity, kBulkSpinLimit * 16u);
 }
 
 __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, uint32_t bytes, uint64_t *bar) {

@@ -40,6 +40,13 @@ namespace tl {
 constexpr int kStreamThreads = 256;
 constexpr int kStreamBlocksPerSM = 6;  // what shared memory allows with 32 KB tiles
 constexpr uint32_t kUnitMaxLevels = 8;
+// mveb_stream_kernel: 32 KB stages a block, blocks per SM (the shared memory of
+// six tiles an SM), store warps a block (after the loader, publisher and waiter).
+constexpr uint32_t kMvebStages = 3;
+constexpr int kMvebBlocksPerSM = 2;
+constexpr uint32_t kMvebStoreWarps = 8;
+constexpr int kMvebThreads = 32 * (3 + (int)kMvebStoreWarps);
+constexpr size_t kMvebStageBytes = 32768 + 128;
 
 template <typename K>
 constexpr uint64_t stream_tile_keys() {
@@ -98,90 +105,181 @@ btree_scatter_keys_kernel(K *__restrict__ A, const K *__restrict__ C, uint64_t n
 }
 
 // ---------------------------------------------------------------- mvEB stream
+// A tile's stage of the ring: the loader warp fills in the tile, the waiter
+// warp clears ok when a wait of the tile ran out.
+struct MvebStage {
+    uint64_t k, p0, p1, base;  // tile, its source ranks, and the rank at sm[0] of the stage
+    int ri;                    // its region; -1: no tile is left
+    int ok;
+};
+
+// The bound is the copy rate once no store waits: with a tile a block at a time
+// (load, publish, wait, store; 6 blocks an SM) every tile met flags that had
+// only just been claimed, and those waits were a sixth of the pass.  Here the
+// loader keeps a ring of stages filled by the bulk-copy engine, the publisher
+// flags each tile the moment its copy lands, while earlier tiles of the block
+// are still being stored, and the waiter has a tile's flags checked before the
+// store warps, which meet at no barrier, come to it.  A block claims tickets in
+// order and a tile is published when its stage is free, that is when tiles with
+// smaller tickets are stored: the smallest unpublished tile always progresses.
+// Measured on B200, 3e8 keys: u32 500 -> 414 us (5.8 TB/s), u64 948 -> 789; two
+// stages in three blocks 442 / 860, six in one 520 / 959 (24 store warps: one
+// loader's tickets and copies come too slowly), 12 and 16 store warps 413 / 818
+// and 419 / 806.
 template <typename K>
-__global__ void __launch_bounds__(kStreamThreads, kStreamBlocksPerSM)
+__global__ void __launch_bounds__(kMvebThreads, kMvebBlocksPerSM)
 mveb_stream_kernel(K *__restrict__ A, K *__restrict__ scr, const __grid_constant__ MvebParams prm,
-                   Ctrl *ctrl, WaitCfg wc, unsigned int *flags) {
+                   Ctrl *ctrl, WaitCfg wc, unsigned int *flags, uint32_t ring) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    K *sm = reinterpret_cast<K *>(smem_raw);  // see load_tile_issue
-    __shared__ unsigned long long s_ticket;
-    __shared__ int s_ok;
-    __shared__ unsigned char s_inv[256];
+    __shared__ uint64_t s_full[kMvebStages], s_ready[kMvebStages], s_empty[kMvebStages];
+    __shared__ MvebStage s_st[kMvebStages];
     const MvebPlan &P = prm.plan;
-    const uint64_t ntiles = P.total_tiles;
-    int loaded_U = -1;
-    uint32_t inv_pk[2] = {0, 0};  // this lane's entries of the unit table (see below)
-    const uint32_t lane = threadIdx.x & 31;
-    // The next ticket is claimed as the tile ends, not as it starts: a tile's
-    // stores wait for the tiles just right of it, claimed just before it, and a
-    // ticket held through a whole tile made those waits long (measured on B200,
-    // 2^30 - 1 u32 keys: stalled waits 8.2e4 -> 4.8e4, 1.83 -> 1.81 ms).
-    TicketPipe tp;
-    for (unsigned long long t = ticket_first(ctrl, &s_ticket); t < ntiles; t = ticket_advance(tp, &s_ticket)) {
-        const uint64_t k = ntiles - 1 - t;
-        int ri;
-        uint64_t p0, p1;
-        mveb_tile(P, k, ri, p0, p1);
-        const MvebRegion &R = P.reg[ri];
-        if ((int)R.U != loaded_U && R.U) {  // block-uniform: unit tables for this height
-            const unsigned char *src = prm.inv + unit_table_off(R.U);
-            __syncthreads();  // every lane has its packed entries of the previous table
-            for (uint32_t q = threadIdx.x; q < (1u << R.U) - 1; q += blockDim.x) s_inv[q] = src[q];
-            __syncthreads();
-            // each lane's entries q = lane + 32 j (j < 8), four per register
-            inv_pk[0] = inv_pk[1] = 0;
-            const uint32_t uu = (1u << R.U) - 1;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < ring; ++s) {
+            mbar_init(&s_full[s], 32);
+            mbar_init(&s_ready[s], 1);
+            mbar_init(&s_empty[s], kMvebStoreWarps + 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    uint32_t s = 0, phase = 0;  // stage of this warp's next tile, and the parity of its round
+    auto stage_keys = [&](uint32_t i) { return reinterpret_cast<K *>(smem_raw + (size_t)i * kMvebStageBytes); };
+    auto advance = [&] {
+        if (++s == ring) {
+            s = 0;
+            phase ^= 1;
+        }
+    };
+    auto wait_bar = [&](uint64_t *bar, uint32_t parity) {
+        const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_long(bar, parity));
+        if (!ok && lane == 0) atomicOr(&ctrl->error, 1u << TL_ERROR_TIMEOUT);
+        return ok;
+    };
+    if (warp == 0) {  // loader
+        uint32_t issued = 0;
+        while (true) {
+            // the first round finds the stages empty: waiting for the parity before the first passes at once
+            if (!wait_bar(&s_empty[s], phase ^ 1)) break;
+            unsigned long long t = 0;
+            if (lane == 0) t = atomicAdd(&ctrl->ticket, 1ull);
+            t = __shfl_sync(0xFFFFFFFFu, t, 0);
+            MvebStage &T = s_st[s];
+            if (t >= P.total_tiles) {
+                if (lane == 0) T.ri = -1;
+                __syncwarp();
+                mbar_arrive(&s_full[s]);
+                return;  // its loads complete before the publisher leaves
+            }
+            const uint64_t k = P.total_tiles - 1 - t;
+            int ri;
+            uint64_t p0, p1;
+            mveb_tile(P, k, ri, p0, p1);
+            K *sm = stage_keys(s);
+            constexpr uint32_t V = 16 / sizeof(K);
+            const uint64_t base = tile_base<16>(A, p0);
+            uint64_t a0 = base != p0 ? base + V : p0;  // first aligned key (base may lie below 0 and wrap)
+            if (a0 > p1) a0 = p1;
+            const uint64_t a1 = a0 + (p1 - a0) / V * V;
+            if (lane < a0 - p0) sm[p0 + lane - base] = A[p0 + lane];
+            if (lane < p1 - a1) sm[a1 + lane - base] = A[a1 + lane];
+            if (lane == 0) {
+                T.k = k, T.p0 = p0, T.p1 = p1, T.base = base;
+                T.ri = ri, T.ok = 1;
+                const uint32_t bytes = (uint32_t)((a1 - a0) * sizeof(K));
+                // the ragged ends of the tile before were stored to where this copy lands
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_expect_tx(&s_full[s], bytes);
+                if (bytes) bulk_load(sm + (a0 - base), A + a0, bytes, &s_full[s]);
+            } else {
+                mbar_arrive(&s_full[s]);
+            }
+            if (issued < ring) ++issued;
+            advance();
+        }
+        for (uint32_t i = 0; i < issued; ++i) {  // a wait ran out: its copies in flight land first
+            if (s-- == 0) s = ring - 1, phase ^= 1;
+            mbar_wait(&s_full[s], phase);
+        }
+    } else if (warp == 1) {  // publisher: "tile read" as soon as its copy has landed
+        while (wait_bar(&s_full[s], phase)) {
+            const int ri = s_st[s].ri;
+            __syncwarp();
+            if (lane == 0 && ri >= 0) {
+                st_relaxed(&flags[s_st[s].k], wc.flag_value);
+                mbar_arrive(&s_empty[s]);
+            }
+            if (ri < 0) break;
+            advance();
+        }
+    } else if (warp == 2) {  // waiter: the tiles under this tile's destinations have been read
+        while (wait_bar(&s_full[s], phase)) {
+            MvebStage &T = s_st[s];
+            const int ri = T.ri;
+            uint64_t k_lo, k_hi;
+            bool ok = true;
+            if (ri >= 0 && mveb_tile_wait(P, P.reg[ri], T.p0, T.p1, k_lo, k_hi))
+                for (uint64_t f = k_lo + lane; f <= k_hi; f += 32)
+                    if (!wait_flag(&flags[f], wc.wait_value, ctrl, wc)) ok = false;
+            if (!ok) T.ok = 0;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_ready[s]);
+            if (ri < 0) break;
+            advance();
+        }
+    } else {  // store warps
+        const uint32_t w = warp - 3;
+        int loaded_U = -1;
+        uint32_t inv_pk[2] = {0, 0};  // this lane's entries q = lane + 32 j (j < 8) of the unit table, four a register
+        while (wait_bar(&s_full[s], phase) && wait_bar(&s_ready[s], phase)) {
+            const MvebStage &T = s_st[s];
+            if (T.ri < 0) break;
+            const MvebRegion &R = P.reg[T.ri];
+            const uint64_t p0 = T.p0, p1 = T.p1, base = T.base;
+            const K *sm = stage_keys(s);
+            if (R.U == 0) {
+                for (uint64_t x = p0 + w * 32 + lane; x < p1; x += 32 * kMvebStoreWarps)
+                    scr[R.slot_base + (x - R.src)] = sm[x - base];
+            } else if (T.ok) {
+                const uint32_t U = R.U;
+                const uint64_t u = (1ull << U) - 1;
+                if ((int)U != loaded_U) {
+                    const unsigned char *src = prm.inv + unit_table_off(U);
+                    inv_pk[0] = inv_pk[1] = 0;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t q = lane + 32u * j;
-                if (q < uu) inv_pk[j >> 2] |= (uint32_t)s_inv[q] << (8 * (j & 3));
-            }
-            loaded_U = R.U;
-        }
-        if (threadIdx.x == 0) s_ok = 1;  // the previous tile's readers are past the ticket barrier
-        const uint64_t base = load_tile<16>(A, p0, p1, sm);
-        publish_read(&flags[k], wc);
-        if (R.U == 0) {
-            for (uint64_t x = p0 + threadIdx.x; x < p1; x += blockDim.x)
-                scr[R.slot_base + (x - R.src)] = sm[x - base];
-            ticket_claim(ctrl, tp);
-            continue;
-        }
-        uint64_t k_lo, k_hi;
-        if (mveb_tile_wait(P, R, p0, p1, k_lo, k_hi)) {
-            for (uint64_t f = k_lo + threadIdx.x; f <= k_hi; f += blockDim.x)
-                if (!wait_flag(&flags[f], wc.wait_value, ctrl, wc)) s_ok = 0;
-            __syncthreads();
-            if (!s_ok) {
-                ticket_claim(ctrl, tp);
-                continue;
-            }
-        }
-        const uint32_t U = R.U;
-        const uint64_t u = (1ull << U) - 1;
-        uint64_t g0, g1;
-        mveb_tile_groups(R, p0, p1, g0, g1);
-        const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-        // a warp's units in batches of 32: their destinations lane-parallel, one
-        // unit per lane, then each unit's keys by the whole warp
-        for (uint64_t gb = g0 + warp; gb < g1; gb += 32ull * nwarps) {
-            const uint64_t gl = gb + (uint64_t)lane * nwarps;
-            const uint64_t my_dst = gl < g1 ? mveb_unit_dst(R, gl) : 0;
-            const uint32_t nb = (uint32_t)std::min<uint64_t>(32, (g1 - gb + nwarps - 1) / nwarps);
-            for (uint32_t j = 0; j < nb; ++j) {
-                const uint64_t gi = gb + (uint64_t)j * nwarps;
-                const uint64_t dst = __shfl_sync(0xFFFFFFFFu, my_dst, j);
-                const uint32_t gsrc = (uint32_t)(R.src + (gi << U) - base);
-                K *d = A + dst + lane;
-                const K *g = sm + gsrc;
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t q = lane + 32u * j;
+                        if (q < (uint32_t)u) inv_pk[j >> 2] |= (uint32_t)src[q] << (8 * (j & 3));
+                    }
+                    loaded_U = (int)U;
+                }
+                uint64_t g0, g1;
+                mveb_tile_groups(R, p0, p1, g0, g1);
+                // a warp's units in batches of 32: their destinations lane-parallel, one
+                // unit per lane, then each unit's keys by the whole warp
+                for (uint64_t gb = g0 + w; gb < g1; gb += 32ull * kMvebStoreWarps) {
+                    const uint64_t gl = gb + (uint64_t)lane * kMvebStoreWarps;
+                    const uint64_t my_dst = gl < g1 ? mveb_unit_dst(R, gl) : 0;
+                    const uint32_t nb = (uint32_t)std::min<uint64_t>(32, (g1 - gb + kMvebStoreWarps - 1) / kMvebStoreWarps);
+                    for (uint32_t j = 0; j < nb; ++j) {
+                        const uint64_t gi = gb + (uint64_t)j * kMvebStoreWarps;
+                        const uint64_t dst = __shfl_sync(0xFFFFFFFFu, my_dst, j);
+                        const uint32_t gsrc = (uint32_t)(R.src + (gi << U) - base);
+                        K *d = A + dst + lane;
+                        const K *g = sm + gsrc;
 #pragma unroll
-                for (int jj = 0; jj < 8; ++jj)
-                    if (lane + 32u * jj < (uint32_t)u) d[32 * jj] = g[(inv_pk[jj >> 2] >> (8 * (jj & 3))) & 0xFFu];
-                if (lane == 0 && R.src + (gi << U) + u < R.src + R.len)
-                    scr[R.slot_base + gi] = sm[gsrc + u];
+                        for (int jj = 0; jj < 8; ++jj)
+                            if (lane + 32u * jj < (uint32_t)u) d[32 * jj] = g[(inv_pk[jj >> 2] >> (8 * (jj & 3))) & 0xFFu];
+                        if (lane == 0 && R.src + (gi << U) + u < R.src + R.len)
+                            scr[R.slot_base + gi] = sm[gsrc + u];
+                    }
+                }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_empty[s]);
+            advance();
         }
-        ticket_claim(ctrl, tp);
     }
 }
 
@@ -327,11 +425,13 @@ static int launch_permute_k(const PermutePlan &pl, K *A, char *ws, cudaStream_t 
     const int smx = sm_count();
     if (is_veb_layout(pl.layout)) {
         auto kern = mveb_stream_kernel<K>;
-        TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        constexpr size_t ring_bytes = kMvebStages * kMvebStageBytes;
+        TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes));
         int per_sm = 0;
-        TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStreamThreads, smem));
+        TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMvebThreads, ring_bytes));
         uint64_t grid = std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * smx, std::max<uint64_t>(pl.ntiles, 1));
-        if (pl.ntiles) kern<<<(unsigned)grid, kStreamThreads, smem, st>>>(A, scr, pl.mp, ctrl, wc, flags), ++nl;
+        const uint32_t ring = (uint32_t)std::min<uint64_t>(kMvebStages, (pl.ntiles + grid - 1) / grid);
+        if (pl.ntiles) kern<<<(unsigned)grid, kMvebThreads, ring_bytes, st>>>(A, scr, pl.mp, ctrl, wc, flags, ring), ++nl;
         TL_CUDA_TRY(cudaGetLastError());
         timer.mid();
         if (pl.scratch_keys) {
@@ -388,10 +488,10 @@ int btree_plan_of(uint64_t n, uint64_t b) {
 }
 
 template <typename Kern>
-static int blocks_per_sm_of(Kern kern, size_t smem) {
+static int blocks_per_sm_of(Kern kern, size_t smem, int threads = kStreamThreads) {
     int per_sm = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStreamThreads, smem) != cudaSuccess)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
         return -1;
     return per_sm;
 }
@@ -402,8 +502,8 @@ int stream_blocks_per_sm(int layout, uint32_t key_bytes) {
     const size_t smem = 32768 + kTileSmemSlack;
     const bool w8 = key_bytes == 8;
     if (is_veb_layout(layout))
-        return w8 ? blocks_per_sm_of(mveb_stream_kernel<uint64_t>, smem)
-                  : blocks_per_sm_of(mveb_stream_kernel<uint32_t>, smem);
+        return w8 ? blocks_per_sm_of(mveb_stream_kernel<uint64_t>, kMvebStages * kMvebStageBytes, kMvebThreads)
+                  : blocks_per_sm_of(mveb_stream_kernel<uint32_t>, kMvebStages * kMvebStageBytes, kMvebThreads);
     if (layout == TL_LAYOUT_BST)
         return w8 ? blocks_per_sm_of(btree_stream_kernel<uint64_t, true>, smem)
                   : blocks_per_sm_of(btree_stream_kernel<uint32_t, true>, smem);
