@@ -232,3 +232,19 @@ def test_batched_queries_over_unaligned_instances(b, kb, num, lo, hi, q, skip):
     at = torch.searchsorted(comp, want).clamp_max(max(comp.numel() - 1, 0))
     present = ok & (comp[at] == want)
     assert bool((present == hit).all())
+
+
+@pytest.mark.parametrize("threads", [256, 512])
+@pytest.mark.parametrize("b", [1, 8, 16])
+@pytest.mark.parametrize("num,lo,hi", [(1, 8, 9), (3, 12, 13), (40, 6, 14), (600, 10, 13), (24, 17, 18)])
+def test_batch_ring_of_stages(num, lo, hi, b, threads):
+    """256-key tiles: fewer items than blocks, up to a full ring a block, and enough of them that items are
+    claimed ahead; both schedules, copy chunks behind the tiles."""
+    keys, off, sizes = _batch(num, lo, hi, 5 + num)
+    ref = _expected(keys.cpu().numpy().view(np.uint64), sizes, b)
+    plan = TB.BatchPlan(off, b=b)
+    plan.set_tuning(tile_keys=[256] * TB.NCLASS, threads=threads)
+    for _ in range(2):
+        got = keys.clone()
+        plan.permute(got)
+        assert np.array_equal(got.cpu().numpy().view(np.uint64), ref)

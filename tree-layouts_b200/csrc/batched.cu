@@ -26,18 +26,23 @@
 #include "batched.h"
 #include "btree_order.h"
 #include "btree_plan.cuh"
+#include "bulk.cuh"
 #include "internal.h"
 
 namespace tl {
 
 constexpr int kBatchThreads = 256;     // query kernel
-// Permute kernel: 256 or 512 threads (tuned), compiled for 4 blocks of 256
-// threads per SM (64 registers a thread).  Its plan sits in shared memory, not
-// in the constant bank as the single-array kernel's does, so at the 6 blocks
-// that shared memory would allow (40 registers) it spills and runs 1.3x slower
-// (measured on B200: 12.6 ms against 9.4 for 2.06e9 keys).
-constexpr int kBatchBlocksPerSM256 = 4;
-constexpr int kBatchBlocksPerSM512 = 2;
+// Permute kernel: blocks of three 32 KB stages, two an SM, with 8 store warps
+// (plan threads 256) or 4 (512): a tuned choice.  1024 arrays of 2^10..2^22
+// keys, b = 8 on B200: 8 store warps 1.65 ms, 6 1.63, 4 1.63; arrays of
+// 2^8..2^14: 73, 80 and 88 us; at 10 and more the registers spill (1.9 ms).
+constexpr int kBatchStages = 3, kBatchBlocksPerSM = 2;
+constexpr int kBatchStoreWarps256 = 8, kBatchStoreWarps512 = 4;
+// Launches with fewer items a stage than this claim an item only when its stage
+// is empty: claimed ahead, the last items queue up behind others (2^8..2^14
+// keys: 81 us ahead, 73 not; large batches gain 2 % from it).
+constexpr uint64_t kClaimAheadItems = 4;
+constexpr size_t kBatchBlockSmem = 100 * 1024;  // dynamic shared memory of a block, beside the stages' plans
 constexpr int kMaxClass = 48;
 
 struct alignas(16) BatchInst {
@@ -58,14 +63,12 @@ struct alignas(16) BatchInst {
 constexpr uint64_t kBatchOrderMinTiles = 64;
 constexpr uint64_t kChunkItemsMax = 64;
 constexpr uint64_t kRangePiece = 2048;
-// An instance takes the ordered schedule only if that moves at most this share
-// of the scratch keys of its fixed-direction schedule: in the batched kernel
-// (plan in shared memory, 64 registers) an ordered tile costs more instructions
-// than a fixed one, and fewer bytes pay for them only where they are many fewer.
-// Measured on B200, 4096 arrays of 2^10..2^22 keys: b = 16 9.02 ms at 0.3
-// against 9.51 fixed and 9.39 ordered everywhere; b = 8 9.34 / 9.42 / 9.69;
-// b = 1 11.76 / 11.76 / 12.37.
-constexpr double kOrderGain = 0.3;
+// An instance takes the ordered schedule if that moves at most this share of the
+// scratch keys of its fixed-direction schedule.  Measured on B200, 1024 arrays of
+// 2^10..2^22 keys at 0.3, 0.6 and 0.9: b = 8 1.75, 1.65, 1.64 ms; b = 1 2.35,
+// 2.27, 2.12; b = 4 2.03, 1.92, 1.88; b = 16 1.59, 1.57, 1.57.  Their longer item
+// lists make the plan, built once, 23 ms instead of 20.
+constexpr double kOrderGain = 0.9;
 constexpr uint64_t kInterleaveRun = 1;  // stream tiles an instance takes in a row
 static_assert(sizeof(BatchInst) % 16 == 0, "BatchInst is copied to shared memory in 16-byte words");
 
@@ -200,12 +203,13 @@ __global__ void batch_owner_kernel(const BatchInst *__restrict__ inst, uint32_t 
 template <typename K>
 static __device__ __forceinline__ void batch_copy_items(K *__restrict__ keys, K *__restrict__ scr, const BatchInst &I,
                                                      const FixSeg *__restrict__ items,
-                                                     const uint64_t *__restrict__ citem, uint64_t c) {
+                                                     const uint64_t *__restrict__ citem, uint64_t c, uint32_t tid,
+                                                     uint32_t nt) {
     const uint64_t i0 = citem[I.chunk_base + c];
     const uint64_t i1 = c + 1 < I.nchunks ? citem[I.chunk_base + c + 1] : I.item_base + I.nitems;
     K *const dst = keys + I.off;
     const K *const src = scr + I.scr_base;
-    for (uint64_t i = i0 + (threadIdx.x >> 5); i < i1; i += blockDim.x >> 5) {
+    for (uint64_t i = i0 + (tid >> 5); i < i1; i += nt >> 5) {
         const uint64_t dl = __ldg(reinterpret_cast<const unsigned long long *>(&items[i].dst_len));
         const uint64_t so = __ldg(reinterpret_cast<const unsigned long long *>(&items[i].src));
         warp_copy_keys(dst + (dl & kSegDstMask), src + so, 0, (uint32_t)(dl >> 48));
@@ -216,7 +220,7 @@ static __device__ __forceinline__ void batch_copy_items(K *__restrict__ keys, K 
 // ranges, taken as one concatenated range.
 template <typename K>
 static __device__ __forceinline__ void batch_copy_ranges(K *__restrict__ keys, K *__restrict__ scr, const BatchInst &I,
-                                                      uint64_t c) {
+                                                      uint64_t c, uint32_t tid, uint32_t nt) {
     const uint64_t lo = c * kCopyChunk, hi = lo + kCopyChunk;
     uint64_t acc = 0;
     const int nr = btree_copy_range_count(I.S);
@@ -225,7 +229,7 @@ static __device__ __forceinline__ void batch_copy_ranges(K *__restrict__ keys, K
         if (!btree_copy_range(I.S, q, r)) continue;
         const uint64_t a = lo > acc ? lo - acc : 0;
         const uint64_t e = min(hi - acc, r.len);
-        if (a < e) copy_keys(keys + I.off + r.dst + a, scr + I.scr_base + r.src + a, e - a, 0, 1);
+        if (a < e) copy_keys(keys + I.off + r.dst + a, scr + I.scr_base + r.src + a, e - a, tid, nt);
         acc += r.len;
     }
 }
@@ -233,117 +237,188 @@ static __device__ __forceinline__ void batch_copy_ranges(K *__restrict__ keys, K
 constexpr uint32_t kNoInst = 0xFFFFFFFFu;
 constexpr uint32_t kPlanWords = sizeof(BatchInst) / 16;
 
-// Warps 1.. copy instance j's plan to a shared-memory buffer with cp.async (they
-// wait for it with their tile's copies, or explicitly after a copy chunk).
-__device__ __forceinline__ void prefetch_plan(const BatchInst *inst, uint32_t j, unsigned char *buf) {
-    if (threadIdx.x < 32) return;
-    const char *src = reinterpret_cast<const char *>(inst + j);
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(buf);
-    for (uint32_t w = threadIdx.x - 32; w < kPlanWords; w += blockDim.x - 32)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + w * 16), "l"(src + (size_t)w * 16)
-                     : "memory");
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
+// Work items in ticket order through a ring of stages.  Each stage has two warps
+// of its own: the first claims an item, fetches its instance's plan, loads the
+// tile, publishes it and waits for the tiles under its bulk keys (a copy chunk:
+// for its instance's tiles); the second works out the tile's runs of top keys
+// and waits for the tiles under them.  The store warps take the stages in turn
+// and meet at no barrier.  A stage claims its next item, and fetches its plan,
+// while its present one is stored; stages claim in turn, so a block stores its
+// items in ticket order.  The smallest item not yet stored is its block's next,
+// its stage is empty, and it waits only for smaller ones: it always progresses.
+// What bounds it is traffic (2 n w plus 2 w a scratch key) once loads, waits and
+// stores overlap: with a block holding one item at a time, load, publish, wait
+// and store in turn, 1024 arrays of 2^10..2^22 keys took 1885 us at b = 8 and
+// 1808 at b = 16; in the ring 1752 and 1589, and with the ordered schedule, whose
+// instructions now hide, in more instances (kOrderGain) 1640 and 1573.  Claiming
+// ahead is 2 % of it; two stages in three blocks took as long.
+struct BatchStage {
+    BatchInst I;
+    TileShared ts;
+    uint64_t t, next, p0, p1, base;
+    int kind;  // kItemTile, kItemChunk, kItemNone
+};
+constexpr int kItemTile = 0, kItemChunk = 1, kItemNone = 2;
 
-// Work items in ticket order; a block holds four tickets: the item it works
-// on, the next (its owner and tile known, its owner's plan copied to the
-// second plan buffer while the current item runs), the one after (its owner
-// copied to shared memory while the current item runs) and a fourth (the
-// atomic claiming it in flight).  Thread 0 starts those copies (cp.async, no
-// registers held across the item) as an item starts; between two items it
-// alone releases the finished tile to its instance's copy chunks (fence, then
-// the done counter) and moves the pipeline on, one barrier on either side.
-// Holding tickets ahead cannot stall the launch: the smallest ticket held and
-// not yet done is always some block's current item, and an item waits only
-// for smaller tickets.
-template <typename K, int kThreads, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks)
+template <typename K, int kStoreWarps>
+__global__ void __launch_bounds__(32 * (2 * kBatchStages + kStoreWarps), kBatchBlocksPerSM)
 batch_permute_kernel(K *__restrict__ keys, K *__restrict__ scr, const BatchInst *__restrict__ inst,
                      const uint32_t *__restrict__ owner, const uint32_t *__restrict__ tile,
                      const FixSeg *__restrict__ items, const uint64_t *__restrict__ citem, BatchTotals tot,
-                     Ctrl *ctrl, WaitCfg wc, unsigned int *flags, unsigned int *done) {
+                     Ctrl *ctrl, WaitCfg wc, unsigned int *flags, unsigned int *done, uint32_t ring,
+                     uint32_t stage_bytes, bool ahead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    K *sm = tile_smem<K>(smem_raw);
-    __shared__ __align__(16) unsigned char s_plan[2][sizeof(BatchInst)];
-    __shared__ unsigned long long s_t;  // the current ticket
-    __shared__ uint32_t s_j, s_k;       // its owner and (a tile) its tile
-    __shared__ uint32_t s_nj;           // the owner of the next ticket (kNoInst past the end)
-    __shared__ uint32_t s_held[2];      // the instance whose plan each buffer holds
-    __shared__ uint32_t s_k1, s_j2;     // the tile of the next ticket, the owner of the one after
-    __shared__ int s_ok;
-    __shared__ TileShared ts;
+    __shared__ __align__(16) unsigned char s_raw[kBatchStages * sizeof(BatchStage)];
+    BatchStage *s_st = reinterpret_cast<BatchStage *>(s_raw);
+    // per stage: claimed (its first warp has its ticket), plan (the item is known), ready, empty
+    __shared__ uint64_t s_claimed[kBatchStages], s_plan[kBatchStages], s_ready[kBatchStages], s_empty[kBatchStages];
     const uint64_t total = tot.tiles + tot.chunks;
-    uint32_t t1 = 0, t2 = 0;  // thread 0: the next ticket and the one after (below 2^31, as built)
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
-        const unsigned long long t0 = atomicAdd(&ctrl->ticket, 1ull);
-        t1 = (uint32_t)atomicAdd(&ctrl->ticket, 1ull);
-        t2 = (uint32_t)atomicAdd(&ctrl->ticket, 1ull);
-        s_t = t0;
-        s_j = t0 < total ? owner[t0] : kNoInst;
-        s_k = t0 < tot.tiles ? tile[t0] : 0;
-        s_nj = t1 < total ? owner[t1] : kNoInst;
-        s_held[0] = s_held[1] = kNoInst;
+        for (uint32_t s = 0; s < ring; ++s) {
+            mbar_init(&s_claimed[s], 1);
+            mbar_init(&s_plan[s], 1);
+            mbar_init(&s_ready[s], 2);
+            mbar_init(&s_empty[s], kStoreWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    while (s_t < total) {
-        const unsigned long long t = s_t;
-        const uint32_t j = s_j, nj = s_nj;
-        uint32_t t3 = 0;
-        if (threadIdx.x == 0) {  // read as the item ends
-            if (t1 < tot.tiles)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(&s_k1)),
-                             "l"(tile + t1) : "memory");
-            if (t2 < total)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(&s_j2)),
-                             "l"(owner + t2) : "memory");
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            t3 = (uint32_t)atomicAdd(&ctrl->ticket, 1ull);
-        }
-        int cb = s_held[0] == j ? 0 : s_held[1] == j ? 1 : -1;
-        if (cb < 0) {  // not prefetched (the block's first item): copy it now
-            cb = s_held[0] == nj ? 1 : 0;
-            const uint4 *src = reinterpret_cast<const uint4 *>(inst + j);
-            uint4 *dst = reinterpret_cast<uint4 *>(s_plan[cb]);
-            for (uint32_t w = threadIdx.x; w < kPlanWords; w += blockDim.x) dst[w] = src[w];
-            __syncthreads();
-            if (threadIdx.x == 0) s_held[cb] = j;  // read again only after the next barrier
-        }
-        const BatchInst &I = *reinterpret_cast<const BatchInst *>(s_plan[cb]);
-        const bool pf = nj != kNoInst && nj != j && s_held[1 - cb] != nj;
-        if (pf) prefetch_plan(inst, nj, s_plan[1 - cb]);
-        const bool is_tile = t < tot.tiles;
-        if (is_tile) {
-            btree_stream_tile(I.S, keys + I.off, scr + I.scr_base, flags + I.tile_base, ctrl, wc, s_k, sm, ts);
-        } else {
-            if (threadIdx.x == 0) s_ok = wait_flag(&done[j], (unsigned int)I.S.ntiles, ctrl, wc) ? 1 : 0;
-            __syncthreads();
-            if (s_ok) {
-                const uint64_t c = t - tot.tiles - I.chunk_base;
-                if (I.S.plan == PLAN_O)
-                    batch_copy_items(keys, scr, I, items, citem, c);
-                else
-                    batch_copy_ranges(keys, scr, I, c);
+    auto wait_bar = [&](uint64_t *bar, uint32_t parity) {
+        const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_long(bar, parity));
+        if (!ok && lane == 0) atomicOr(&ctrl->error, 1u << TL_ERROR_TIMEOUT);
+        return ok;
+    };
+    uint32_t phase = 0;
+    if (warp < kBatchStages) {  // a stage's first warp
+        const uint32_t s = warp;
+        if (s >= ring) return;
+        BatchStage &T = s_st[s];
+        K *sm = tile_smem<K>(smem_raw) + (size_t)s * (stage_bytes / sizeof(K));
+        uint32_t held = kNoInst, stored = kNoInst;  // the instance whose plan is at hand; of the tile being stored
+        while (true) {
+            // the next item's ticket and plan, while this stage's item is being stored
+            if (!ahead && !wait_bar(&s_empty[s], phase ^ 1)) return;
+            if (!wait_bar(&s_claimed[s ? s - 1 : ring - 1], s ? phase : phase ^ 1)) return;
+            unsigned long long t = 0;
+            if (lane == 0) {
+                t = atomicAdd(&ctrl->ticket, 1ull);
+                T.next = t;  // and so has its value before the next stage claims
+                mbar_arrive(&s_claimed[s]);
             }
-            load_tile_wait();  // the plan prefetch, where there is one
-        }
-        __syncthreads();  // the item is done (every store of a tile issued); a prefetched plan has landed
-        if (threadIdx.x == 0) {
-            const unsigned long long n = t1;
-            load_tile_wait();
-            const uint32_t k1 = t1 < tot.tiles ? s_k1 : 0, j2 = t2 < total ? s_j2 : kNoInst;
-            if (is_tile) {  // the tile's stores, every thread's, before its count
+            t = __shfl_sync(0xFFFFFFFFu, t, 0);
+            const bool is_tile = t < tot.tiles;
+            const uint32_t j = t < total ? owner[t] : kNoInst;
+            const uint64_t k = is_tile ? tile[t] : 0;
+            const bool other = t < total && j != held;
+            uint4 plan[(kPlanWords + 31) / 32];  // in registers until the stage's own copy is free
+            if (other) {
+                const uint4 *src = reinterpret_cast<const uint4 *>(inst + j);
+#pragma unroll
+                for (uint32_t i = 0; i < (kPlanWords + 31) / 32; ++i)
+                    if (lane + 32 * i < kPlanWords) plan[i] = src[lane + 32 * i];
+                held = j;
+            }
+            if (!wait_bar(&s_empty[s], phase ^ 1)) return;
+            if (other) {
+                uint4 *dst = reinterpret_cast<uint4 *>(&T.I);
+#pragma unroll
+                for (uint32_t i = 0; i < (kPlanWords + 31) / 32; ++i)
+                    if (lane + 32 * i < kPlanWords) dst[lane + 32 * i] = plan[i];
+                __syncwarp();
+            }
+            const BatchInst &I = T.I;
+            const BtreeStream &S = I.S;
+            K *A = keys + I.off;
+            unsigned int *fl = flags + I.tile_base;
+            uint64_t p0 = 0, p1 = 0, w_lo = 1, w_hi = 0;
+            if (lane == 0) {
+                T.t = t;
+                T.kind = is_tile ? kItemTile : t < total ? kItemChunk : kItemNone;
+            }
+            if (is_tile) {
+                btree_tile(S, k, p0, p1);
+                const uint64_t base = tile_base(A, p0);
+                if (lane == 0) {
+                    T.p0 = p0, T.p1 = p1, T.base = base;
+                    T.ts.ok0 = T.ts.ok1 = 1;
+                    mbar_arrive(&s_plan[s]);
+                }
+                load_tile_issue(A, p0, p1, sm, lane, 32);
+            }
+            if (stored != kNoInst && lane == 0) {  // the last tile's stores, every warp's, before its count
                 __threadfence();
-                atomicAdd(&done[j], 1u);
+                atomicAdd(&done[stored], 1u);
             }
-            if (pf) s_held[1 - cb] = nj;
-            s_t = n;
-            s_j = nj;
-            s_k = k1;
-            s_nj = j2;
-            t1 = t2;
-            t2 = t3;
+            stored = kNoInst;
+            if (is_tile) {
+                if (lane == 0) T.ts.reg = btree_stream_regime(S, p0, p1);
+                // a look at the flags while the copies are in flight mostly finds them set
+                bool pending = false;
+                if (btree_tile_wait(S, p0, p1, w_lo, w_hi))
+                    for (uint64_t f = w_lo + lane; f <= w_hi; f += 32)
+                        if (f != k && !(S.plan == PLAN_O && !btree_o_direct(S, k, f)))  // else its keys go to scratch
+                            pending |= ld_acquire(&fl[f]) != wc.wait_value;
+                load_tile_wait();
+                __syncwarp();
+                if (lane == 0) st_relaxed(&fl[k], wc.flag_value);  // published: every copy has landed
+                if (pending)
+                    for (uint64_t f = w_lo + lane; f <= w_hi; f += 32)
+                        if (f != k && !(S.plan == PLAN_O && !btree_o_direct(S, k, f)))
+                            if (!wait_flag(&fl[f], wc.wait_value, ctrl, wc)) T.ts.ok1 = 0;
+                stored = j;
+            } else if (lane == 0) {
+                mbar_arrive(&s_plan[s]);
+                if (t < total) T.ts.ok1 = wait_flag(&done[j], (unsigned int)S.ntiles, ctrl, wc) ? 1 : 0;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_ready[s]);
+            if (t >= total) return;
+            phase ^= 1;
         }
-        __syncthreads();
+    } else if (warp < 2 * kBatchStages) {  // a stage's second warp
+        const uint32_t s = warp - kBatchStages;
+        if (s >= ring) return;
+        BatchStage &T = s_st[s];
+        while (wait_bar(&s_plan[s], phase)) {
+            const int kind = T.kind;
+            const BatchInst &I = T.I;
+            if (kind == kItemTile)
+                btree_tile_runs_warp(I.S, T.p0, T.p1, reinterpret_cast<uintptr_t>(keys + I.off),
+                                     reinterpret_cast<uintptr_t>(scr + I.scr_base), (uint32_t)sizeof(K),
+                                     flags + I.tile_base, ctrl, wc, T.ts);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_ready[s]);
+            if (kind == kItemNone) break;
+            phase ^= 1;
+        }
+    } else {  // store warps
+        const uint32_t tb = threadIdx.x - 64 * kBatchStages, nb = 32 * kStoreWarps;
+        uint32_t s = 0;
+        while (wait_bar(&s_ready[s], phase)) {
+            const BatchStage &T = s_st[s];
+            if (T.kind == kItemNone) break;
+            const BatchInst &I = T.I;
+            if (T.kind == kItemTile) {
+                if (T.ts.ok0 && T.ts.ok1) {
+                    const K *tl = tile_smem<K>(smem_raw) + (size_t)s * (stage_bytes / sizeof(K)) + (T.p0 - T.base);
+                    btree_store_bulk(I.S, keys + I.off, scr + I.scr_base, ctrl, T.p0, T.p1, tl, T.ts, tb, nb);
+                    btree_store_top<K, true>(I.S, tl, T.ts, tb, nb);
+                }
+            } else if (T.ts.ok1) {
+                const uint64_t c = T.t - tot.tiles - I.chunk_base;
+                if (I.S.plan == PLAN_O)
+                    batch_copy_items(keys, scr, I, items, citem, c, tb, nb);
+                else
+                    batch_copy_ranges(keys, scr, I, c, tb, nb);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_empty[s]);
+            if (++s == ring) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
     }
 }
 
@@ -891,17 +966,21 @@ static int launch_batch_permute(const tl_batch_plan_impl &P, K *keys, char *ws, 
     wc.flag_value = 1;
     wc.wait_value = debug_force_timeout() ? 0xFFFFFFFFu : 1u;
     wc.spin_limit = debug_spin_limit();
-    const size_t smem = (size_t)P.tot.max_tile * sizeof(K) + kTileSmemSlack;  // the largest tile
-    auto kern = threads == 512 ? batch_permute_kernel<K, 512, kBatchBlocksPerSM512>
-                               : batch_permute_kernel<K, 256, kBatchBlocksPerSM256>;
+    // as many stages as let kBatchBlocksPerSM blocks share an SM, each for the largest tile
+    const size_t stage = ((size_t)P.tot.max_tile * sizeof(K) + 128 + 127) / 128 * 128;
+    uint32_t ring = (uint32_t)std::max<size_t>(1, std::min<size_t>(kBatchStages, (kBatchBlockSmem - 128) / stage));
+    const size_t smem = ring * stage + 128;
+    auto kern = threads == 512 ? batch_permute_kernel<K, kBatchStoreWarps512> : batch_permute_kernel<K, kBatchStoreWarps256>;
+    const int nthreads = 32 * (2 * kBatchStages + (threads == 512 ? kBatchStoreWarps512 : kBatchStoreWarps256));
     TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nthreads, smem));
     const uint64_t work = P.tot.tiles + P.tot.chunks;
     if (work == 0) return TL_SUCCESS;
     const uint64_t grid = std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * batch_sms(), work);
-    kern<<<(unsigned)grid, threads, smem, st>>>(keys, scr, P.inst, P.owner, P.tile, P.items, P.citem, P.tot, ctrl, wc,
-                                                 flags, done);
+    ring = (uint32_t)std::min<uint64_t>(ring, (work + grid - 1) / grid);
+    kern<<<(unsigned)grid, nthreads, smem, st>>>(keys, scr, P.inst, P.owner, P.tile, P.items, P.citem, P.tot, ctrl, wc,
+                                                 flags, done, ring, (uint32_t)stage, work >= kClaimAheadItems * grid * ring);
     TL_CUDA_TRY(cudaGetLastError());
     return TL_SUCCESS;
 }

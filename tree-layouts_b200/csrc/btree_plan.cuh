@@ -642,7 +642,7 @@ struct TileShared {
     Regime reg;
 };
 
-// Warp 0's part of btree_stream_tile: the tile's runs (one lane per slot, a
+// One warp's part of a stream tile: the tile's runs (one lane per slot, a
 // slot per level of each group of top keys, with their plan-O table lookups),
 // their prefix sums and store bases, and the waits for the tiles under their
 // direct parts.  Kept out of line so that its 64-bit state does not crowd the
@@ -651,7 +651,7 @@ static __device__ __noinline__ void btree_tile_runs_warp(const BtreeStream &S, u
                                                          uintptr_t ab, uintptr_t sb, uint32_t kb,
                                                          unsigned int *flags, Ctrl *ctrl, const WaitCfg &wc,
                                                          TileShared &ts) {
-    const uint32_t lane = threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31;
     const uint64_t own = p0 >> S.tile_shift;
     TopGroup G0{}, G1{};
     const int ng = btree_stream_groups(S, p0, p1, G0, G1);
@@ -702,6 +702,93 @@ __device__ __forceinline__ void bar_sync_tail() {
     asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x - 32) : "memory");
 }
 
+// A stream tile's bulk keys, stored by threads tb of nb: [p0, p1) sits at tile[0..].
+template <typename K>
+__device__ __forceinline__ void btree_store_bulk(const BtreeStream &S, K *__restrict__ A, K *__restrict__ scr, Ctrl *ctrl,
+                                                 uint64_t p0, uint64_t p1, const K *tile, const TileShared &ts,
+                                                 uint32_t tb, uint32_t nb) {
+    const uint32_t cnt = (uint32_t)(p1 - p0);
+    const Regime &R = ts.reg;  // fields read from shared memory where used
+    if (R.kind == 0) {
+        for (uint64_t x = p0 + tb; x < p1; x += nb) {
+            if (btree_is_top(S, x)) continue;
+            uint64_t idx;
+            const K key = tile[x - p0];
+            if (btree_place(S, x, idx))
+                A[idx] = key;
+            else if (idx < S.nscratch)
+                scr[idx] = key;
+            else
+                btree_o_bad(ctrl);
+        }
+    } else if (R.kind == 1) {
+        // the loops keep the regime in registers (stores through K * could alias it)
+        K *tgt = (R.to_A ? A : scr) + R.dbase;
+        const FastDiv32 fd = S.fd32;
+        const uint32_t d = fd.d, r0 = R.r0, skip = R.skip;
+#pragma unroll 4
+        for (uint32_t o = tb; o < cnt; o += nb) {
+            const uint32_t v = r0 + o;
+            const uint32_t ql = fd.div(v);
+            if (v - ql * d != skip) tgt[v - ql] = tile[o];
+        }
+    } else if (R.kind == 3 && !btree_regime_ok(S, R, cnt)) {
+        if (tb == 0) btree_o_bad(ctrl);
+    } else if (R.kind == 3) {
+        K *tlo = (R.to_A ? A : scr + R.slo) + R.dbase, *thi = (R.hi_A ? A : scr + R.shi) + R.dbase;
+        const FastDiv32 fd = S.fd32;
+        const uint32_t d = fd.d, r0 = R.r0, skip = R.skip;
+        const uint32_t split = (uint32_t)(R.dsplit - R.dbase);  // below tile_keys + b
+#pragma unroll 4
+        for (uint32_t o = tb; o < cnt; o += nb) {
+            const uint32_t v = r0 + o;
+            const uint32_t ql = fd.div(v);
+            const uint32_t j = v - ql;
+            if (v - ql * d != skip) (j < split ? tlo : thi)[j] = tile[o];
+        }
+    }
+}
+
+// A stream tile's top keys, stored by threads tb of nb.  kRunRegs keeps the
+// current store run in registers across the loop instead of reading it from
+// shared memory for every key (the BST instance: many short runs per tile;
+// measured +3 % there, but not for b = 16, whose kernel keeps the
+// shared-memory reads and its lower register count).
+template <typename K, bool kRunRegs = false>
+__device__ __forceinline__ void btree_store_top(const BtreeStream &S, const K *tile, const TileShared &ts, uint32_t tb,
+                                                uint32_t nb) {
+    // top keys, level by level: consecutive threads store consecutive positions
+    const FastDiv32 fdb = S.fd32b;
+    const bool bst = S.g.b == 1;
+    const uint32_t total = ts.cum[ts.nslots];
+    uint32_t r = 0;  // the run of gi only moves forward as gi grows
+    if constexpr (kRunRegs) {
+        uint32_t c0 = ts.cum[0], c1 = ts.cum[1];
+        StoreRun run = ts.runs[0];
+        for (uint32_t gi = tb; gi < total; gi += nb) {
+            if (gi >= c1) {
+                do {
+                    ++r;
+                } while (gi >= ts.cum[r + 1]);
+                c0 = ts.cum[r];
+                c1 = ts.cum[r + 1];
+                run = ts.runs[r];
+            }
+            const uint32_t e = gi - c0;
+            K *dst = reinterpret_cast<K *>(e < run.nlo ? run.blo : run.bhi);
+            dst[e] = tile[run.off0 + (e + (bst ? e : fdb.div(run.rb + e))) * run.mult];
+        }
+    } else {
+        for (uint32_t gi = tb; gi < total; gi += nb) {
+            while (gi >= ts.cum[r + 1]) ++r;
+            const StoreRun run = ts.runs[r];
+            const uint32_t e = gi - ts.cum[r];
+            K *dst = reinterpret_cast<K *>(e < run.nlo ? run.blo : run.bhi);
+            dst[e] = tile[run.off0 + (e + (bst ? e : fdb.div(run.rb + e))) * run.mult];
+        }
+    }
+}
+
 // Stream pass for tile k of one array (block-wide).  False if a bounded wait
 // expired (the tile's stores were skipped and the error is recorded).  Warps
 // 1.. load the tile, publish it and store its bulk keys (after waiting for the
@@ -709,11 +796,7 @@ __device__ __forceinline__ void bar_sync_tail() {
 // lane per level, with their table lookups) and waits for the tiles under
 // their direct parts, so that its work stays off the load's path.  Then the
 // whole block stores the top keys.  Every wait is on a tile with an earlier
-// ticket, and the publish does not depend on warp 0.  kRunRegs keeps the
-// current store run in registers across the top-key loop instead of reading it
-// from shared memory for every key (the BST instance: many short runs per
-// tile; measured +3 % there, but not for b = 16, whose kernel keeps the
-// shared-memory reads and its lower register count).
+// ticket, and the publish does not depend on warp 0.
 template <typename K, bool kRunRegs = false>
 __device__ __forceinline__ bool btree_stream_tile(const BtreeStream &S, K *__restrict__ A, K *__restrict__ scr,
                                                   unsigned int *flags, Ctrl *ctrl, const WaitCfg &wc, uint64_t k,
@@ -721,7 +804,6 @@ __device__ __forceinline__ bool btree_stream_tile(const BtreeStream &S, K *__res
     uint64_t p0, p1;
     btree_tile(S, k, p0, p1);
     const uint64_t base = tile_base(A, p0);
-    const uint32_t cnt = (uint32_t)(p1 - p0);
     const K *tile = sm + (p0 - base);
     if (threadIdx.x < 32) {
         if (threadIdx.x == 0) ts.ok0 = 1;  // the previous tile's readers are past the ticket barrier
@@ -745,76 +827,11 @@ __device__ __forceinline__ bool btree_stream_tile(const BtreeStream &S, K *__res
                 if (!wait_flag(&flags[f], wc.wait_value, ctrl, wc)) ts.ok1 = 0;
             }
         bar_sync_tail();
-        if (ts.ok1) {
-            const Regime &R = ts.reg;  // fields read from shared memory where used
-            if (R.kind == 0) {
-                for (uint64_t x = p0 + tb; x < p1; x += nb) {
-                    if (btree_is_top(S, x)) continue;
-                    uint64_t idx;
-                    const K key = sm[x - base];
-                    if (btree_place(S, x, idx))
-                        A[idx] = key;
-                    else if (idx < S.nscratch)
-                        scr[idx] = key;
-                    else
-                        btree_o_bad(ctrl);
-                }
-            } else if (R.kind == 1) {
-                // the loops keep the regime in registers (stores through K * could alias it)
-                K *tgt = (R.to_A ? A : scr) + R.dbase;
-                const uint32_t d = S.fd32.d, r0 = R.r0, skip = R.skip;
-#pragma unroll 4
-                for (uint32_t o = tb; o < cnt; o += nb) {
-                    const uint32_t v = r0 + o;
-                    const uint32_t ql = S.fd32.div(v);
-                    if (v - ql * d != skip) tgt[v - ql] = tile[o];
-                }
-            } else if (R.kind == 3 && !btree_regime_ok(S, R, cnt)) {
-                if (tb == 0) btree_o_bad(ctrl);
-            } else if (R.kind == 3) {
-                K *tlo = (R.to_A ? A : scr + R.slo) + R.dbase, *thi = (R.hi_A ? A : scr + R.shi) + R.dbase;
-                const uint32_t d = S.fd32.d, r0 = R.r0, skip = R.skip;
-                const uint32_t split = (uint32_t)(R.dsplit - R.dbase);  // below tile_keys + b
-#pragma unroll 4
-                for (uint32_t o = tb; o < cnt; o += nb) {
-                    const uint32_t v = r0 + o;
-                    const uint32_t ql = S.fd32.div(v);
-                    const uint32_t j = v - ql;
-                    if (v - ql * d != skip) (j < split ? tlo : thi)[j] = tile[o];
-                }
-            }
-        }
+        if (ts.ok1) btree_store_bulk(S, A, scr, ctrl, p0, p1, tile, ts, tb, nb);
     }
     __syncthreads();
     if (!ts.ok0 || !ts.ok1) return false;
-    // top keys, level by level: consecutive threads store consecutive positions
-    const uint32_t total = ts.cum[ts.nslots];
-    uint32_t r = 0;  // the run of gi only moves forward as gi grows
-    if constexpr (kRunRegs) {
-        uint32_t c0 = ts.cum[0], c1 = ts.cum[1];
-        StoreRun run = ts.runs[0];
-        for (uint32_t gi = threadIdx.x; gi < total; gi += blockDim.x) {
-            if (gi >= c1) {
-                do {
-                    ++r;
-                } while (gi >= ts.cum[r + 1]);
-                c0 = ts.cum[r];
-                c1 = ts.cum[r + 1];
-                run = ts.runs[r];
-            }
-            const uint32_t e = gi - c0;
-            K *dst = reinterpret_cast<K *>(e < run.nlo ? run.blo : run.bhi);
-            dst[e] = tile[btree_top_item_off(S, run, e)];
-        }
-    } else {
-        for (uint32_t gi = threadIdx.x; gi < total; gi += blockDim.x) {
-            while (gi >= ts.cum[r + 1]) ++r;
-            const StoreRun run = ts.runs[r];
-            const uint32_t e = gi - ts.cum[r];
-            K *dst = reinterpret_cast<K *>(e < run.nlo ? run.blo : run.bhi);
-            dst[e] = tile[btree_top_item_off(S, run, e)];
-        }
-    }
+    btree_store_top<K, kRunRegs>(S, tile, ts, threadIdx.x, blockDim.x);
     return true;
 }
 
@@ -959,13 +976,12 @@ TL_HD bool btree_copy_range(const BtreeStream &S, int j, CopyRange &r) {
 // per thread in flight, all from one contiguous stretch, so the DRAM rows it
 // touches stay few.  The scratch is read once, so its loads are streaming.
 template <typename K, int kUnr = 4>
-__device__ __forceinline__ void copy_keys(K *__restrict__ dst, const K *__restrict__ src, uint64_t len,
-                                          uint64_t blk, uint64_t nblk) {
+__device__ __forceinline__ void copy_keys(K *__restrict__ dst, const K *__restrict__ src, uint64_t len, uint32_t tid,
+                                          uint32_t nt) {
     constexpr uint32_t V = 16 / sizeof(K);
-    const uint64_t tid = blk * blockDim.x + threadIdx.x;
     const uintptr_t da = reinterpret_cast<uintptr_t>(dst), sa = reinterpret_cast<uintptr_t>(src);
     if (((da ^ sa) & 15) != 0) {
-        for (uint64_t x = tid; x < len; x += nblk * blockDim.x) dst[x] = __ldcs(src + x);
+        for (uint64_t x = tid; x < len; x += nt) dst[x] = __ldcs(src + x);
         return;
     }
     uint64_t head = ((16 - (da & 15)) & 15) / sizeof(K);
@@ -976,17 +992,17 @@ __device__ __forceinline__ void copy_keys(K *__restrict__ dst, const K *__restri
     if (tid < len - tail0) dst[tail0 + tid] = __ldcs(src + tail0 + tid);
     uint4 *dv = reinterpret_cast<uint4 *>(dst + head);
     const uint4 *sv = reinterpret_cast<const uint4 *>(src + head);
-    const uint64_t chunk = (uint64_t)kUnr * blockDim.x;
-    for (uint64_t c0 = blk * chunk; c0 < nvec; c0 += nblk * chunk) {
+    const uint64_t chunk = (uint64_t)kUnr * nt;
+    for (uint64_t c0 = 0; c0 < nvec; c0 += chunk) {
         uint4 a[kUnr];
 #pragma unroll
         for (int u = 0; u < kUnr; ++u) {
-            const uint64_t v = c0 + u * blockDim.x + threadIdx.x;
+            const uint64_t v = c0 + u * nt + tid;
             if (v < nvec) a[u] = __ldcs(sv + v);
         }
 #pragma unroll
         for (int u = 0; u < kUnr; ++u) {
-            const uint64_t v = c0 + u * blockDim.x + threadIdx.x;
+            const uint64_t v = c0 + u * nt + tid;
             if (v < nvec) dv[v] = a[u];
         }
     }

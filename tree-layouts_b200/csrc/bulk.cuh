@@ -67,18 +67,30 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 }
 
 // Bounded wait for phase `parity` of an mbarrier.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned int limit = kBulkSpinLimit) {
-    for (unsigned int it = 0; it <= limit; ++it) {
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
+    for (unsigned int it = 0; it <= kBulkSpinLimit; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         __nanosleep(64);
     }
     return false;
 }
 
-// For a phase that another warp's read-flag wait may hold up (about a second):
-// the bound lies several times above that wait's.
+// For a phase that another warp's read-flag waits may hold up (each bounded by
+// a few seconds): bounded by time, 20 s, as a try_wait may itself suspend.
+__device__ __forceinline__ uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 __device__ __forceinline__ bool mbar_wait_long(uint64_t *bar, uint32_t parity) {
-    return mbar_wait(bar, parity, kBulkSpinLimit * 16u);
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = global_ns();
+    do {
+        __nanosleep(64);
+        if (mbar_try_wait(bar, parity)) return true;
+    } while (global_ns() - t0 < 20000000000ull);
+    return false;
 }
 
 __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, uint32_t bytes, uint64_t *bar) {
