@@ -192,3 +192,18 @@ def test_veb_stream_expired_wait_reports_timeout():
     t = to_dev(keys)
     T.permute("mveb", t)
     assert np.array_equal(from_dev(t), O.permute("mveb", keys, 16))
+
+
+@pytest.mark.parametrize("layout,b", [("btree", 8), ("btree", 16), ("bst", 1)])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+@pytest.mark.parametrize("tiles", [385, 593, 900, 3551, 3600])
+def test_btree_stream_ring_of_stages(layout, b, dtype, tiles):
+    """From the smallest arrays that move by tiles: one to four tiles a block, and both sides of the count from
+    which tiles are claimed ahead (4 for each of 3 stages of 2 blocks on 148 SMs), off the 16-byte boundary."""
+    n = tiles * 32768 // np.dtype(dtype).itemsize - 37
+    keys = data.sorted_keys_np(n, 1, 5, n, dtype)
+    buf = to_dev(np.concatenate([np.zeros(1, dtype), keys, np.zeros(1, dtype)]))
+    T.permute(layout, buf[1:1 + n], b)
+    out = from_dev(buf)
+    assert np.array_equal(out[1:1 + n], O.permute(layout, keys, b))
+    assert out[0] == 0 and out[-1] == 0

@@ -38,10 +38,6 @@ constexpr int kBatchThreads = 256;     // query kernel
 // 2^8..2^14: 73, 80 and 88 us; at 10 and more the registers spill (1.9 ms).
 constexpr int kBatchStages = 3, kBatchBlocksPerSM = 2;
 constexpr int kBatchStoreWarps256 = 8, kBatchStoreWarps512 = 4;
-// Launches with fewer items a stage than this claim an item only when its stage
-// is empty: claimed ahead, the last items queue up behind others (2^8..2^14
-// keys: 81 us ahead, 73 not; large batches gain 2 % from it).
-constexpr uint64_t kClaimAheadItems = 4;
 constexpr size_t kBatchBlockSmem = 100 * 1024;  // dynamic shared memory of a block, beside the stages' plans
 constexpr int kMaxClass = 48;
 

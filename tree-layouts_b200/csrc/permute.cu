@@ -37,8 +37,6 @@
 
 namespace tl {
 
-constexpr int kStreamThreads = 256;
-constexpr int kStreamBlocksPerSM = 6;  // what shared memory allows with 32 KB tiles
 constexpr uint32_t kUnitMaxLevels = 8;
 // mveb_stream_kernel: 32 KB stages a block, blocks per SM (the shared memory of
 // six tiles an SM), store warps a block (after the loader, publisher and waiter).
@@ -55,19 +53,139 @@ constexpr uint64_t stream_tile_keys() {
 
 static inline uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
-// kBst: the instance for b = 1 (see btree_stream_tile's kRunRegs).
+constexpr int kBtreeStages = 3, kBtreeBlocksPerSM = 2, kBtreeStoreWarps = 8;
+constexpr int kBtreeThreads = 32 * (2 * kBtreeStages + kBtreeStoreWarps);
+
+struct BtreeStage {
+    TileShared ts;
+    uint64_t ticket, p0, p1, base;
+    int last;  // no tile is left
+};
+
+// A ring of three 32 KB stages a block.  A stage's first warp claims a tile, loads
+// it, publishes it as read and waits for the tiles under its bulk keys; its second
+// warp works out the tile's runs of top keys (one lane per level, with their table
+// lookups) and waits for the tiles under their direct parts; the store warps take
+// the stages in turn and meet at no barrier.  Stages claim in turn, so a block
+// stores in ticket order, and every wait is on a tile with an earlier ticket: the
+// smallest tile not yet stored is its block's next and always progresses.  With
+// `ahead` (kClaimAheadItems tiles a stage or more) a stage claims its next tile
+// while its present one is stored.  The bound is the copy rate: with a block
+// holding one tile at a time (load, publish, wait, store; six blocks an SM) the
+// phases overlapped only between blocks.  Measured on B200, device time of the
+// whole permutation: b = 16, 5e8 u64 keys 1361 -> 1287 us (1313 not ahead), u32
+// 928 -> 832; b = 8, 2^24 u32 82 -> 71; BST of 2^27 - 1 u64 536 -> 494.  With 4
+// store warps 1334, 1049, 85 and 577, with 16 (spills) 1462, 895, 72 and 546.
+// kBst: the instance for b = 1 (see btree_store_top's kRunRegs).
 template <typename K, bool kBst = false>
-__global__ void __launch_bounds__(kStreamThreads, kStreamBlocksPerSM)
+__global__ void __launch_bounds__(kBtreeThreads, kBtreeBlocksPerSM)
 btree_stream_kernel(K *__restrict__ A, K *__restrict__ scr, const __grid_constant__ BtreeStream S, Ctrl *ctrl,
-                    WaitCfg wc, unsigned int *flags) {
+                    WaitCfg wc, unsigned int *flags, uint32_t ring, uint32_t stage_keys, bool ahead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    K *sm = tile_smem<K>(smem_raw);
-    __shared__ unsigned long long s_ticket;
-    __shared__ TileShared ts;
-    TicketPipe tp;
-    for (unsigned long long t = ticket_first(ctrl, &s_ticket); t < S.ntiles; t = ticket_advance(tp, &s_ticket)) {
-        ticket_claim(ctrl, tp);
-        btree_stream_tile<K, kBst>(S, A, scr, flags, ctrl, wc, btree_tile_of_ticket(S, t), sm, ts);
+    __shared__ BtreeStage s_st[kBtreeStages];
+    __shared__ uint64_t s_claimed[kBtreeStages], s_tile[kBtreeStages], s_ready[kBtreeStages], s_empty[kBtreeStages];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < ring; ++s) {
+            mbar_init(&s_claimed[s], 1);
+            mbar_init(&s_tile[s], 1);
+            mbar_init(&s_ready[s], 2);
+            mbar_init(&s_empty[s], kBtreeStoreWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    auto wait_bar = [&](uint64_t *bar, uint32_t parity) {
+        const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_long(bar, parity));
+        if (!ok && lane == 0) atomicOr(&ctrl->error, 1u << TL_ERROR_TIMEOUT);
+        return ok;
+    };
+    uint32_t phase = 0;
+    if (warp < kBtreeStages) {  // a stage's first warp
+        const uint32_t s = warp;
+        if (s >= ring) return;
+        BtreeStage &T = s_st[s];
+        K *sm = tile_smem<K>(smem_raw) + (size_t)s * stage_keys;
+        while (true) {
+            if (!ahead && !wait_bar(&s_empty[s], phase ^ 1)) return;
+            if (!wait_bar(&s_claimed[s ? s - 1 : ring - 1], s ? phase : phase ^ 1)) return;
+            unsigned long long t = 0;
+            if (lane == 0) {
+                t = atomicAdd(&ctrl->ticket, 1ull);
+                T.ticket = t;  // and so has its value before the next stage claims
+                mbar_arrive(&s_claimed[s]);
+            }
+            t = __shfl_sync(0xFFFFFFFFu, t, 0);
+            const uint64_t k = t < S.ntiles ? btree_tile_of_ticket(S, t) : 0;
+            if (!wait_bar(&s_empty[s], phase ^ 1)) return;
+            if (t >= S.ntiles) {
+                if (lane == 0) {
+                    T.last = 1;
+                    mbar_arrive(&s_tile[s]);
+                    mbar_arrive(&s_ready[s]);
+                }
+                return;
+            }
+            uint64_t p0, p1, w_lo, w_hi;
+            btree_tile(S, k, p0, p1);
+            const uint64_t base = tile_base(A, p0);
+            if (lane == 0) {
+                T.last = 0;
+                T.p0 = p0, T.p1 = p1, T.base = base;
+                T.ts.ok0 = T.ts.ok1 = 1;
+                mbar_arrive(&s_tile[s]);
+            }
+            load_tile_issue(A, p0, p1, sm, lane, 32);
+            if (lane == 0) T.ts.reg = btree_stream_regime(S, p0, p1);
+            // a look at the flags while the copies are in flight mostly finds them set
+            bool pending = false;
+            if (btree_tile_wait(S, p0, p1, w_lo, w_hi))
+                for (uint64_t f = w_lo + lane; f <= w_hi; f += 32)
+                    if (f != k && !(S.plan == PLAN_O && !btree_o_direct(S, k, f)))  // else its keys go to scratch
+                        pending |= ld_acquire(&flags[f]) != wc.wait_value;
+            load_tile_wait();
+            __syncwarp();
+            if (lane == 0) st_relaxed(&flags[k], wc.flag_value);  // published: every copy has landed
+            if (pending)
+                for (uint64_t f = w_lo + lane; f <= w_hi; f += 32)
+                    if (f != k && !(S.plan == PLAN_O && !btree_o_direct(S, k, f)))
+                        if (!wait_flag(&flags[f], wc.wait_value, ctrl, wc)) T.ts.ok1 = 0;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_ready[s]);
+            phase ^= 1;
+        }
+    } else if (warp < 2 * kBtreeStages) {  // a stage's second warp
+        const uint32_t s = warp - kBtreeStages;
+        if (s >= ring) return;
+        BtreeStage &T = s_st[s];
+        while (wait_bar(&s_tile[s], phase)) {
+            const int last = T.last;
+            if (!last)
+                btree_tile_runs_warp(S, T.p0, T.p1, reinterpret_cast<uintptr_t>(A), reinterpret_cast<uintptr_t>(scr),
+                                     (uint32_t)sizeof(K), flags, ctrl, wc, T.ts);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_ready[s]);
+            if (last) break;
+            phase ^= 1;
+        }
+    } else {  // store warps
+        const uint32_t tb = threadIdx.x - 64 * kBtreeStages, nb = 32 * kBtreeStoreWarps;
+        uint32_t s = 0;
+        while (wait_bar(&s_ready[s], phase)) {
+            const BtreeStage &T = s_st[s];
+            if (T.last) break;
+            if (T.ts.ok0 && T.ts.ok1) {
+                const K *tl = tile_smem<K>(smem_raw) + (size_t)s * stage_keys + (T.p0 - T.base);
+                btree_store_bulk(S, A, scr, ctrl, T.p0, T.p1, tl, T.ts, tb, nb);
+                btree_store_top<K, kBst>(S, tl, T.ts, tb, nb);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_empty[s]);
+            if (++s == ring) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
     }
 }
 
@@ -421,7 +539,6 @@ static int launch_permute_k(const PermutePlan &pl, K *A, char *ws, cudaStream_t 
     wc.spin_limit = debug_spin_limit();
     // flags and control block are contiguous: one stream-ordered memset clears both
     TL_CUDA_TRY(cudaMemsetAsync(flags, 0, pl.bytes - pl.off_flags, st));
-    const size_t smem = (size_t)pl.tile_keys * sizeof(K) + kTileSmemSlack;
     const int smx = sm_count();
     if (is_veb_layout(pl.layout)) {
         auto kern = mveb_stream_kernel<K>;
@@ -446,11 +563,16 @@ static int launch_permute_k(const PermutePlan &pl, K *A, char *ws, cudaStream_t 
         }
     } else {
         auto kern = pl.bs.g.b == 1 ? btree_stream_kernel<K, true> : btree_stream_kernel<K, false>;
-        TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const size_t stage = (size_t)pl.tile_keys * sizeof(K) + 128, ring_bytes = kBtreeStages * stage + 128;
+        TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes));
         int per_sm = 0;
-        TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStreamThreads, smem));
+        TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBtreeThreads, ring_bytes));
         uint64_t grid = std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * smx, std::max<uint64_t>(pl.ntiles, 1));
-        if (pl.ntiles) kern<<<(unsigned)grid, kStreamThreads, smem, st>>>(A, scr, pl.bs, ctrl, wc, flags), ++nl;
+        const uint32_t ring = (uint32_t)std::min<uint64_t>(kBtreeStages, (pl.ntiles + grid - 1) / grid);
+        if (pl.ntiles)
+            kern<<<(unsigned)grid, kBtreeThreads, ring_bytes, st>>>(A, scr, pl.bs, ctrl, wc, flags, ring,
+                                                                    (uint32_t)(stage / sizeof(K)),
+                                                                    pl.ntiles >= kClaimAheadItems * grid * ring), ++nl;
         TL_CUDA_TRY(cudaGetLastError());
         timer.mid();
         if (pl.ordered && pl.ot.nsegs) {
@@ -488,7 +610,7 @@ int btree_plan_of(uint64_t n, uint64_t b) {
 }
 
 template <typename Kern>
-static int blocks_per_sm_of(Kern kern, size_t smem, int threads = kStreamThreads) {
+static int blocks_per_sm_of(Kern kern, size_t smem, int threads) {
     int per_sm = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
@@ -499,16 +621,16 @@ static int blocks_per_sm_of(Kern kern, size_t smem, int threads = kStreamThreads
 // Resident blocks per SM of the stream kernel instance launch_permute_k picks
 // for the layout (the BST has its own instance), at the 32 KB tile.
 int stream_blocks_per_sm(int layout, uint32_t key_bytes) {
-    const size_t smem = 32768 + kTileSmemSlack;
+    const size_t btree_ring = kBtreeStages * (size_t)(32768 + 128) + 128;
     const bool w8 = key_bytes == 8;
     if (is_veb_layout(layout))
         return w8 ? blocks_per_sm_of(mveb_stream_kernel<uint64_t>, kMvebStages * kMvebStageBytes, kMvebThreads)
                   : blocks_per_sm_of(mveb_stream_kernel<uint32_t>, kMvebStages * kMvebStageBytes, kMvebThreads);
     if (layout == TL_LAYOUT_BST)
-        return w8 ? blocks_per_sm_of(btree_stream_kernel<uint64_t, true>, smem)
-                  : blocks_per_sm_of(btree_stream_kernel<uint32_t, true>, smem);
-    return w8 ? blocks_per_sm_of(btree_stream_kernel<uint64_t, false>, smem)
-              : blocks_per_sm_of(btree_stream_kernel<uint32_t, false>, smem);
+        return w8 ? blocks_per_sm_of(btree_stream_kernel<uint64_t, true>, btree_ring, kBtreeThreads)
+                  : blocks_per_sm_of(btree_stream_kernel<uint32_t, true>, btree_ring, kBtreeThreads);
+    return w8 ? blocks_per_sm_of(btree_stream_kernel<uint64_t, false>, btree_ring, kBtreeThreads)
+              : blocks_per_sm_of(btree_stream_kernel<uint32_t, false>, btree_ring, kBtreeThreads);
 }
 
 int permute_plan_of(int layout, uint64_t n, uint64_t b, uint32_t key_bytes) {

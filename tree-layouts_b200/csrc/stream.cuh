@@ -3,13 +3,13 @@
 //
 // The in-place pass walks the array one tile at a time.  Tiles are handed out by
 // an atomic ticket counter, so a CTA holding ticket t knows every ticket below t
-// is already owned by a running CTA.  A CTA first copies its whole source tile
-// into shared memory and then publishes "tile read".  Before storing, it waits
-// (acquire) for the flags of the tiles whose source overlaps the destinations
-// it will write.  Those tiles always hold smaller tickets, and a CTA publishes
-// its flag before it waits on anything, so every wait ends.  Waits
-// are still bounded: on expiry the CTA records TL_ERROR_TIMEOUT in the control
-// block, skips its stores, and the host reports the error.
+// is already owned by a running CTA.  A tile is first copied whole into shared
+// memory and then published as read.  Before its stores, the flags of the tiles
+// whose source overlaps their destinations are waited for (acquire).  Those tiles
+// always hold smaller tickets, and a CTA stores its tiles in ticket order, so
+// every wait ends.  Waits are still bounded: on expiry the CTA records
+// TL_ERROR_TIMEOUT in the control block, skips the tile's stores, and the host
+// reports the error.
 #pragma once
 
 #include "tl_common.cuh"
@@ -64,16 +64,6 @@ __device__ __forceinline__ bool wait_flag(const unsigned int *flag, unsigned int
     return false;
 }
 
-// Block-wide: publish that this tile's source has been read into shared memory.
-// Every load of the tile has returned its data (cp.async.wait_all, or register
-// loads already stored to shared memory) before the barrier, so no write that
-// follows the flag can reach them: a relaxed store suffices, and thread 0 does
-// not wait for its own earlier global stores to drain as a fence would make it.
-__device__ __forceinline__ void publish_read(unsigned int *flag, const WaitCfg &wc) {
-    __syncthreads();
-    if (threadIdx.x == 0) st_relaxed(flag, wc.flag_value);
-}
-
 // Block-wide ticket loop with the next ticket claimed one tile ahead: thread 0
 // issues the atomic for ticket t+1 before tile t is processed and publishes it
 // after.  A block holds at most its current and its next ticket; the current
@@ -100,11 +90,6 @@ __device__ __forceinline__ unsigned long long ticket_advance(const TicketPipe &t
     return *s_ticket;
 }
 
-// Bytes of dynamic shared memory a tile kernel asks for beyond its tile: room
-// to start the buffer on a 128-byte line, and the tile's head of up to 128
-// bytes (see load_tile_issue).
-constexpr size_t kTileSmemSlack = 128 + 128;
-
 // The tile buffer of a tile kernel: its dynamic shared memory rounded up to a
 // 128-byte line (whatever the static shared memory before it).
 template <typename K>
@@ -112,7 +97,7 @@ __device__ __forceinline__ K *tile_smem(unsigned char *dyn) {
     return reinterpret_cast<K *>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
 }
 
-// The base of load_tile for a tile starting at p0: p0 rounded down to a
+// The base of a loaded tile, for one starting at p0: p0 rounded down to a
 // Line-byte boundary of the global address (Line = 128 for a buffer from
 // tile_smem, 16 for one that keeps its own placement).
 template <uint32_t Line = 128, typename K>
@@ -126,9 +111,7 @@ __device__ __forceinline__ uint64_t tile_base(const K *src, uint64_t p0) {
 // line, so a warp's 16-byte cp.async chunks (global -> shared without
 // registers, every thread with all of its copies in flight) fill whole sectors
 // on both sides; shifted against the line, each chunk fetches its own 32-byte
-// sector, twice the L2 traffic.  (The vEB stream kernel measured faster with
-// its buffer where the static shared memory leaves it and Line = 16.)  The
-// ragged ends use plain loads.  In two halves: issue returns base with the
+// sector, twice the L2 traffic.  The ragged ends use plain loads.  In two halves: issue returns base with the
 // interior's copies still in flight, load_tile_wait waits for them.  Threads
 // tid of nt (default: the whole block) share the copies.
 template <uint32_t Line = 128, typename K>
@@ -154,12 +137,5 @@ __device__ __forceinline__ uint64_t load_tile_issue(const K *__restrict__ src, u
 }
 
 __device__ __forceinline__ void load_tile_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-template <uint32_t Line = 128, typename K>
-__device__ __forceinline__ uint64_t load_tile(const K *__restrict__ src, uint64_t p0, uint64_t p1, K *sm) {
-    const uint64_t base = load_tile_issue<Line>(src, p0, p1, sm);
-    load_tile_wait();
-    return base;
-}
 
 }  // namespace tl

@@ -298,6 +298,11 @@ __device__ __forceinline__ unsigned long long next_tile(unsigned long long t, co
     return ticket_advance(tp, s_ticket);
 }
 
+// Named barrier among the threads of warps 1.. of the block.
+__device__ __forceinline__ void bar_sync_tail() {
+    asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x - 32) : "memory");
+}
+
 // Sorted tile z of a B-tree or BST.  In most tiles (kinds 1 and 3) the bulk
 // keys are one stretch of the layout (or of scratch, split at a tile boundary):
 // cp.async copies it as it lies, at its own offset within a 128-byte line,
