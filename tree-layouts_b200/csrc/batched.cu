@@ -59,12 +59,15 @@ struct alignas(16) BatchInst {
 constexpr uint64_t kBatchOrderMinTiles = 64;
 constexpr uint64_t kChunkItemsMax = 64;
 constexpr uint64_t kRangePiece = 2048;
-// An instance takes the ordered schedule if that moves at most this share of the
-// scratch keys of its fixed-direction schedule.  Measured on B200, 1024 arrays of
-// 2^10..2^22 keys at 0.3, 0.6 and 0.9: b = 8 1.75, 1.65, 1.64 ms; b = 1 2.35,
-// 2.27, 2.12; b = 4 2.03, 1.92, 1.88; b = 16 1.59, 1.57, 1.57.  Their longer item
-// lists make the plan, built once, 23 ms instead of 20.
-constexpr double kOrderGain = 0.9;
+// An instance takes the ordered schedule if that moves at most kOrderGain of the
+// scratch keys of its fixed-direction schedule, and, above kOrderGainSpace, only
+// in no more scratch space (the ordered schedule gives each tile that receives
+// scratch keys a tile of scratch: without this, 300 arrays of 2^18..2^20 keys at
+// b = 16 need 277 MB instead of 191).  Measured on B200, 1024 arrays of
+// 2^10..2^22 keys, 0.3 everywhere against this: b = 8 1.75 -> 1.64 ms, b = 1 2.35
+// -> 2.12, b = 4 2.03 -> 1.96 (1.88 whatever the space), b = 16 1.59 -> 1.57.
+// Their longer item lists make the plan, built once, 23 ms instead of 20.
+constexpr double kOrderGain = 0.9, kOrderGainSpace = 0.3;
 constexpr uint64_t kInterleaveRun = 1;  // stream tiles an instance takes in a row
 static_assert(sizeof(BatchInst) % 16 == 0, "BatchInst is copied to shared memory in 16-byte words");
 
@@ -246,7 +249,7 @@ constexpr uint32_t kPlanWords = sizeof(BatchInst) / 16;
 // stores overlap: with a block holding one item at a time, load, publish, wait
 // and store in turn, 1024 arrays of 2^10..2^22 keys took 1885 us at b = 8 and
 // 1808 at b = 16; in the ring 1752 and 1589, and with the ordered schedule, whose
-// instructions now hide, in more instances (kOrderGain) 1640 and 1573.  Claiming
+// instructions now hide, in more instances (kOrderGain) 1637 and 1572.  Claiming
 // ahead is 2 % of it; two stages in three blocks took as long.
 struct BatchStage {
     BatchInst I;
@@ -692,8 +695,9 @@ static int order_instances(tl_batch_plan_impl &P, const std::vector<int64_t> &of
                 const BtreeStream &S = h[cand[i]].S;
                 if (S.g.h < 1 || S.ntiles < kBatchOrderMinTiles || S.ntiles >= (1ull << 32)) continue;
                 btree_compute_order(S, ov[i]);
-                if (!ordered_schedule_forced() &&
-                    order_scratch_keys(S, ov[i]) > kOrderGain * (double)fixed_scratch_keys(S))
+                const double moved = (double)order_scratch_keys(S, ov[i]), fixed = (double)fixed_scratch_keys(S);
+                const bool wider = ov[i].scratch_tiles * S.tile_keys > S.nscratch;
+                if (!ordered_schedule_forced() && moved > (wider ? kOrderGainSpace : kOrderGain) * fixed)
                     ov[i] = OrderVectors();
             }
         };
