@@ -100,19 +100,21 @@ def query_bytes_model(layout, n, b, kb):
 
 
 def query_grouped(layout, n, kb, q):
-    """Whether the library searches a batch grouped by value first: BST and vEB
-    batches of 2^21 queries or more over a BST layout of 64 MB or more or a vEB
-    layout of 4 MB or more (the thresholds of csrc/query.cu's launch_query)."""
-    return (layout in ("bst", "mveb", "veb") and (1 << 21) <= q < (1 << 32)
-            and n * kb >= (64 << 20 if layout == "bst" else 4 << 20))
+    """Whether the library groups a batch by value in device memory first: BST
+    batches of more than 2^22 queries over 1 GB (2^28 - 1 u32 keys) or more (csrc/query.cu's
+    launch_query)."""
+    return layout == "bst" and (1 << 22) < q < (1 << 32) and n * kb >= (1 << 30) - 1024
 
 
-def query_kernel_name(layout, b, kb):
+def query_kernel_name(layout, b, kb, n, q):
     """The kernel the library launches for a query batch over a 32-byte aligned
     layout (torch allocations are)."""
     if layout == "btree":
         nb = b * kb
         if nb in (64, 128, 256):
+            if q >= 1 << 20 and n < 1 << 31:
+                return (f"btree_query_top_kernel (top levels in shared memory, then {max(2, nb // 64)} lanes per node, "
+                        "32-byte loads)")
             return f"btree_query_group32_kernel ({max(2, nb // 64)} lanes per node, 32-byte loads)"
         if nb % 32 == 0 and nb <= 256:
             return "btree_query_v32_kernel (a thread per query, 32-byte loads)"
@@ -120,7 +122,7 @@ def query_kernel_name(layout, b, kb):
             return "btree_query_vec_kernel (a thread per query, 16-byte loads)"
         return "btree_query_kernel (a lane per key)"
     if layout == "bst":
-        return "bst_query_kernel"
+        return "bst_query_kernel" if query_grouped(layout, n, kb, q) else "bst_query_sorted_kernel"
     return "veb_query_kernel"
 
 
@@ -375,7 +377,7 @@ def learned_section(args, dev):
            "n": n, "q": q, "plain_queries_per_s": round(q / (pm * 1e-3), 1),
            "learned_queries_per_s": round(q / (lm * 1e-3), 1), "speedup": round(pm / lm, 3),
            "exact": exact, "plain_ms": round(pm, 3), "learned_ms": round(lm, 3),
-           "kernels": {"plain": query_kernel_name("btree", b, 8),
+           "kernels": {"plain": query_kernel_name("btree", b, 8, n, q),
                        "learned": "learned_query_group_kernel (2 lanes per node, a per-warp queue of "
                                   "prepared starts)"},
            "fallback_frac": round(int(stats[0].item()) / q, 4),
@@ -576,8 +578,8 @@ def layouts_section(args, L, dev, stream, local, peak, peak_kind):
                      "pass2_ms": st["pass2_ms"], "schedule": st["schedule"], "kernel": st["kernel"],
                      "stalled_waits": st["stalled_waits"], "steps": args.steps, "clocks": clk, "parity": rep}
         if keep:
-            # the plain queries of the layout (device time; BST and vEB batches
-            # this large are searched grouped by value, the grouping included)
+            # the plain queries of the layout (device time; a grouping of the batch
+            # by value, where the library makes one, included)
             Q = data.queries_torch(pristine, q, 0.5, qseed)
             ans = torch.empty(q, dtype=torch.int64, device=dev)
             tabs = T.VebTablesDevice(n, dev, standard=layout == "veb") if layout in ("mveb", "veb") else None
@@ -591,7 +593,7 @@ def layouts_section(args, L, dev, stream, local, peak, peak_kind):
             out[name]["queries"] = {
                 "q": q, "ms": round(qms, 3), "queries_per_s": round(qps, 1),
                 "frac_of_byte_model": round(qps * qbytes / (peak * 1e9), 4), "bytes_per_query": qbytes,
-                "kernel": query_kernel_name(layout, b or 16, kb) + (", batch grouped by value" if grouped else ""),
+                "kernel": query_kernel_name(layout, b or 16, kb, n, q) + (", batch grouped by value" if grouped else ""),
                 "hits": int((ans != n).sum().item()),
                 "parity": P.check_answers(layout, b or 16, host, Q, ans, 1 << 20, qseed)}
             del Q, ans, tabs
@@ -682,11 +684,12 @@ def run_ours(args, rank, world, local):
                 rms.append(r)
         assert torch.equal(A, pristine), "reverse permutation check failed"
         r_med = statistics.median(rms)
-        rinfo = {"kernel": "device copy + " + ("veb_gather_kernel" if layout in ("mveb", "veb") else "btree_gather_kernel"),
+        rinfo = {"kernel": "mveb_unstream_kernel" if layout in ("mveb", "veb") else "btree_unstream_kernel",
                  "ms": round(r_med, 4), "GBps": round(bytes_step / (r_med * 1e-3) / 1e9, 1),
                  "frac_of_peak": round(bytes_step / (r_med * 1e-3) / 1e9 / peak, 4),
                  "equal_to_sorted": True,
-                 "note": "2*n*w / device time; the pass moves 4*n*w (a copy to the workspace, then the gather)"}
+                 "note": "2*n*w / device time; large arrays go back in place, small ones (vEB <= 32 MB, "
+                         "B-tree <= 192 MB, BST under a fixed schedule) through a copy, 4*n*w"}
         del layout_copy, ws
         A.copy_(pristine)
         T.permute(layout, A, b or 16)  # the layout again, for the queries below
@@ -747,7 +750,7 @@ def run_ours(args, rank, world, local):
                               "roofline_queries_per_s": round(peak * 1e9 / qbytes, 1),
                               "frac": round(qps * qbytes / (peak * 1e9), 4),
                               "model": "w + 8 + one node fetch per level below the L2-resident depth"},
-                 "hits": hits, "kernel": query_kernel_name(layout, b or 16, kb)
+                 "hits": hits, "kernel": query_kernel_name(layout, b or 16, kb, n, q)
                  + (", batch grouped by value" if query_grouped(layout, n, kb, q) else ""),
                  "binary_search_queries_per_s": round(q / (sms * 1e-3), 1),
                  "binary_search_hits": int((sans != n).sum().item())}

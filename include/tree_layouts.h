@@ -159,8 +159,10 @@ int tl_permute_algorithm(int layout, int algorithm, void *dev_A, uint64_t n, uin
  * same layout, b and key width) back to sorted order, in place.  No counterpart
  * in the reference, whose README describes conversions between sorted order and
  * the layouts but implements only sorted -> layout.  Workspace, stream and ms
- * as for tl_permute (dev_workspace NULL: a cached buffer of
- * tl_unpermute_workspace_bytes, which holds a copy of the array). */
+ * as for tl_permute.  tl_unpermute_workspace_bytes has room for a copy of the
+ * array; with dev_workspace NULL the cached buffer is only as large as the
+ * layout and size need (large arrays go back in place, through scratch for the
+ * keys that took scratch on the way there). */
 int tl_unpermute_workspace_bytes(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, uint64_t *bytes);
 int tl_unpermute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes, void *dev_workspace,
                  uint64_t workspace_bytes, void *stream, float *ms);
@@ -264,8 +266,8 @@ int tl_batch_query(const tl_batch_plan *plan, const void *dev_keys, const void *
                    const uint32_t *dev_inst, uint64_t q, uint64_t *dev_answers, void *dev_workspace,
                    uint64_t workspace_bytes, void *stream, float *ms);
 /* Tuning per size class c = floor(log2 n_j), 48 entries each: keys per stream
- * tile (a power of two, 256 .. 96 KB / key_bytes); plus the permute block size
- * (256 or 512); 0 / NULL keeps a value.  pin_levels and query_chunk are kept and
+ * tile (a power of two, 256 .. 96 KB / key_bytes); plus the permute block shape
+ * (256: eight store warps, 512: four); 0 / NULL keeps a value.  pin_levels and query_chunk are kept and
  * read back, but the queries have nothing to tune.  Changing tile sizes rebuilds
  * the plan from dev_offsets. */
 int tl_batch_set_tuning(tl_batch_plan *plan, const uint32_t *tile_keys, const uint32_t *pin_levels,
@@ -390,14 +392,14 @@ int tl_debug_stream_blocks_per_sm(int layout, uint32_t key_bytes);
  * schedule applies to on it, whatever it saves; 0 restores the default. */
 int tl_debug_set_schedule(int mode);
 /* Measurement hook, query kernels: 0 the default; 2 B-tree nodes in 16-byte
- * loads by a thread per query; 3 / 4 vEB two / four descents per thread in
- * lock-step; 5 B-tree a thread per query with 32-byte loads and the top levels
- * pinned in shared memory; 6 B-tree a thread per query with 32-byte loads (in
- * place of a group of lanes per node, for the learned query too); 7 B-tree one
- * 32-byte load per lane of the group (b * w / 32 lanes); 19 BST and vEB
- * batches searched as given, 20 always grouped by value (by default only
- * batches of 2^21 queries or more over BST layouts of 64 MB or more and vEB
- * layouts of 4 MB or more). */
+ * loads by a thread per query; 5 B-tree a thread per query with 32-byte loads and
+ * the top levels pinned in shared memory; 6 B-tree a thread per query with 32-byte
+ * loads (in place of a group of lanes per node, for the learned query too); 7
+ * B-tree one 32-byte load per lane of the group (b * w / 32 lanes); 8 the learned
+ * query with 64-bit indices; 9 B-tree top levels in shared memory at any batch
+ * size; 19 BST batches never grouped by value in device memory, 20 always (by
+ * default only more than 2^22 queries over 1 GB or more); 30 / 31 batched queries
+ * always / never ordered by instance. */
 void tl_debug_set_query_variant(int v);
 /* Instances of a batched plan on the ordered-tile schedule and their keys: by
  * default those of 64 tiles or more (at the plan's tile size for their size

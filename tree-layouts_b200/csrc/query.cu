@@ -1,10 +1,11 @@
 // Batched exact point queries over the three layouts (sm_100a).
 //
-// Each kernel is persistent (grid = SMs x resident CTAs) and walks the query
-// array with a grid stride.  The first P positions of the layout - the top
-// levels for every layout, since each one stores its root region first - are
-// copied once per CTA into shared memory, so the first levels of every descent
-// cost a shared-memory load instead of an L2/HBM round trip.
+// Each kernel is persistent (grid = SMs x resident CTAs) and copies the top
+// levels, the layout's first positions, once per CTA into shared memory, so the
+// first levels of every descent cost a shared-memory load instead of an L2/HBM
+// round trip.  The B-tree kernels walk the query array with a grid stride; the
+// BST, vEB and sorted-array kernels take it in chunks that a block orders by
+// value in shared memory first, so that neighbours share their lower nodes.
 //
 // Answers are the layout position of the key or n (gpu/src/query-bst.cuh:41,
 // gpu/src/query-btree.cuh:59, gpu/src/query-mveb.cuh:65).  For keys present in
@@ -403,6 +404,13 @@ btree_query_group32_kernel(const K *__restrict__ A, uint64_t n, const K *__restr
 constexpr uint32_t kTopBins = 4096;
 constexpr int kTopThreads = 1024;
 constexpr uint64_t kTopBytes = 40 * 1024;
+// 128-byte nodes keep the kernel above over larger layouts, whose deep levels are
+// no longer bound by wavefronts (the cause beyond that was not isolated): b = 16
+// u64, kernel above against this, 2^27 queries over 2^29 keys 9.48 / 8.51 ms, over
+// 8e8 9.68 / 9.83, over 2^30 9.92 / 10.62; 2^26 over 6.4e8 4.78 / 4.53.  Other
+// nodes gain at every size (64-byte over 7.6 GB 4.26 / 3.94, 256-byte over 7.2 GB
+// 7.39 / 5.57).
+constexpr uint64_t kTopMaxBytes128 = 5ull << 30;
 
 template <typename K, int NB, int G>
 __global__ void __launch_bounds__(kTopThreads, 2)
@@ -1000,7 +1008,7 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
 }
 
 // ---------------------------------------------------------------- partition
-// Queries close in value walk close paths through a BST or vEB layout, whose
+// Queries close in value walk close paths through a BST, whose
 // lower levels hold each subtree's keys together.  Grouping a batch by value
 // lets a node fetched once from HBM serve the rest of its group from L2 or L1.
 // The batch is split into 2^bits buckets of its value range [min q, max q]
@@ -1552,7 +1560,8 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
             return TL_SUCCESS;
         };
         if ((base & 31) == 0 && m && a.n < (1ull << 31) &&
-            (g_query_variant == 9 || (g_query_variant == 0 && a.q >= (1ull << 20)))) {
+            (g_query_variant == 9 ||
+             (g_query_variant == 0 && a.q >= (1ull << 20) && (node_bytes != 128 || a.n * sizeof(K) <= kTopMaxBytes128)))) {
             switch (node_bytes) {
                 case 64: rc = topped(btree_query_top_kernel<K, 64, 2>, 2); break;
                 case 128: rc = topped(btree_query_top_kernel<K, 128, 2>, 2); break;
