@@ -112,7 +112,7 @@ def query_kernel_name(layout, b, kb, n, q):
     if layout == "btree":
         nb = b * kb
         if nb in (64, 128, 256):
-            if q >= 1 << 20 and n < 1 << 31:
+            if q >= 1 << 20 and n < 1 << 31 and (nb != 128 or n * kb <= 5 << 30):
                 return (f"btree_query_top_kernel (top levels in shared memory, then {max(2, nb // 64)} lanes per node, "
                         "32-byte loads)")
             return f"btree_query_group32_kernel ({max(2, nb // 64)} lanes per node, 32-byte loads)"
