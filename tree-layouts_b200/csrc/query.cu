@@ -409,7 +409,8 @@ constexpr uint64_t kTopBytes = 40 * 1024;
 // u64, kernel above against this, 2^27 queries over 2^29 keys 9.48 / 8.51 ms, over
 // 8e8 9.68 / 9.83, over 2^30 9.92 / 10.62; 2^26 over 6.4e8 4.78 / 4.53.  Other
 // nodes gain at every size (64-byte over 7.6 GB 4.26 / 3.94, 256-byte over 7.2 GB
-// 7.39 / 5.57).
+// 7.39 / 5.57).  Skewed batches would gain there too (2^28 Zipf queries over 2^30
+// keys 20.0 / 14.8 ms), but a batch's skew is not known at the launch.
 constexpr uint64_t kTopMaxBytes128 = 5ull << 30;
 
 template <typename K, int NB, int G>
