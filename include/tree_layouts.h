@@ -371,6 +371,12 @@ int tl_debug_emulate_algorithm(int layout, int algorithm, uint64_t n, uint64_t b
                                uint64_t *steps);
 /* Host replay of tl_unpermute's gather on n 64-bit words (test hook). */
 int tl_debug_emulate_unpermute(int layout, uint64_t n, uint64_t b, uint64_t *host_A);
+/* Host replay of how the B-tree query builds and searches the top levels it
+ * holds in shared memory (test hook), on n words that need not be in layout
+ * order: ranks[i] = the top keys below queries[i]; *violations = accesses out of
+ * range.  TL_ERROR_UNSUPPORTED where that form does not apply. */
+int tl_debug_emulate_btree_top(const void *host_A, uint64_t n, uint64_t b, uint32_t key_bytes,
+                               const void *host_queries, uint64_t q, uint64_t *ranks, uint64_t *violations);
 /* sizeof of the ABI structs, for bindings to check their mirrors:
  * 0 tl_veb_table, 1 tl_rank_model, 2 tl_rank_leaf, 3 tl_rank_train_config. */
 int tl_debug_struct_size(int which);

@@ -139,3 +139,39 @@ def test_algorithm_variants_not_built_are_refused_before_device_work():
     assert lib.tl_permute_algorithm(T.LAYOUT_BTREE, 1, C.c_void_p(256), 1000, 0, 8, None, None) == T.ERROR_INVALID_VALUE
     assert lib.tl_permute_algorithm(T.LAYOUT_BTREE, 1, C.c_void_p(256), 1000, 1 << 31, 8, None,
                                     None) == T.ERROR_INVALID_VALUE
+
+
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+@pytest.mark.parametrize("node_bytes", [64, 128, 256])
+def test_btree_top_search_stays_in_range_for_any_words(dtype, node_bytes):
+    """The search of the B-tree's top levels, replayed on the host: ranks among a
+    layout's top keys are exact, and words in no order at all (sorted keys never
+    permuted, shuffled, random, a layout permuted twice) reach nothing out of
+    range."""
+    L = T.lib()
+    L.tl_debug_emulate_btree_top.argtypes = [C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint32, C.c_void_p, C.c_uint64,
+                                             C.c_void_p, C.c_void_p]
+    b = node_bytes // np.dtype(dtype).itemsize
+    top = np.iinfo(dtype).max
+
+    def replay(words, Q):
+        ranks, viol = np.empty(len(Q), np.uint64), np.zeros(1, np.uint64)
+        assert L.tl_debug_emulate_btree_top(words.ctypes.data, len(words), b, words.itemsize, Q.ctypes.data, len(Q),
+                                            ranks.ctypes.data, viol.ctypes.data) == 0
+        return ranks, int(viol[0])
+
+    rng = np.random.default_rng(node_bytes)
+    for n in [b, b + 1, (b + 1) ** 2 - 1, (b + 1) ** 2, 60_001]:
+        keys = np.cumsum(rng.integers(1, 50_000, n), dtype=np.uint64).astype(dtype)
+        lay = O.permute("btree", keys, b)
+        Q = np.concatenate([keys[:2000], keys[-50:] + 1, rng.integers(0, top, 2000, dtype=dtype, endpoint=True),
+                            np.array([0, top], dtype)]).astype(dtype)
+        m = b
+        while m * (b + 1) + b <= n and (m * (b + 1) + b) * keys.itemsize <= 40 * 1024:
+            m = m * (b + 1) + b
+        ranks, viol = replay(lay, Q)
+        assert viol == 0
+        assert np.array_equal(ranks, np.searchsorted(np.sort(lay[:m]), Q).astype(np.uint64))
+        for words in (keys, keys[::-1].copy(), rng.permutation(keys), rng.integers(0, top, n, dtype=dtype),
+                      O.permute("btree", lay, b), np.full(n, top, dtype)):
+            assert replay(words, Q)[1] == 0

@@ -194,6 +194,11 @@ int tl_debug_order_tables_match(int layout, uint64_t n, uint64_t b, uint32_t key
     return debug_order_tables_match(layout, n, b, key_bytes, S(stream));
 }
 
+int tl_debug_emulate_btree_top(const void *host_A, uint64_t n, uint64_t b, uint32_t key_bytes,
+                               const void *host_queries, uint64_t q, uint64_t *ranks, uint64_t *violations) {
+    return emulate_btree_top(host_A, n, b, key_bytes, host_queries, q, ranks, violations);
+}
+
 // Measurement hook: query kernel variants (0: the default).
 void tl_debug_set_query_variant(int v) { set_query_variant(v); }
 

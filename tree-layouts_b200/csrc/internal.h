@@ -117,6 +117,8 @@ int emulate_permute(int layout, uint64_t n, uint64_t b, uint64_t *A, uint64_t *v
 // query.cu: kernel selection for measurements (0: the default)
 void set_query_variant(int v);
 int query_variant();
+int emulate_btree_top(const void *A, uint64_t n, uint64_t b, uint32_t key_bytes, const void *Q, uint64_t q,
+                      uint64_t *ranks, uint64_t *violations);
 // cycles.cu: the cycle-leader family (and the hybrid BST's last level); for
 // the hybrid *perfect = keys of the front part the involutions finish
 int permute_cycles(int layout, int algorithm, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes,

@@ -11,6 +11,7 @@
 // gpu/src/query-btree.cuh:59, gpu/src/query-mveb.cuh:65).  For keys present in
 // the layout the descent visits the same nodes as the reference's searches.
 #include <algorithm>
+#include <vector>
 
 #include "internal.h"
 #include "tl_common.cuh"
@@ -413,6 +414,79 @@ constexpr uint64_t kTopBytes = 40 * 1024;
 // keys 20.0 / 14.8 ms), but a batch's skew is not known at the launch.
 constexpr uint64_t kTopMaxBytes128 = 5ull << 30;
 
+// Keys of the whole levels that kTopBytes hold (0: not one).
+template <typename K>
+constexpr uint64_t btree_top_keys(uint64_t n, uint64_t b) {
+    uint64_t m = 0;
+    for (uint64_t t = b; t <= n && t <= kTopBytes / sizeof(K); t = t * (b + 1) + b) m = t;
+    return m;
+}
+
+// The top's index arithmetic, shared with its host replay (emulate_btree_top).
+// Keys that are not in layout order give no meaningful answer, but every index
+// stays in range for them too: bin numbers are clamped and no bin is left unset.
+
+// Sorted rank of the top's position p: the x-th multiple of mult (x not a
+// multiple of B + 1) on its level.
+template <uint32_t B>
+TL_HD uint32_t top_rank_of(uint32_t p, uint32_t m) {
+    uint32_t end = B + 1, mult = (m + 1) / (B + 1);  // the level's end + 1, its keys' spacing
+    while (p + 1 >= end) {
+        end *= B + 1;
+        mult /= B + 1;
+    }
+    const uint32_t t = p + 1 - end / (B + 1);
+    return (t + 1 + t / B) * mult - 1;
+}
+
+// The position of sorted rank r.
+template <uint32_t B>
+TL_HD uint32_t top_position(uint32_t r, uint32_t m) {
+    uint32_t x = r + 1, end = m + 1;
+    while (x % (B + 1) == 0) {
+        x /= B + 1;
+        end /= B + 1;
+    }
+    return end / (B + 1) - 1 + (x - x / (B + 1) - 1);
+}
+
+template <typename K>
+TL_HD uint32_t top_shift(K first, K last) {
+    const uint32_t span = bit_length((uint64_t)(K)(last - first)), bits = bit_length(kTopBins - 1);
+    return span > bits ? span - bits : 0;
+}
+
+// The bin of a key, kTopBins for all past the last.
+template <typename K>
+TL_HD uint32_t top_bin(K key, K first, uint32_t shift) {
+    const K k = (K)(key - first) >> shift;
+    return k < (K)kTopBins ? (uint32_t)k : kTopBins;
+}
+
+// Rank r in the bins it is the first rank of: those past the bin of rank r - 1, up to its own.
+template <typename Top, typename K, typename Bin>
+TL_HD void top_fill(Top top, uint32_t m, K first, uint32_t shift, uint32_t r, Bin bin) {
+    const uint32_t hi = r < m ? top_bin((K)top[r], first, shift) : kTopBins;
+    for (uint32_t k = r ? top_bin((K)top[r - 1], first, shift) + 1 : 0; k <= hi; ++k) bin[k] = (uint16_t)r;
+}
+
+// The number of top keys below q.
+template <typename Top, typename K, typename Bin>
+TL_HD uint32_t top_rank(Top top, Bin bin, uint32_t m, K first, uint32_t shift, K q) {
+    if (q < first) return 0;
+    const uint32_t k = top_bin(q, first, shift);
+    if (k == kTopBins) return m;
+    uint32_t r = bin[k], r1 = bin[k + 1];
+    while (r < r1) {
+        const uint32_t mid = (r + r1) >> 1;
+        if ((K)top[mid] < q)
+            r = mid + 1;
+        else
+            r1 = mid;
+    }
+    return r;
+}
+
 template <typename K, int NB, int G>
 __global__ void __launch_bounds__(kTopThreads, 2)
 btree_query_top_kernel(const K *__restrict__ A, uint32_t n, uint32_t m, const K *__restrict__ Q, uint64_t nq,
@@ -427,24 +501,12 @@ btree_query_top_kernel(const K *__restrict__ A, uint32_t n, uint32_t m, const K 
     const uint32_t g = lane % G;
     const uint32_t gshift = lane - g;
     const uint32_t cmax = (uint32_t)(((uint64_t)n + 1) / (B + 1));
-    // position p of the top: the x-th multiple of mult (x not a multiple of b + 1) on its level
-    for (uint32_t p = threadIdx.x; p < m; p += kTopThreads) {
-        uint32_t end = B + 1, mult = (m + 1) / (B + 1);  // the level's end + 1, its keys' spacing
-        while (p + 1 >= end) {
-            end *= B + 1;
-            mult /= B + 1;
-        }
-        const uint32_t t = p + 1 - end / (B + 1);
-        top[(t + 1 + t / B) * mult - 1] = __ldg(A + p);
-    }
+    for (uint32_t p = threadIdx.x; p < m; p += kTopThreads) top[top_rank_of<B>(p, m)] = __ldg(A + p);
+    for (uint32_t k = threadIdx.x; k <= kTopBins; k += kTopThreads) bin[k] = 0;
     __syncthreads();
     const K first = top[0];
-    const uint32_t span = bit_length((uint64_t)(top[m - 1] - first)), bits = bit_length(kTopBins - 1);
-    const uint32_t shift = span > bits ? span - bits : 0;
-    for (uint32_t r = threadIdx.x; r <= m; r += kTopThreads) {
-        const uint32_t hi = r < m ? (uint32_t)((top[r] - first) >> shift) : kTopBins;
-        for (uint32_t k = r ? (uint32_t)((top[r - 1] - first) >> shift) + 1 : 0; k <= hi; ++k) bin[k] = (uint16_t)r;
-    }
+    const uint32_t shift = top_shift(first, top[m - 1]);
+    for (uint32_t r = threadIdx.x; r <= m; r += kTopThreads) top_fill(top, m, first, shift, r, bin);
     __syncthreads();
     const uint64_t warps = (uint64_t)gridDim.x * (kTopThreads / 32);
     const uint64_t wid = ((uint64_t)blockIdx.x * kTopThreads + threadIdx.x) / 32;
@@ -452,32 +514,11 @@ btree_query_top_kernel(const K *__restrict__ A, uint32_t n, uint32_t m, const K 
         const uint64_t qi = base + lane / G;
         const bool have = qi < nq;
         const K q = have ? __ldcs(Q + qi) : K(0);
-        uint32_t r = 0;  // top keys below q
-        if (q >= first) {
-            const K k = (K)(q - first) >> shift;
-            uint32_t r1 = m;
-            r = m;
-            if (k < kTopBins) {
-                r = bin[k];
-                r1 = bin[k + 1];
-            }
-            while (r < r1) {
-                const uint32_t mid = (r + r1) >> 1;
-                if (top[mid] < q)
-                    r = mid + 1;
-                else
-                    r1 = mid;
-            }
-        }
+        const uint32_t r = top_rank(top, bin, m, first, shift, q);  // top keys below q
         uint32_t i = m + r * B, res = n;
         bool live = have && i < n;
         if (r < m && top[r] == q) {  // a key of the top: its position there
-            uint32_t x = r + 1, end = m + 1;
-            while (x % (B + 1) == 0) {
-                x /= B + 1;
-                end /= B + 1;
-            }
-            res = end / (B + 1) - 1 + (x - x / (B + 1) - 1);
+            res = top_position<B>(r, m);
             live = false;
         }
         while (__any_sync(0xFFFFFFFFu, live)) {
@@ -1549,8 +1590,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         // keys 20 / 23, 32 / 31, 54 / 42) the whole top levels that 40 KB hold are
         // searched in shared memory (10 KB, two levels at b = 16: 838 against 702
         // us over 1e8 keys).  Variant 9 takes this form at any size.
-        uint64_t m = 0;
-        for (uint64_t t = a.b; t <= a.n && t * sizeof(K) <= kTopBytes; t = t * (a.b + 1) + a.b) m = t;
+        const uint64_t m = btree_top_keys<K>(a.n, a.b);
         auto topped = [&](auto kern, uint64_t lanes_per_query) -> int {
             const size_t bytes = m * sizeof(K) + (kTopBins + 1) * sizeof(uint16_t);
             TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -1689,6 +1729,72 @@ int query(const QueryArgs &a, cudaStream_t st, float *ms) {
         *ms = timer.elapsed();
     }
     return TL_SUCCESS;
+}
+
+// ---------------------------------------------------------------- replay
+namespace {
+// An array whose accesses are checked: one out of range counts and goes nowhere.
+template <typename V>
+struct Checked {
+    V *v;
+    uint32_t len;
+    uint64_t *violations;
+    mutable V nowhere{};
+    TL_HD V &operator[](uint32_t i) const {
+        if (i < len) return v[i];
+        ++*violations;
+        return nowhere;
+    }
+};
+
+template <typename K, uint32_t B>
+void replay_top(const K *A, uint32_t m, const K *Q, uint64_t q, uint64_t *ranks, uint64_t *violations) {
+    std::vector<K> top_keys(m);
+    std::vector<uint16_t> bins(kTopBins + 1, 0);
+    const Checked<K> top{top_keys.data(), m, violations};
+    const Checked<uint16_t> bin{bins.data(), kTopBins + 1, violations};
+    for (uint32_t p = 0; p < m; ++p) {
+        const uint32_t r = top_rank_of<B>(p, m);
+        top[r] = A[p];
+        if (top_position<B>(r, m) != p) ++*violations;
+    }
+    const K first = top_keys[0];
+    const uint32_t shift = top_shift(first, top_keys[m - 1]);
+    for (uint32_t r = 0; r <= m; ++r) top_fill(top, m, first, shift, r, bin);
+    for (uint64_t i = 0; i < q; ++i) {
+        ranks[i] = top_rank(top, bin, m, first, shift, Q[i]);
+        if (ranks[i] > m) ++*violations;
+    }
+}
+
+template <typename K>
+int emulate_top(const K *A, uint64_t n, uint64_t b, const K *Q, uint64_t q, uint64_t *ranks, uint64_t *violations) {
+    const uint64_t m = btree_top_keys<K>(n, b);
+    if (!m) return TL_ERROR_UNSUPPORTED;
+    switch (b * sizeof(K)) {
+        case 64: replay_top<K, 64 / sizeof(K)>(A, (uint32_t)m, Q, q, ranks, violations); break;
+        case 128: replay_top<K, 128 / sizeof(K)>(A, (uint32_t)m, Q, q, ranks, violations); break;
+        case 256: replay_top<K, 256 / sizeof(K)>(A, (uint32_t)m, Q, q, ranks, violations); break;
+        default: return TL_ERROR_UNSUPPORTED;
+    }
+    return TL_SUCCESS;
+}
+}  // namespace
+
+// Host replay of btree_query_top_kernel's set-up and of its search of the top
+// levels (test hook): the top keys below each query, and the accesses that left
+// their array.  The words of A need not be in layout order.
+int emulate_btree_top(const void *A, uint64_t n, uint64_t b, uint32_t key_bytes, const void *Q, uint64_t q,
+                      uint64_t *ranks, uint64_t *violations) {
+    if (!A || !Q || !ranks || !violations || b == 0) return TL_ERROR_INVALID_VALUE;
+    *violations = 0;
+    if (key_bytes == 8)
+        return emulate_top(static_cast<const uint64_t *>(A), n, b, static_cast<const uint64_t *>(Q), q, ranks,
+                           violations);
+    if (key_bytes == 4)
+        return emulate_top(static_cast<const uint32_t *>(A), n, b, static_cast<const uint32_t *>(Q), q, ranks,
+                           violations);
+    return TL_ERROR_INVALID_VALUE;
 }
 
 }  // namespace tl
