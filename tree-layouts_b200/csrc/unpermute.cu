@@ -239,42 +239,50 @@ static inline uint64_t btree_gather_keys(uint64_t tile_keys, uint64_t b, uint32_
 
 // The bulk keys of a boundary tile into the tile buffer, by warps 1..: four a
 // thread at a time; a load has returned once its key is in shared memory, and a
-// warp then takes off the layout keys it read, a subtraction a tile.  (Out of
-// line: its state would spill the common path's registers; 1.41 -> 1.67 ms on
-// the 5e8-key B-tree.)
+// warp then takes off the layout keys it read, a subtraction a tile.  The lanes
+// meet in between: the one that subtracts does so for keys that others loaded.
+// (Out of line: its state would spill the common path's registers; 1.41 -> 1.67 ms
+// on the 5e8-key B-tree.)
 template <typename K, bool kCopy>
 static __device__ __noinline__ void gather_boundary(const BtreeStream &S, const K *src, const K *scr, K *sm, uint64_t p0,
                                                     uint32_t cnt, Ctrl *ctrl, unsigned int *rem, int *ok) {
     const uint32_t tb = threadIdx.x - 32, nb = blockDim.x - 32, lane = tb & 31u;
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
     for (uint32_t b0 = tb & ~31u; b0 < cnt; b0 += 4 * nb) {
-        uint64_t idx[4];
         K v[4];
-        uint32_t how[4];  // 1 layout, 2 scratch
+        uint32_t from[4];  // the tile a layout key was read from
+        uint32_t have = 0;
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             const uint32_t o = b0 + x * nb + lane;
-            how[x] = 0;
+            from[x] = kNone;
             if (o >= cnt || btree_is_top(S, p0 + o)) continue;
             if (kCopy) {
-                how[x] = 1;
+                have |= 1u << x;
                 v[x] = src[btree_pos(S.g, S.fd, p0 + o)];
             } else {
-                how[x] = btree_place(S, p0 + o, idx[x]) ? 1 : 2;
-                if (how[x] == 2 && idx[x] >= S.nscratch) {
+                uint64_t idx;
+                const bool direct = btree_place(S, p0 + o, idx);
+                if (!direct && idx >= S.nscratch) {
                     btree_o_bad(ctrl);
                     *ok = 0;
-                    how[x] = 0;
+                    continue;
                 }
-                if (how[x]) v[x] = (how[x] == 1 ? src : scr)[idx[x]];
+                have |= 1u << x;
+                v[x] = (direct ? src : scr)[idx];
+                if (direct) from[x] = (uint32_t)(idx >> S.tile_shift);
             }
         }
 #pragma unroll
+        for (int x = 0; x < 4; ++x)
+            if ((have >> x) & 1u) sm[gskew(b0 + x * nb + lane)] = v[x];
+        if (kCopy) continue;
+        __syncwarp();  // every lane's keys are in shared memory before any is taken off a count
+#pragma unroll
         for (int x = 0; x < 4; ++x) {
-            if (how[x]) sm[gskew(b0 + x * nb + lane)] = v[x];
-            if (kCopy) continue;
-            const unsigned act = __ballot_sync(0xFFFFFFFFu, how[x] == 1);
-            if (how[x] == 1) {
-                const uint32_t u = (uint32_t)(idx[x] >> S.tile_shift);
+            const uint32_t u = from[x];
+            const unsigned act = __ballot_sync(0xFFFFFFFFu, u != kNone);
+            if (u != kNone) {
                 const unsigned same = __match_any_sync(act, u);
                 if ((int)lane == __ffs(same) - 1) atomicSub(&rem[u], (unsigned)__popc(same));
             }
