@@ -429,3 +429,26 @@ def test_sorted_array_ordered_chunks(kb, n, skip):
     ans = torch.empty(70_000, dtype=torch.int64, device="cuda")
     T.query("sorted", arr, Q, ans)
     _check_answers(arr, keys, Q, ans)
+
+
+def _with_duplicates(n, seed, dtype):
+    """n sorted keys, runs of one value geometrically long."""
+    rng = np.random.default_rng(seed)
+    return np.repeat(np.cumsum(rng.integers(1, 5, n)).astype(dtype), rng.geometric(0.3, n))[:n].copy()
+
+
+@pytest.mark.parametrize("layout,b", [("bst", 1), ("btree", 8), ("btree", 16), ("btree", 32), ("btree", 5), ("mveb", 0),
+                                      ("veb", 0)])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+def test_duplicate_keys_answer_the_first_on_the_path(layout, b, dtype):
+    """Equal keys: the answer is the one that the search from the root meets
+    first, as the oracle's, for small batches and for those whose top levels are
+    searched in shared memory; one value all over, and several divisions."""
+    for n in (2, 31, 100, 4095, 65_537, 1_000_003):
+        for keys in (_with_duplicates(n, n, dtype), np.full(n, 7, dtype)):
+            tree = O.permute(layout, keys, b or 16)
+            for q in (5000, (1 << 20) + 77):
+                Q = data.queries_np(keys, q, 0.7, 3)
+                Q[:3] = keys[0], keys[-1], keys[-1] + 1
+                assert np.array_equal(gpu_answers(layout, tree, Q, b or 16), O.search(layout, tree, Q, b or 16)), \
+                    (layout, b, n, q)

@@ -8,8 +8,8 @@
 // value in shared memory first, so that neighbours share their lower nodes.
 //
 // Answers are the layout position of the key or n (gpu/src/query-bst.cuh:41,
-// gpu/src/query-btree.cuh:59, gpu/src/query-mveb.cuh:65).  For keys present in
-// the layout the descent visits the same nodes as the reference's searches.
+// gpu/src/query-btree.cuh:59, gpu/src/query-mveb.cuh:65); of equal keys it is the
+// one that the reference's search from the root meets first.
 #include <algorithm>
 #include <vector>
 
@@ -450,6 +450,21 @@ TL_HD uint32_t top_position(uint32_t r, uint32_t m) {
     return end / (B + 1) - 1 + (x - x / (B + 1) - 1);
 }
 
+// Equal keys: of those at sorted rank r and after, the one that the search from
+// the root meets first.  Its path holds, a level up, the next multiple of that
+// level's spacing, and its keys do not fall on the way up.
+template <uint32_t B, typename Top>
+TL_HD uint32_t top_first_on_path(Top top, uint32_t m, uint32_t r) {
+    const auto q = top[r];
+    uint32_t x = r + 1;
+    for (uint32_t s = B + 1; s <= m; s *= B + 1) {
+        const uint32_t up = (x + s - 1) / s * s;
+        if (up > m || top[up - 1] != q) break;
+        x = up;
+    }
+    return x - 1;
+}
+
 template <typename K>
 TL_HD uint32_t top_shift(K first, K last) {
     const uint32_t span = bit_length((uint64_t)(K)(last - first)), bits = bit_length(kTopBins - 1);
@@ -518,7 +533,7 @@ btree_query_top_kernel(const K *__restrict__ A, uint32_t n, uint32_t m, const K 
         uint32_t i = m + r * B, res = n;
         bool live = have && i < n;
         if (r < m && top[r] == q) {  // a key of the top: its position there
-            res = top_position<B>(r, m);
+            res = top_position<B>(top_first_on_path<B>(top, m, r), m);
             live = false;
         }
         while (__any_sync(0xFFFFFFFFu, live)) {
@@ -665,8 +680,9 @@ __device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t le
 // Chunks of the batch in value order, the top P = 2^T - 1 keys (as they lie) in
 // shared memory.  With 1-based nodes x the children are 2x and 2x + 1; the top is
 // walked without tests for equality, and an equal key there is where the path
-// last went left.  Neighbours in the order share their nodes far down (a level of
-// 2^k nodes is 2^k consecutive keys), so a level's loads fall into a few lines.
+// last went left (of several, the first such turn).  Neighbours in the order
+// share their nodes far down (a level of 2^k nodes is 2^k consecutive keys), so a
+// level's loads fall into a few lines.
 // Measured on B200, before (as given below 2^21 queries or 64 MB, else grouped in
 // device memory) -> now: 2^24 queries over 2^27 - 1 u32 keys 1118 -> 1054 us, over
 // 2^26 - 1 1181 -> 844, over 2^24 - 1 1574 -> 660; 2^20 over 2^27 - 1 keys 265 -> 87, over
@@ -694,9 +710,11 @@ bst_query_sorted_kernel(const K *__restrict__ A, uint64_t n64, uint32_t P, uint3
             const K q = __ldg(Q + qi);
             uint32_t y = 1;
             for (uint32_t c = 0; c < levels; ++c) y = 2 * y + (sm[y] < q);
-            const uint32_t at = y >> __ffs(~y);
+            uint32_t at = y >> __ffs(~y);
             I x = y, res = n;
             if (at && sm[at] == q) {
+                // of equal keys the highest: the path's left turns above it, while they are equal too
+                for (uint32_t up = at >> __ffs(~at); up && sm[up] == q; up = at >> __ffs(~at)) at = up;
                 res = at - 1;
                 x = n + 1;
             }
@@ -777,13 +795,15 @@ sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uin
 // stretch, so here a descent goes down a piece of up to kVebPieceLevels levels
 // at a time: a thread reads the piece's 2^h - 1 keys together (aligned 32-byte
 // sectors), and the number of them below q is q's path through all h levels.
-// The order inside a piece is never looked at, only that it is contiguous: each
-// block works that out from the tables as given (veb_piece_levels), so tables
-// of any split rule do, and a depth where nothing longer is contiguous is a
-// piece of one level.  pos[] needs an entry per piece (8 for the 29 levels of a
-// 3e8-key mvEB), one column per thread in shared memory.  The levels above the
-// first pieces (division 0 only, as many as the budget holds) are gathered into
-// shared memory in BFS order, where a level costs one bank access.
+// With keys equal to q among them, the number of those tells which node of the
+// path the highest of them is.  The order inside a piece is looked at only for
+// that node's place (VebSchedule::slot): each block works out from the tables as
+// given what is contiguous (veb_piece_levels), so tables of any split rule do,
+// and a depth where nothing longer is contiguous is a piece of one level.  pos[]
+// needs an entry per piece (8 for the 29 levels of a 3e8-key mvEB), one column per
+// thread in shared memory.  The levels above the first pieces (division 0 only, as
+// many as the budget holds) are gathered into shared memory in BFS order, where a
+// level costs one bank access.
 //
 // What bounds it: a load of a thread's own line is an L1 wavefront, so a level
 // at a time costs 29 a query; a 15-key piece costs at most 3 for 4 levels and a
@@ -797,6 +817,10 @@ sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uin
 // wavefronts, twice the instructions); 512-thread blocks 5.8; chunks of 4096 /
 // 8192 / 32768 queries 4.76 / 4.46 / 4.62; 64 KB of pinned levels 4.6 (L1 is
 // smaller).  It holds for every batch: 2^10 queries 27 -> 14 us, 2^20 369 -> 95.
+// Equal keys are met in the pieces on the way, where following the counts to the
+// bottom and looking at the path's last left turn took 4.24 ms against 3.99 (u64
+// 1.70 against 1.75 for 2^24 queries) and gave the lowest of equal keys; looking
+// at the left turns above it too took 4.41.
 //
 // Tables whose pieces do not chain (not built by buildTable), a piece that
 // reaches past its division, and divisions beyond the first kVebSchedTables
@@ -814,6 +838,7 @@ struct VebStep {
 };
 struct VebSchedule {
     VebStep step[kVebMaxSteps];
+    unsigned char slot[kVebMaxSteps][1u << kVebPieceLevels];  // the place in its piece of a node, in BFS order from 1
     uint32_t steps;  // 0: level by level
     uint32_t top, ktop;  // levels held in shared memory, and the step that starts below them
 };
@@ -896,6 +921,14 @@ __device__ void veb_schedule(const tl_veb_table *__restrict__ gtab, uint32_t d, 
     }
 }
 
+// VebSchedule::slot of one piece's node (0: none), relative to the depth's leftmost piece.
+__device__ __forceinline__ void veb_slot(const tl_veb_table *tab, VebSchedule &sch, uint32_t k, uint32_t node) {
+    const uint32_t c = sch.step[k].c, e = node ? 31 - __clz(node) : 0;
+    if (k < sch.steps && node && e < sch.step[k].h)
+        sch.slot[k][node] = (unsigned char)(veb_node_pos(tab, c + e, ((1ull << c) << e) | (node & ((1u << e) - 1))) -
+                                            veb_node_pos(tab, c, 1ull << c));
+}
+
 // One descent level by level.  Returns 1 found (res), 2 absent, 0 left the
 // division [offset, limit) (the caller tries the next one).
 template <typename K>
@@ -923,9 +956,7 @@ __device__ __noinline__ int veb_descend_levels(const K *__restrict__ A, const tl
 
 // idx == nullptr: perfect layout, one table (timeQueryvEB); otherwise the
 // non-perfect table set (timeQueryvEB_nonperfect): the divisions in order, each
-// query until it is resolved.  A division's path is followed to its end on
-// counts alone; an equal key is then where the path last went left, one chain of
-// the recurrence and one load.  I: index type (32 bits when n < 2^31).
+// query until it is resolved.  I: index type (32 bits when n < 2^31).
 template <typename K, typename I>
 __global__ void __launch_bounds__(kSortThreads, 1)
 veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t max_top, uint32_t chunk,
@@ -952,6 +983,10 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                      idx ? __ldg(idx + j) : n64, sched[j], s_tabs[j], s_piece[j]);
     }
     __syncthreads();
+    constexpr uint32_t kSlots = kVebMaxSteps << kVebPieceLevels;  // a schedule's
+    static_assert(kVebSchedTables * kSlots <= kSortThreads, "a slot a thread");
+    if (const uint32_t j = threadIdx.x / kSlots; j < min(num_tables, kVebSchedTables))
+        veb_slot(s_tabs[j], sched[j], (threadIdx.x % kSlots) >> kVebPieceLevels, threadIdx.x & ((1u << kVebPieceLevels) - 1));
     const uint32_t top = sched[0].top;
     for (uint32_t x = threadIdx.x + 1; x < (1u << top); x += kSortThreads) {
         const uint64_t p = veb_node_pos(s_tab, 31 - __clz(x), x) - 1;
@@ -973,11 +1008,18 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                 const uint32_t steps = j < kVebSchedTables ? sched[j].steps : 0;
                 bool slow = steps == 0, left = false;
                 I i = 1;
-                uint32_t c = 0, k = 0;
+                uint32_t k = 0;
                 if (j == 0 && top) {
                     uint32_t x = 1;
-                    for (; c < top; ++c) x = 2 * x + (tree[x] < q);
+                    for (uint32_t c = 0; c < top; ++c) x = 2 * x + (tree[x] < q);
                     i = x;
+                    // an equal key is where the path last went left, or above that at a left turn equal too
+                    uint32_t hit = 0;
+                    for (uint32_t at = x >> __ffs(~x); at && tree[at] == q; at >>= __ffs(~at)) hit = at;
+                    if (hit) {
+                        res = (I)(veb_node_pos(s_tab, 31 - __clz(hit), hit) - 1);
+                        break;
+                    }
                     for (; k < sched[0].ktop; ++k) {
                         const VebStep &st = sched[0].step[k];
                         const I b = i >> (top - st.c);
@@ -1013,12 +1055,29 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                             }
                     }
                     uint32_t l = 0;
+                    bool some = false;  // a slot with q's low word, in the piece or next to it
 #pragma unroll
                     for (int t = 0; t < NS; ++t)
 #pragma unroll
-                        for (uint32_t e = 0; e < KPL; ++e) l |= (v[t][e] < q ? 1u : 0u) << (t * KPL + e);
-                    i = (i << h) + (I)__popc((l >> o) & ((1u << m) - 1));
-                    c += h;
+                        for (uint32_t e = 0; e < KPL; ++e) {
+                            l |= (v[t][e] < q ? 1u : 0u) << (t * KPL + e);
+                            some |= (uint32_t)v[t][e] == (uint32_t)q;
+                        }
+                    const uint32_t piece = ((1u << m) - 1) << o, lt = __popc(l & piece);
+                    if (some) {
+                        uint32_t eq = 0;
+#pragma unroll
+                        for (int t = 0; t < NS; ++t)
+#pragma unroll
+                            for (uint32_t e = 0; e < KPL; ++e) eq |= (v[t][e] == q ? 1u : 0u) << (t * KPL + e);
+                        eq = __popc(eq & piece);
+                        if (eq) {  // of the piece's keys lt + 1 .. lt + eq in order, the highest in the tree
+                            const uint32_t x = (lt + eq) & ~0u << (31 - __clz(lt ^ (lt + eq))), z = __ffs(x);
+                            res = s + sched[j].slot[k][1u << (h - z) | x >> z];
+                            break;
+                        }
+                    }
+                    i = (i << h) + (I)lt;
                 }
                 const tl_veb_table *tab = idx ? tables + __ldg(table_idx + j) : tables;
                 if (slow) {
@@ -1027,20 +1086,8 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                                                       lim64, r);
                     if (rc == 1) res = (I)r;
                     if (rc) break;
-                } else {
-                    // the smallest key of the path at or above q: above the path's trailing right turns
-                    const I right = ~i;
-                    const uint32_t up = sizeof(I) == 8 ? __ffsll((long long)right) : __ffs((int)right);
-                    const I node = up ? (i >> (up - 1)) >> 1 : 0;
-                    if (node) {
-                        const tl_veb_table *t = j < kVebSchedTables ? s_tabs[j] : tab;
-                    const I at = offset + (I)(veb_node_pos(t, c - up, node) - 1);
-                        if (at < limit && __ldg(A + at) == q) {
-                            res = at;
-                            break;
-                        }
-                    }
-                    if (!left) break;  // past the deepest level: absent
+                } else if (res != n || !left) {
+                    break;  // found, or past the deepest level: absent
                 }
                 offset = limit;
             }
