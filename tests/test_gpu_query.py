@@ -452,3 +452,50 @@ def test_duplicate_keys_answer_the_first_on_the_path(layout, b, dtype):
                 Q[:3] = keys[0], keys[-1], keys[-1] + 1
                 assert np.array_equal(gpu_answers(layout, tree, Q, b or 16), O.search(layout, tree, Q, b or 16)), \
                     (layout, b, n, q)
+
+
+@pytest.mark.parametrize("layout", ["mveb", "bst"])
+def test_threads_query_with_different_batches(layout):
+    """Host threads whose launches of one kernel ask for different amounts of
+    shared memory, in tight loops through the C entry: none refuses another's."""
+    import ctypes as C
+    import threading
+
+    import torch
+    n, L = 2**20 + 5, T.lib()
+    keys = data.sorted_keys_torch(n, 1, 16, 3, 8)
+    batches = [keys[torch.randint(0, n, (q,), device="cuda")] for q in (1 << 20, 1 << 10, 1 << 10, 1 << 10)]
+    answers = [torch.empty_like(Q) for Q in batches]
+    streams = [torch.cuda.Stream() for _ in batches]
+    T.permute(layout, keys)
+    tabs = T.VebTablesDevice(n)
+    calls = []
+    for Q, ans, st in zip(batches, answers, streams):
+        tail = (C.c_void_p(Q.data_ptr()), C.c_uint64(Q.numel()), C.c_void_p(ans.data_ptr()), C.c_void_p(st.cuda_stream),
+                None)
+        calls.append((C.c_void_p(keys.data_ptr()), C.c_uint64(n)) + tail if layout == "bst" else
+                     (C.c_void_p(keys.data_ptr()), C.c_void_p(tabs.tables.data_ptr()), C.c_void_p(tabs.idx.data_ptr()),
+                      C.c_void_p(tabs.table_idx.data_ptr()), C.c_uint64(n), C.c_uint32(tabs.d),
+                      C.c_uint32(tabs.num_tables)) + tail)
+    fn = L.tl_query_bst_u64 if layout == "bst" else L.tl_query_veb_nonperfect_u64
+    torch.cuda.synchronize()
+    refused, done = [0] * len(calls), threading.Event()
+
+    def work(w):
+        for _ in range(200):
+            if done.is_set():
+                break
+            for _ in range(100):
+                refused[w] += fn(*calls[w]) != 0
+            streams[w].synchronize()
+        if w == 0:
+            done.set()
+
+    threads = [threading.Thread(target=work, args=(w,)) for w in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert refused == [0] * len(calls)
+    for Q, ans in zip(batches, answers):
+        assert torch.equal(keys[ans], Q)

@@ -972,7 +972,9 @@ static int launch_batch_permute(const tl_batch_plan_impl &P, K *keys, char *ws, 
     const size_t smem = ring * stage + 128;
     auto kern = threads == 512 ? batch_permute_kernel<K, kBatchStoreWarps512> : batch_permute_kernel<K, kBatchStoreWarps256>;
     const int nthreads = 32 * (2 * kBatchStages + (threads == 512 ? kBatchStoreWarps512 : kBatchStoreWarps256));
-    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the same limit whatever the plan's tiles: another thread's smaller plan must not lower it under this launch
+    if (smem > kBatchBlockSmem) return TL_ERROR_UNSUPPORTED;  // (tiles are at most 64 KB: never)
+    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchBlockSmem));
     int per_sm = 0;
     TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nthreads, smem));
     const uint64_t work = P.tot.tiles + P.tot.chunks;

@@ -1465,7 +1465,18 @@ static int query_sm_count() {
     return g_qsm;
 }
 
-constexpr size_t kSmemLimit = 64 * 1024;
+// Dynamic shared memory a launch of each kernel may ask for at most.  A launch
+// sets this as its kernel's limit, not its own need: the limit belongs to the
+// kernel, and a smaller call on another host thread, between this one's limit and
+// its launch, would have the launch refused (seen with 2^10 beside 2^22 vEB
+// queries; below 48 KB too, once a limit has been set).
+constexpr size_t kSmemLimit = 64 * 1024;                                                       // persistent_grid
+constexpr size_t kChunkSmemMax = 32768 + kBstChunk * sizeof(uint16_t);                         // BST and sorted chunks
+constexpr size_t kTopSmemMax = kTopBytes + (kTopBins + 1) * sizeof(uint16_t);                  // btree_query_top_kernel
+constexpr size_t kVebTopMax = 32768;
+constexpr size_t veb_smem_max(size_t index_bytes) {
+    return kVebMaxSteps * kSortThreads * index_bytes + kVebTopMax + kSortChunk * sizeof(uint16_t);
+}
 
 // Resident blocks per SM of a kernel, asked of the runtime once per thread, device
 // and shape (the question and the attribute cost a small batch's call a
@@ -1486,7 +1497,7 @@ static int resident_blocks(const void *kern, size_t smem, int *per_sm) {
             *per_sm = known[i].per_sm;
             return TL_SUCCESS;
         }
-    // one limit for every shape (a later smaller one must not lower it); all ask for at most kPinBytes
+    // all ask for at most kPinBytes
     static_assert(kPinBytes <= kSmemLimit, "the pinned prefix fits the limit");
     if (smem > kSmemLimit) return TL_ERROR_UNSUPPORTED;
     TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
@@ -1546,7 +1557,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
             const uint64_t chunk = (a.q + slots * rounds - 1) / (slots * rounds);  // equal chunks, the fewest rounds
             const size_t bytes = ((size_t)1 << L) * sizeof(K) + chunk * sizeof(uint16_t);
             auto launch = [&](auto kern) -> int {
-                TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+                TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemMax));
                 kern<<<(unsigned)std::min(slots, (a.q + chunk - 1) / chunk), kSortThreads, bytes, st>>>(
                     A, a.n, L, (uint32_t)chunk, Q, a.q, a.answers);
                 TL_CUDA_TRY(cudaGetLastError());
@@ -1577,7 +1588,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         const uint64_t chunk = (a.q + slots * rounds - 1) / (slots * rounds);  // equal chunks, the fewest rounds
         const size_t smem = (top + 1) * sizeof(K) + chunk * sizeof(uint16_t);
         auto launch = [&](auto kern) -> int {
-            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemMax));
             kern<<<(unsigned)std::min(slots, (a.q + chunk - 1) / chunk), kSortThreads, smem, st>>>(
                 A, a.n, (uint32_t)top, (uint32_t)chunk, Q, a.q, a.answers);
             return TL_SUCCESS;
@@ -1640,7 +1651,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         const uint64_t m = btree_top_keys<K>(a.n, a.b);
         auto topped = [&](auto kern, uint64_t lanes_per_query) -> int {
             const size_t bytes = m * sizeof(K) + (kTopBins + 1) * sizeof(uint16_t);
-            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmemMax));
             const uint64_t need = (a.q * lanes_per_query + kTopThreads - 1) / kTopThreads;
             kern<<<(unsigned)std::min<uint64_t>(2 * (uint64_t)query_sm_count(), need), kTopThreads, bytes, st>>>(
                 A, (uint32_t)a.n, (uint32_t)m, Q, a.q, a.answers);
@@ -1727,7 +1738,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         // pinned levels: at most 32 KB from 2^20 queries, else 16 KB (a block
         // gathers them; 2^18 queries over 3e8 u32 keys 41 against 44 us, 2^20 97
         // against 94)
-        const size_t top_bytes = a.q >= (1ull << 20) ? 32 * 1024 : 16 * 1024;
+        const size_t top_bytes = a.q >= (1ull << 20) ? kVebTopMax : kVebTopMax / 2;
         uint32_t max_top = 0;
         while (max_top + 1 < dmax && (sizeof(K) << (max_top + 1)) <= top_bytes) ++max_top;
         auto launch = [&](auto kern) -> int {
@@ -1736,7 +1747,8 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
             const uint64_t chunk = (a.q + slots * rounds - 1) / (slots * rounds);  // equal chunks, the fewest rounds
             const size_t smem = (size_t)cols * kSortThreads * (narrow ? 4 : 8) + (sizeof(K) << max_top) +
                                 chunk * sizeof(uint16_t);
-            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)veb_smem_max(narrow ? 4 : 8)));
             const uint64_t blocks = std::min(slots, (a.q + chunk - 1) / chunk);
             kern<<<(unsigned)blocks, kSortThreads, smem, st>>>(A, a.n, cols, max_top, (uint32_t)chunk, a.tables,
                                                               np ? a.idx : nullptr, np ? a.table_idx : nullptr,

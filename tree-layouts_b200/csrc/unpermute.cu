@@ -700,10 +700,13 @@ static int gather_sms() {
     return g_gather_sms;
 }
 
-// Blocks of a persistent launch over the tiles.
+// Blocks of a persistent launch over the tiles.  The limit is the same for every
+// call: one thread's smaller need (another b) must not lower it under another's launch.
+constexpr size_t kGatherSmemMax = 40 * 1024;
 template <typename Kern>
 static int gather_grid(Kern kern, size_t smem, uint64_t ntiles, unsigned *grid) {
-    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kGatherSmemMax) return TL_ERROR_UNSUPPORTED;  // (a 32 KB tile and its padding: never)
+    TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGatherSmemMax));
     int per_sm = 0;
     TL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGatherThreads, smem));
     *grid = (unsigned)std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * gather_sms(), ntiles);
