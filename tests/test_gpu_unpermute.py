@@ -104,3 +104,28 @@ def test_expired_reverse_wait_reports_timeout_and_context_survives():
         T.set_wait(0, False)
     T.unpermute("btree", lay, 16)
     assert torch.equal(lay, keys)
+
+
+def test_restores_from_a_copy_build_no_tile_tables():
+    """B-trees that go back from a copy use no ordered-tile tables and take no
+    place in the library's cache of them (64 geometries): after 70 such restores a
+    permutation of a new size still has the ordered schedule.  In a process of its
+    own, as the cache is the process's."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = f"""
+import ctypes as C
+import sys
+sys.path.insert(0, {os.path.join(root, "tree-layouts_b200")!r})
+import torch
+import tree_layouts as T
+plan = T.lib().tl_debug_permute_plan
+plan.argtypes = [C.c_int, C.c_uint64, C.c_uint64, C.c_uint32]
+words = torch.arange(2_000_000, device="cuda", dtype=torch.int64)
+for x in range(70):
+    T.unpermute("btree", words[:1_700_000 + 4321 * x].clone(), 16)
+assert plan(1, 3_000_000, 16, 8) == 2
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)

@@ -687,6 +687,16 @@ int permute_workspace_bytes_fixed(int layout, uint64_t n, uint64_t b, uint32_t k
     return TL_SUCCESS;
 }
 
+int permute_plan_fixed(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, PermutePlan &pl) {
+    return make_plan(layout, n, b, key_bytes, pl, ORDER_NEVER);
+}
+
+bool permute_takes_order(int layout, uint64_t n, uint64_t b, uint32_t key_bytes) {
+    PermutePlan fx;
+    return !is_veb_layout(layout) && n > 1 && make_plan(layout, n, b, key_bytes, fx, ORDER_NEVER) == TL_SUCCESS &&
+           order_wanted(fx, ORDER_AUTO);
+}
+
 int permute_plan_device(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, cudaStream_t st, PermutePlan &pl) {
     if (n > 1 && !is_veb_layout(layout)) {
         // a geometry not seen before: its ordered-tile tables with kernels on

@@ -30,6 +30,10 @@ struct PermutePlan {
 // applies and its tables reach the device (its pointers are then device
 // pointers), else the fixed directions.
 int permute_plan_device(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, cudaStream_t st, PermutePlan &pl);
+// The plan with the fixed directions, which needs no tables.
+int permute_plan_fixed(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, PermutePlan &pl);
+// Whether the default plan is on the ordered schedule, its tables permitting.
+bool permute_takes_order(int layout, uint64_t n, uint64_t b, uint32_t key_bytes);
 // The plan for a host replay: the ordered schedule wherever there is one (its
 // tables in ov), or the fixed directions.
 int permute_plan_replay(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, bool ordered, OrderVectors &ov,
