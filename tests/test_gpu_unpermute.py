@@ -129,3 +129,19 @@ for x in range(70):
 assert plan(1, 3_000_000, 16, 8) == 2
 """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
+
+
+@pytest.mark.parametrize("layout", ["mveb", "veb"])
+@pytest.mark.parametrize("n,kb", [(7 << 20, 8), ((7 << 20) + 1, 8), ((14 << 20) - 1, 4), ((14 << 20) + 5, 4)])
+def test_veb_forms_round_trip_at_their_line(layout, n, kb):
+    """vEB arrays of 56 MB go back from a copy, larger ones in place."""
+    import torch
+    keys = data.sorted_keys_torch(n, 1, 3, 5, kb)
+    buf = torch.full((n + 65,), -1, dtype=keys.dtype, device="cuda")
+    t = buf[1:n + 1]
+    t.copy_(keys)
+    T.permute(layout, t)
+    assert not torch.equal(t, keys)
+    T.unpermute(layout, t)
+    assert torch.equal(t, keys)
+    assert int(buf[0]) == -1 and bool((buf[n + 1:] == -1).all())

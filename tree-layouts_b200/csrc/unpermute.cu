@@ -652,8 +652,10 @@ static inline uint64_t align256(uint64_t x) { return (x + 255) / 256 * 256; }
 // 64 MB 72 / 60 / 66, 128 MB 136 / 107 / 102, 256 MB 260 / 192 / 162; b = 2 u32 of
 // 8 MB 29 / 29 / 56, 256 MB 610 / 256 / 272; BST u64 of 16 MB 23 / 24 / 34, 256 MB
 // 252 / 214 / 219 on the fixed directions (39 % of its keys take scratch), 2 GB
-// on the ordered schedule 1129 in place; mvEB u64 from a copy / in place: 16 MB 23
-// / 26, 32 MB 35 / 33, 64 MB 55 / 44, 128 MB 95 / 64.
+// on the ordered schedule 1129 in place; one call's wall time of an
+// mvEB from a copy / in place: u64 of 32 MB 43 / 57, 48 MB 53 / 59, 64 MB 70 / 67,
+// 96 MB 91 / 83, u32 of 48 MB 57 / 61, 64 MB 76 / 71; standard vEB u32 of 48 MB 63 /
+// 81, 64 MB 81 / 85.
 // (Key by key: permute_by_keys, decided before there is a plan.)
 enum ReverseForm { REVERSE_KEYS, REVERSE_COPY, REVERSE_IN_PLACE };
 // Workspace of the in-place form: the scratch (starting at the array's own offset
@@ -675,7 +677,7 @@ static ReverseSpace reverse_space(const PermutePlan &pl) {
 // a place in the library's cache of them.)
 static bool reverse_copies(int layout, uint64_t n, uint64_t b, uint32_t key_bytes) {
     const uint64_t bytes = n * key_bytes;
-    if (is_veb_layout(layout)) return bytes <= (32ull << 20);
+    if (is_veb_layout(layout)) return bytes <= (56ull << 20);
     if (layout == TL_LAYOUT_BTREE && b > 1) return bytes <= (192ull << 20);
     return !permute_takes_order(layout, n, b, key_bytes);
 }
