@@ -323,7 +323,9 @@ __device__ __forceinline__ void bar_sync_tail() {
 // kTops: top keys a thread loads at a time.  Where they are a ninth of the keys or
 // more (b <= 8), four at 5 blocks an SM (48 registers): b = 8 over 6e7 u64 keys 220
 // us against 226 with one at 6 blocks, b = 3 over 2^27 509 / 528, BST over 2^28 - 1
-// 1126 / 1214; above, one at 6 blocks: b = 16 over 5e8 1403 against 1491 us.
+// 1126 / 1214; above, one at 6 blocks: b = 16 over 5e8 1403 against 1491 us.  From a
+// copy two at a time (one call, four / one / two / eight: BST over 1.7e7 u32 keys 98 /
+// 104 / 92 / 108, over 4e7 184 / 184 / 171 / 202, b = 8 over 3.4e7 133 / - / 128 / -).
 template <typename K, bool kCopy, int kTops>
 __global__ void __launch_bounds__(kGatherThreads, kTops == 1 ? kGatherBlocksPerSM : kGatherBlocksPerSM - 1)
 btree_unstream_kernel(K *__restrict__ A, const K *__restrict__ scr, const __grid_constant__ BtreeStream S,
@@ -742,7 +744,7 @@ static int launch_from_copy(const PermutePlan &pl, const KeysGeometry &kg, Rever
     } else {
         uint32_t top_at = 0;
         const size_t smem = btree_gather_keys(pl.tile_keys, pl.b, sizeof(K), &top_at) * sizeof(K) + 128;
-        auto kern = pl.b <= 8 ? btree_unstream_kernel<K, true, 4> : btree_unstream_kernel<K, true, 1>;
+        auto kern = pl.b <= 8 ? btree_unstream_kernel<K, true, 2> : btree_unstream_kernel<K, true, 1>;
         rc = gather_grid(kern, smem, pl.ntiles, &grid);
         if (rc) return rc;
         BtreeStream S = pl.bs;  // left to right with slots at their positions: last-level and tail tiles are staged
