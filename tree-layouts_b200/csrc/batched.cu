@@ -66,7 +66,8 @@ constexpr uint64_t kRangePiece = 2048;
 // b = 16 need 277 MB instead of 191).  Measured on B200, 1024 arrays of
 // 2^10..2^22 keys, 0.3 everywhere against this: b = 8 1.75 -> 1.64 ms, b = 1 2.35
 // -> 2.12, b = 4 2.03 -> 1.96 (1.88 whatever the space), b = 16 1.59 -> 1.57.
-// Their longer item lists make the plan, built once, 23 ms instead of 20.
+// Their tables and item lists are 1 to 2 ms of a plan of 9, which a plan that only
+// answers queries pays too.
 constexpr double kOrderGain = 0.9, kOrderGainSpace = 0.3;
 constexpr uint64_t kInterleaveRun = 1;  // stream tiles an instance takes in a row
 static_assert(sizeof(BatchInst) % 16 == 0, "BatchInst is copied to shared memory in 16-byte words");
@@ -85,7 +86,7 @@ struct tl_batch_plan_impl {
     uint32_t num = 0, key_bytes = 8;
     uint64_t b = 8;
     BatchInst *inst = nullptr;   // device
-    BatchGeo *geo = nullptr;     // device: per instance, for the queries
+    BatchGeo *geo = nullptr;     // device, behind inst: per instance, for the queries
     BatchTotals tot{};
     uint32_t tile_keys[kMaxClass];
     uint32_t pin_levels[kMaxClass];  // kept for tl_batch_get_tuning; the queries do not use it
@@ -94,8 +95,8 @@ struct tl_batch_plan_impl {
     uint32_t *owner = nullptr;   // device: owner instance of every tile ticket, then of every copy chunk
     uint32_t *tile = nullptr;    // device: the tile of its owner every tile ticket processes
     char *otab = nullptr;        // device: the ordered instances' tile tables (uint2 tab, then uint32 order)
-    FixSeg *items = nullptr;     // device: the ordered instances' copy items
-    uint64_t *citem = nullptr;   // device: first copy item of every copy chunk of an ordered instance
+    FixSeg *items = nullptr;     // device, behind otab: the ordered instances' copy items
+    uint64_t *citem = nullptr;   // device, behind items: first copy item of every copy chunk of an ordered instance
     uint64_t ordered = 0;        // instances on the ordered schedule
     uint64_t ordered_keys = 0;   // their keys
     uint64_t off_flags = 0, off_done = 0, off_ctrl = 0, ws_bytes = 0;
@@ -624,26 +625,20 @@ static void default_tuning(tl_batch_plan_impl &P) {
 
 static void free_order_buffers(tl_batch_plan_impl &P) {
     if (P.otab) cudaFree(P.otab);
-    if (P.items) cudaFree(P.items);
-    if (P.citem) cudaFree(P.citem);
     P.otab = nullptr;
     P.items = nullptr;
     P.citem = nullptr;
     P.ordered = P.ordered_keys = 0;
 }
 
-// A device copy of v, landed when this returns (copied on st, then waited for:
-// a plain cudaMemcpy from pageable memory may return before its DMA lands).
-template <typename T>
-static int upload(T *&dst, const std::vector<T> &v, cudaStream_t st) {
-    if (cudaMalloc(reinterpret_cast<void **>(&dst), std::max<size_t>(v.size(), 1) * sizeof(T)) != cudaSuccess) {
-        cudaGetLastError();
-        dst = nullptr;
-        return TL_ERROR_OUT_OF_MEMORY;
-    }
-    if (!v.empty()) TL_CUDA_TRY(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-    TL_CUDA_TRY(cudaStreamSynchronize(st));
-    return TL_SUCCESS;
+// Device memory of a plan: one cudaMalloc (0.1 to 0.2 ms) for what was built
+// together.  Not from the pool: the cudaFree of such memory waits for the kernels
+// that may still read the plan, that of pool memory does not.
+static int plan_memory(void **p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return TL_SUCCESS;
+    cudaGetLastError();
+    *p = nullptr;
+    return TL_ERROR_OUT_OF_MEMORY;
 }
 
 // Keys through scratch under an instance's fixed-direction schedule and under
@@ -726,8 +721,6 @@ static int order_instances(tl_batch_plan_impl &P, const std::vector<int64_t> &of
         memcpy(tb.data() + toff[i], ov[i].tab.data(), N * sizeof(uint2));
         memcpy(tb.data() + toff[i] + N * sizeof(uint2), ov[i].order.data(), N * sizeof(uint32_t));
     }
-    int rc = upload(P.otab, tb, st);
-    if (rc) return rc;
     std::vector<FixSeg> items;
     std::vector<uint64_t> citem;
     const uint64_t vec = 16 / P.key_bytes;
@@ -737,10 +730,7 @@ static int order_instances(tl_batch_plan_impl &P, const std::vector<int64_t> &of
         I.chunk_base = citem.size();
         if (ord_of[j] >= 0) {
             const OrderVectors &v = ov[ord_of[j]];
-            const size_t N = v.order.size();
-            const char *t = P.otab + toff[ord_of[j]];
-            btree_set_ordered(I.S, reinterpret_cast<const uint2 *>(t),
-                              reinterpret_cast<const uint32_t *>(t + N * sizeof(uint2)), v.scratch_tiles);
+            btree_set_ordered(I.S, nullptr, nullptr, v.scratch_tiles);  // its tables below
             const uint64_t T = I.S.tile_keys, n = I.S.g.n;
             I.item_base = items.size();
             for (const uint4 &r : v.ranges)  // whole-tile runs, in pieces
@@ -776,14 +766,29 @@ static int order_instances(tl_batch_plan_impl &P, const std::vector<int64_t> &of
     }
     P.tot.scratch = bs;
     P.tot.chunks = citem.size();
-    rc = upload(P.items, items, st);
-    if (!rc) rc = upload(P.citem, citem, st);
-    if (!rc) {
-        TL_CUDA_TRY(cudaMemcpyAsync(P.inst, h.data(), h.size() * sizeof(BatchInst), cudaMemcpyHostToDevice, st));
-        TL_CUDA_TRY(cudaStreamSynchronize(st));
+    const size_t items_at = (tbytes + 15) / 16 * 16, citem_at = items_at + items.size() * sizeof(FixSeg);
+    const int rc = plan_memory(reinterpret_cast<void **>(&P.otab), citem_at + citem.size() * sizeof(uint64_t));
+    if (rc) {
+        free_order_buffers(P);
+        return rc;
     }
-    if (rc) free_order_buffers(P);
-    return rc;
+    P.items = reinterpret_cast<FixSeg *>(P.otab + items_at);
+    P.citem = reinterpret_cast<uint64_t *>(P.otab + citem_at);
+    for (size_t i = 0; i < cand.size(); ++i) {
+        if (ord_of[cand[i]] < 0) continue;
+        BtreeStream &S = h[cand[i]].S;
+        S.tab = reinterpret_cast<const uint2 *>(P.otab + toff[i]);
+        S.order = reinterpret_cast<const uint32_t *>(P.otab + toff[i] + ov[i].order.size() * sizeof(uint2));
+    }
+    // copied on st, then waited for: a plain cudaMemcpy from pageable memory may return before its DMA lands
+    TL_CUDA_TRY(cudaMemcpyAsync(P.otab, tb.data(), tbytes, cudaMemcpyHostToDevice, st));
+    if (!items.empty())
+        TL_CUDA_TRY(cudaMemcpyAsync(P.items, items.data(), items.size() * sizeof(FixSeg), cudaMemcpyHostToDevice, st));
+    if (!citem.empty())
+        TL_CUDA_TRY(cudaMemcpyAsync(P.citem, citem.data(), citem.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+    TL_CUDA_TRY(cudaMemcpyAsync(P.inst, h.data(), h.size() * sizeof(BatchInst), cudaMemcpyHostToDevice, st));
+    TL_CUDA_TRY(cudaStreamSynchronize(st));
+    return TL_SUCCESS;
 }
 
 // The order in which the persistent kernel takes the stream tiles: each
@@ -817,7 +822,22 @@ static int interleave_tiles(const tl_batch_plan_impl &P, const std::vector<int64
     }
     // tile indices and the kernel's tickets are 32-bit
     if (sum != P.tot.tiles || sum + P.tot.chunks >= (1ull << 31)) return TL_ERROR_UNSUPPORTED;
-    std::stable_sort(runs.begin(), runs.end(), [](const Run &a, const Run &b) { return a.key < b.key; });
+    // by progress, ties in instance order: into as many buckets of equal width as there are runs, then each bucket
+    // (sorted whole, 1.3e5 runs took 4.7 ms of a plan of 11)
+    {
+        const size_t M = runs.size();
+        auto bucket = [&](const Run &q) { return std::min(M - 1, (size_t)(q.key * (double)M)); };
+        std::vector<uint32_t> at(M + 1, 0);
+        for (const Run &q : runs) ++at[bucket(q) + 1];
+        for (size_t k = 0; k < M; ++k) at[k + 1] += at[k];
+        std::vector<Run> in(std::move(runs));
+        runs.resize(M);
+        for (const Run &q : in) runs[at[bucket(q)]++] = q;  // at[k] is now the end of bucket k
+        for (size_t k = 0, lo = 0; k < M; lo = at[k++])
+            if (at[k] - lo > 1)
+                std::stable_sort(runs.begin() + lo, runs.begin() + at[k],
+                                 [](const Run &a, const Run &b) { return a.key < b.key; });
+    }
     own.clear();
     loc.clear();
     own.reserve(sum);
@@ -906,16 +926,16 @@ int batch_plan_create(const int64_t *dev_offsets, uint32_t num, uint64_t b, uint
     P->b = b;
     P->key_bytes = key_bytes;
     default_tuning(*P);
-    if (cudaMalloc(reinterpret_cast<void **>(&P->inst), (size_t)num * sizeof(BatchInst)) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void **>(&P->geo), (size_t)num * sizeof(BatchGeo)) != cudaSuccess) {
-        cudaFree(P->inst);
+    const size_t geo_at = ((size_t)num * sizeof(BatchInst) + 31) / 32 * 32;
+    int rc = plan_memory(reinterpret_cast<void **>(&P->inst), geo_at + (size_t)num * sizeof(BatchGeo));
+    if (rc) {
         delete P;
-        return TL_ERROR_OUT_OF_MEMORY;
+        return rc;
     }
-    int rc = build_plan(*P, dev_offsets, st);
+    P->geo = reinterpret_cast<BatchGeo *>(reinterpret_cast<char *>(P->inst) + geo_at);
+    rc = build_plan(*P, dev_offsets, st);
     if (rc) {
         cudaFree(P->inst);
-        cudaFree(P->geo);
         if (P->owner) cudaFree(P->owner);
         if (P->tile) cudaFree(P->tile);
         free_order_buffers(*P);
@@ -929,8 +949,7 @@ int batch_plan_create(const int64_t *dev_offsets, uint32_t num, uint64_t b, uint
 int batch_plan_destroy(tl_batch_plan *plan) {
     if (!plan) return TL_ERROR_INVALID_VALUE;
     auto *P = reinterpret_cast<tl_batch_plan_impl *>(plan);
-    cudaFree(P->inst);
-    cudaFree(P->geo);
+    cudaFree(P->inst);  // first: it waits for work in flight, the frees of pool memory do not
     if (P->owner) cudaFree(P->owner);
     if (P->tile) cudaFree(P->tile);
     free_order_buffers(*P);
