@@ -431,6 +431,20 @@ def test_sorted_array_ordered_chunks(kb, n, skip):
     _check_answers(arr, keys, Q, ans)
 
 
+@pytest.mark.parametrize("layout", ["mveb", "veb"])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+@pytest.mark.parametrize("n", [(1 << 22) - 1, 1 << 22, 5_000_011])
+def test_duplicate_keys_on_either_side_of_the_veb_forms(layout, dtype, n):
+    """The same for the two forms of the vEB search, which meet equal keys in the
+    pieces (from 2^22 keys) or at the path's left turns."""
+    keys = _with_duplicates(n, n, dtype)
+    tree = O.permute(layout, keys, 16)
+    for q in (1000, (1 << 17) + 77):
+        Q = data.queries_np(keys, q, 0.7, 3)
+        Q[:3] = keys[0], keys[-1], keys[-1] + 1
+        assert np.array_equal(gpu_answers(layout, tree, Q), O.search(layout, tree, Q)), q
+
+
 def _with_duplicates(n, seed, dtype):
     """n sorted keys, runs of one value geometrically long."""
     rng = np.random.default_rng(seed)
@@ -499,3 +513,23 @@ def test_threads_query_with_different_batches(layout):
     assert refused == [0] * len(calls)
     for Q, ans in zip(batches, answers):
         assert torch.equal(keys[ans], Q)
+
+
+@pytest.mark.parametrize("layout", ["mveb", "veb", "bst"])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+@pytest.mark.parametrize("last", [0, 1])
+def test_small_layouts_and_the_largest_key(layout, dtype, last):
+    """Layouts held whole in shared memory, perfect and of several divisions, on
+    either side of what is held at each batch size; with and without the type's
+    largest value among the keys, queried for it."""
+    top = int(np.iinfo(dtype).max)
+    for n in (1, 2, 3, 5, 30, 31, 255, 1000, 2047, 2048, 4101, 8191, 8192, 16383, 16384):
+        keys = data.sorted_keys_np(n, 1, 5, n, dtype)
+        if last:
+            keys[-1] = top
+        tree = O.permute(layout, keys, 16)
+        for q in (1500, (1 << 17) + 3):
+            Q = data.queries_np(keys, q, 0.5, n + 1)
+            Q[:5] = 0, top, top - 1, keys[0], keys[-1]
+            Q[5:40] = top
+            assert np.array_equal(gpu_answers(layout, tree, Q), O.search(layout, tree, Q)), (layout, n, q)

@@ -688,25 +688,32 @@ __device__ __forceinline__ void chunk_order(const K *__restrict__ Q, uint32_t le
 // 2^26 - 1 1181 -> 844, over 2^24 - 1 1574 -> 660; 2^20 over 2^27 - 1 keys 265 -> 87, over
 // 2^20 - 1 62 -> 31.  Chunks of 8192 or 16384, or 64 KB of top levels, take L1 from
 // the descents (1205, 1193, 1471 us); one block an SM 1.5 times the time.
+// Trees of up to 1 MB, and arrays of up to 8 MB in the search below, are searched in
+// the batch's order: L1 and L2 serve them in any, and the ordering only costs (2^24
+// queries, as given / in ordered chunks, us: BST over 255 u64 keys 95 / 187, over
+// 65535 250 / 278, over 4e5 395 / 361, u32 over 1.5e5 222 / 248, over 4e5 304 / 291;
+// sorted u64 over 255 115 / 191, over 4e5 552 / 579, over 1e6 622 / 657).
+constexpr uint64_t kBstOrderBytes = 1ull << 20, kSortedOrderBytes = 8ull << 20;
 constexpr uint32_t kBstChunk = 4096;
 constexpr int kBstBlocksPerSM = 2;
 
 template <typename K, typename I>
 __global__ void __launch_bounds__(kSortThreads, kBstBlocksPerSM)
-bst_query_sorted_kernel(const K *__restrict__ A, uint64_t n64, uint32_t P, uint32_t chunk, const K *__restrict__ Q,
-                        uint64_t nq, uint64_t *__restrict__ ans) {
+bst_query_sorted_kernel(const K *__restrict__ A, uint64_t n64, uint32_t P, uint32_t chunk, bool sorted,
+                        const K *__restrict__ Q, uint64_t nq, uint64_t *__restrict__ ans) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K *sm = reinterpret_cast<K *>(smem_raw);                     // [P + 1], from 1
     uint16_t *order = reinterpret_cast<uint16_t *>(sm + P + 1);  // [chunk]
     __shared__ ChunkSort cs;
     const I n = (I)n64;
     for (uint32_t x = threadIdx.x; x < P; x += kSortThreads) sm[x + 1] = __ldg(A + x);
+    __syncthreads();
     const uint32_t levels = bit_length((uint64_t)P);
     for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
         const uint32_t len = (uint32_t)min((uint64_t)chunk, nq - c0);
-        chunk_order<kBstChunk / kSortThreads>(Q + c0, len, order, cs);  // its barriers also cover the top
+        if (sorted) chunk_order<kBstChunk / kSortThreads>(Q + c0, len, order, cs);
         for (uint32_t slot = threadIdx.x; slot < len; slot += kSortThreads) {
-            const uint64_t qi = c0 + order[slot];
+            const uint64_t qi = c0 + (sorted ? order[slot] : slot);
             const K q = __ldg(Q + qi);
             uint32_t y = 1;
             for (uint32_t c = 0; c < levels; ++c) y = 2 * y + (sm[y] < q);
@@ -743,8 +750,8 @@ constexpr uint64_t kSortedChunkMin = 1ull << 16;
 
 template <typename K, typename I>
 __global__ void __launch_bounds__(kSortThreads, kBstBlocksPerSM)
-sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uint32_t chunk, const K *__restrict__ Q,
-                          uint64_t nq, uint64_t *__restrict__ ans) {
+sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uint32_t chunk, bool sorted,
+                          const K *__restrict__ Q, uint64_t nq, uint64_t *__restrict__ ans) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K *tree = reinterpret_cast<K *>(smem_raw);                              // tree[1 .. 2^L - 1]
     uint16_t *order = reinterpret_cast<uint16_t *>(tree + ((size_t)1 << L));  // [chunk]
@@ -761,11 +768,12 @@ sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uin
         }
         tree[node] = __ldg(A + base + (len >> 1));
     }
+    __syncthreads();
     for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
         const uint32_t cl = (uint32_t)min((uint64_t)chunk, nq - c0);
-        chunk_order<kBstChunk / kSortThreads>(Q + c0, cl, order, cs);  // its barriers also cover the tree
+        if (sorted) chunk_order<kBstChunk / kSortThreads>(Q + c0, cl, order, cs);
         for (uint32_t slot = threadIdx.x; slot < cl; slot += kSortThreads) {
-            const uint64_t qi = c0 + order[slot];
+            const uint64_t qi = c0 + (sorted ? order[slot] : slot);
             const K q = __ldg(Q + qi);
             I base = 0, len = n;
             uint32_t node = 1;
@@ -817,10 +825,19 @@ sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uin
 // wavefronts, twice the instructions); 512-thread blocks 5.8; chunks of 4096 /
 // 8192 / 32768 queries 4.76 / 4.46 / 4.62; 64 KB of pinned levels 4.6 (L1 is
 // smaller).  It holds for every batch: 2^10 queries 27 -> 14 us, 2^20 369 -> 95.
-// Equal keys are met in the pieces on the way, where following the counts to the
-// bottom and looking at the path's last left turn took 4.24 ms against 3.99 (u64
-// 1.70 against 1.75 for 2^24 queries) and gave the lowest of equal keys; looking
-// at the left turns above it too took 4.41.
+// From 2^22 keys equal keys are met in the pieces on the way (kPieceEq): a compare
+// more a key, and no load at the end.  Below, where L1 and L2 serve the layout and
+// instructions bound it, they are looked for at the path's left turns, a load for a
+// miss and two for a hit.  2^24 queries, pieces / left turns (us): u32 mvEB 2e4 keys
+// 502 / 430, 4e5 707 / 669, 3e6 741 / 795, 3e8 1012 / 1144; u32 standard vEB 1e6 796 /
+// 707, 1e7 797 / 783, 3e7 819 / 885; u64 mvEB 1.6e4 532 / 507, 1e6 1040 / 1088, 1e7
+// 1202 / 1263.
+//
+// A layout whose first division fits 64 KB (16 KB below 2^22 queries, where the
+// blocks' gathering counts) is held whole, its batch searched as given if it has no
+// other division: 2^24 queries over 255 u64 keys 391 -> 221 us, 4095 437 -> 258, 4101
+// 559 -> 485, 8191 486 -> 270 (with the layout's first keys pinned and a level at a
+// time 292, 481, 830 and 702).
 //
 // Tables whose pieces do not chain (not built by buildTable), a piece that
 // reaches past its division, and divisions beyond the first kVebSchedTables
@@ -829,6 +846,7 @@ sorted_query_chunk_kernel(const K *__restrict__ A, uint64_t n64, uint32_t L, uin
 // only ever issues hits).
 constexpr uint32_t kVebPieceLevels = 4;
 constexpr uint32_t kVebMaxSteps = 16;
+constexpr uint64_t kVebPieceEqMin = 1ull << 22;  // keys
 constexpr uint32_t kVebSchedTables = 4;  // divisions with a piece schedule (the rest hold a few keys)
 
 struct VebStep {
@@ -839,6 +857,7 @@ struct VebStep {
 struct VebSchedule {
     VebStep step[kVebMaxSteps];
     unsigned char slot[kVebMaxSteps][1u << kVebPieceLevels];  // the place in its piece of a node, in BFS order from 1
+    unsigned char at[64];  // the step whose piece holds a depth
     uint32_t steps;  // 0: level by level
     uint32_t top, ktop;  // levels held in shared memory, and the step that starts below them
 };
@@ -880,7 +899,8 @@ __device__ __forceinline__ uint32_t veb_piece_levels(const tl_veb_table *tab, ui
 // The piece schedule of a table of d levels, by one warp: tab gets the table,
 // piece is 64 bytes of scratch.  The levels [0, out.top) go to shared memory:
 // down to the start of a piece, at most max_top, all of their keys below
-// position `limit` (the rightmost node of a depth has the largest position).
+// position `limit` (the rightmost node of a depth has the largest position); or
+// all d of them where max_top allows it.
 __device__ void veb_schedule(const tl_veb_table *__restrict__ gtab, uint32_t d, uint32_t max_steps, uint32_t max_top,
                              uint64_t limit, VebSchedule &out, tl_veb_table *tab, unsigned char *piece) {
     const uint32_t lane = threadIdx.x & 31;
@@ -917,16 +937,24 @@ __device__ void veb_schedule(const tl_veb_table *__restrict__ gtab, uint32_t d, 
         uint32_t kt = 0;
         while (kt + 1 < k && out.step[kt + 1].c <= min(max_top, full)) ++kt;
         out.ktop = kt;
-        out.top = k ? out.step[kt].c : 0;
+        out.top = k ? (max_top >= d ? d : out.step[kt].c) : 0;
     }
 }
 
-// VebSchedule::slot of one piece's node (0: none), relative to the depth's leftmost piece.
+// VebSchedule::slot and ::at of one piece's node (0: none).  The recurrence of its
+// position goes through nodes of the piece, up to the piece's root.
 __device__ __forceinline__ void veb_slot(const tl_veb_table *tab, VebSchedule &sch, uint32_t k, uint32_t node) {
-    const uint32_t c = sch.step[k].c, e = node ? 31 - __clz(node) : 0;
-    if (k < sch.steps && node && e < sch.step[k].h)
-        sch.slot[k][node] = (unsigned char)(veb_node_pos(tab, c + e, ((1ull << c) << e) | (node & ((1u << e) - 1))) -
-                                            veb_node_pos(tab, c, 1ull << c));
+    if (k >= sch.steps || !node || node >= 1u << sch.step[k].h) return;
+    const uint32_t c = sch.step[k].c, e = 31 - __clz(node);
+    uint32_t p = 0, i = node;
+    for (uint32_t d = c + e; d != c;) {
+        const uint32_t R = (uint32_t)tab[d].R, D = tab[d].D;
+        p += R + (i & R) * (uint32_t)tab[d].L;
+        i >>= d - D;
+        d = D;
+    }
+    sch.slot[k][node] = (unsigned char)p;
+    if (node == 1u << e) sch.at[c + e] = (unsigned char)k;
 }
 
 // One descent level by level.  Returns 1 found (res), 2 absent, 0 left the
@@ -956,16 +984,20 @@ __device__ __noinline__ int veb_descend_levels(const K *__restrict__ A, const tl
 
 // idx == nullptr: perfect layout, one table (timeQueryvEB); otherwise the
 // non-perfect table set (timeQueryvEB_nonperfect): the divisions in order, each
-// query until it is resolved.  I: index type (32 bits when n < 2^31).
-template <typename K, typename I>
+// query until it is resolved.  I: index type (32 bits when n < 2^31).  kPieceEq:
+// equal keys are met in the pieces on the way; else the path is followed to its
+// end on counts, and they are where it last went left (of several, the first such
+// turn while the one below is equal too).
+template <typename K, typename I, bool kPieceEq>
 __global__ void __launch_bounds__(kSortThreads, 1)
-veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t max_top, uint32_t chunk,
+veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t max_top, uint32_t chunk, bool sorted,
                  const tl_veb_table *__restrict__ tables, const uint64_t *__restrict__ idx,
                  const uint32_t *__restrict__ table_idx, uint32_t num_tables, const K *__restrict__ Q, uint64_t nq,
                  uint64_t *__restrict__ ans) {
     constexpr uint32_t KPL = 32 / sizeof(K);             // keys per sector
     constexpr uint32_t M = (1u << kVebPieceLevels) - 1;  // keys of the longest piece
     constexpr int NS = (M + KPL - 1 + KPL - 1) / KPL;    // sectors it may span
+    constexpr K kAbsent = ~K(0);  // in the tree: no key there (a parent's position is below its children's)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     I *pos = reinterpret_cast<I *>(smem_raw) + threadIdx.x;  // [cols][kSortThreads], this thread's column
     K *tree = reinterpret_cast<K *>(smem_raw + (size_t)cols * kSortThreads * sizeof(I));  // [2^max_top], from 1
@@ -988,18 +1020,20 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
     if (const uint32_t j = threadIdx.x / kSlots; j < min(num_tables, kVebSchedTables))
         veb_slot(s_tabs[j], sched[j], (threadIdx.x % kSlots) >> kVebPieceLevels, threadIdx.x & ((1u << kVebPieceLevels) - 1));
     const uint32_t top = sched[0].top;
+    const uint64_t end0 = min(n64, idx ? __ldg(idx) : n64);  // of division 0
+    const bool whole = top >= bit_length(n64);               // it is all in shared memory
     for (uint32_t x = threadIdx.x + 1; x < (1u << top); x += kSortThreads) {
         const uint64_t p = veb_node_pos(s_tab, 31 - __clz(x), x) - 1;
-        tree[x] = p < n64 ? __ldg(A + p) : K(0);
+        tree[x] = p < end0 ? __ldg(A + p) : kAbsent;
     }
     __syncthreads();
     const uint32_t a_off = (uint32_t)(reinterpret_cast<uintptr_t>(A) & 31) / sizeof(K);
     const I low = a_off ? KPL : 0;  // a piece from here on can be read in whole sectors
     for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < nq; c0 += (uint64_t)gridDim.x * chunk) {
         const uint32_t len = (uint32_t)min((uint64_t)chunk, nq - c0);
-        chunk_order<0>(Q + c0, len, order, cs);
+        if (sorted) chunk_order<0>(Q + c0, len, order, cs);
         for (uint32_t slot = threadIdx.x; slot < len; slot += kSortThreads) {
-            const uint64_t qi = c0 + order[slot];
+            const uint64_t qi = c0 + (sorted ? order[slot] : slot);
             const K q = __ldg(Q + qi);
             I res = n, offset = 0;
             for (uint32_t j = 0; j < num_tables; ++j) {
@@ -1008,17 +1042,28 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                 const uint32_t steps = j < kVebSchedTables ? sched[j].steps : 0;
                 bool slow = steps == 0, left = false;
                 I i = 1;
-                uint32_t k = 0;
+                uint32_t k = 0, c = 0;
                 if (j == 0 && top) {
                     uint32_t x = 1;
-                    for (uint32_t c = 0; c < top; ++c) x = 2 * x + (tree[x] < q);
+                    for (; c < top; ++c) x = 2 * x + (tree[x] < q);
                     i = x;
                     // an equal key is where the path last went left, or above that at a left turn equal too
-                    uint32_t hit = 0;
-                    for (uint32_t at = x >> __ffs(~x); at && tree[at] == q; at >>= __ffs(~at)) hit = at;
+                    uint32_t at = x >> __ffs(~x), hit = 0;
+                    if (whole && q != kAbsent)
+                        while (at && tree[at] == kAbsent) at >>= __ffs(~at);
+                    if (kPieceEq || whole)
+                        for (; at && tree[at] == q; at >>= __ffs(~at)) hit = at;
                     if (hit) {
-                        res = (I)(veb_node_pos(s_tab, 31 - __clz(hit), hit) - 1);
-                        break;
+                        const I p = (I)(veb_node_pos(s_tab, 31 - __clz(hit), hit) - 1);
+                        if (p < limit) {
+                            res = p;
+                            break;
+                        }
+                    }
+                    if (whole) {  // absent, or past the division's end where the path's last node is
+                        if (!idx || veb_node_pos(s_tab, top - 1, x >> 1) <= lim64) break;
+                        offset = limit;
+                        continue;
                     }
                     for (; k < sched[0].ktop; ++k) {
                         const VebStep &st = sched[0].step[k];
@@ -1061,10 +1106,10 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
 #pragma unroll
                         for (uint32_t e = 0; e < KPL; ++e) {
                             l |= (v[t][e] < q ? 1u : 0u) << (t * KPL + e);
-                            some |= (uint32_t)v[t][e] == (uint32_t)q;
+                            if constexpr (kPieceEq) some |= (uint32_t)v[t][e] == (uint32_t)q;
                         }
                     const uint32_t piece = ((1u << m) - 1) << o, lt = __popc(l & piece);
-                    if (some) {
+                    if (kPieceEq && some) {
                         uint32_t eq = 0;
 #pragma unroll
                         for (int t = 0; t < NS; ++t)
@@ -1078,6 +1123,7 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                         }
                     }
                     i = (i << h) + (I)lt;
+                    c += h;
                 }
                 const tl_veb_table *tab = idx ? tables + __ldg(table_idx + j) : tables;
                 if (slow) {
@@ -1086,8 +1132,21 @@ veb_query_kernel(const K *__restrict__ A, uint64_t n64, uint32_t cols, uint32_t 
                                                       lim64, r);
                     if (rc == 1) res = (I)r;
                     if (rc) break;
-                } else if (res != n || !left) {
-                    break;  // found, or past the deepest level: absent
+                } else {
+                    if constexpr (!kPieceEq)
+                        while (true) {
+                            const I right = ~i;
+                            const uint32_t up = sizeof(I) == 8 ? __ffsll((long long)right) : __ffs((int)right);
+                            i = (i >> (up - 1)) >> 1;
+                            if (!i) break;
+                            c -= up;
+                            const uint32_t kk = sched[j].at[c], d = c - sched[j].step[kk].c;
+                            const I at = offset + (I)(pos[kk * kSortThreads] - 1 +
+                                                      sched[j].slot[kk][(1u << d) | ((uint32_t)i & ((1u << d) - 1))]);
+                            if (__ldg(A + at) != q) break;
+                            res = at;
+                        }
+                    if (res != n || !left) break;  // found, or past the deepest level: absent
                 }
                 offset = limit;
             }
@@ -1474,8 +1533,10 @@ constexpr size_t kSmemLimit = 64 * 1024;                                        
 constexpr size_t kChunkSmemMax = 32768 + kBstChunk * sizeof(uint16_t);                         // BST and sorted chunks
 constexpr size_t kTopSmemMax = kTopBytes + (kTopBins + 1) * sizeof(uint16_t);                  // btree_query_top_kernel
 constexpr size_t kVebTopMax = 32768;
-constexpr size_t veb_smem_max(size_t index_bytes) {
-    return kVebMaxSteps * kSortThreads * index_bytes + kVebTopMax + kSortChunk * sizeof(uint16_t);
+constexpr size_t kVebWholeMax = 65536;
+constexpr size_t veb_smem_max(size_t index_bytes) {  // (the wide index comes with layouts that are not held whole)
+    return kVebMaxSteps * kSortThreads * index_bytes + (index_bytes == 4 ? kVebWholeMax : kVebTopMax) +
+           kSortChunk * sizeof(uint16_t);
 }
 
 // Resident blocks per SM of a kernel, asked of the runtime once per thread, device
@@ -1559,7 +1620,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
             auto launch = [&](auto kern) -> int {
                 TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemMax));
                 kern<<<(unsigned)std::min(slots, (a.q + chunk - 1) / chunk), kSortThreads, bytes, st>>>(
-                    A, a.n, L, (uint32_t)chunk, Q, a.q, a.answers);
+                    A, a.n, L, (uint32_t)chunk, tree_bytes > kSortedOrderBytes, Q, a.q, a.answers);
                 TL_CUDA_TRY(cudaGetLastError());
                 return TL_SUCCESS;
             };
@@ -1590,7 +1651,7 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         auto launch = [&](auto kern) -> int {
             TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemMax));
             kern<<<(unsigned)std::min(slots, (a.q + chunk - 1) / chunk), kSortThreads, smem, st>>>(
-                A, a.n, (uint32_t)top, (uint32_t)chunk, Q, a.q, a.answers);
+                A, a.n, (uint32_t)top, (uint32_t)chunk, tree_bytes > kBstOrderBytes, Q, a.q, a.answers);
             return TL_SUCCESS;
         };
         const int rc = a.n < (1ull << 31) ? launch(bst_query_sorted_kernel<K, uint32_t>)
@@ -1739,7 +1800,9 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
         // gathers them; 2^18 queries over 3e8 u32 keys 41 against 44 us, 2^20 97
         // against 94)
         const size_t top_bytes = a.q >= (1ull << 20) ? kVebTopMax : kVebTopMax / 2;
-        uint32_t max_top = 0;
+        // a small layout is held whole, and its batch searched as given
+        const bool whole = (sizeof(K) << dmax) <= (a.q >= (1ull << 22) ? kVebWholeMax : kVebTopMax / 2);
+        uint32_t max_top = whole ? dmax : 0;
         while (max_top + 1 < dmax && (sizeof(K) << (max_top + 1)) <= top_bytes) ++max_top;
         auto launch = [&](auto kern) -> int {
             const uint64_t slots = query_sm_count();
@@ -1750,12 +1813,14 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
             TL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)veb_smem_max(narrow ? 4 : 8)));
             const uint64_t blocks = std::min(slots, (a.q + chunk - 1) / chunk);
-            kern<<<(unsigned)blocks, kSortThreads, smem, st>>>(A, a.n, cols, max_top, (uint32_t)chunk, a.tables,
+            kern<<<(unsigned)blocks, kSortThreads, smem, st>>>(A, a.n, cols, max_top, (uint32_t)chunk, !whole || (np && a.num_tables > 1), a.tables,
                                                               np ? a.idx : nullptr, np ? a.table_idx : nullptr,
                                                               np ? a.num_tables : 1u, Q, a.q, a.answers);
             return TL_SUCCESS;
         };
-        const int rc = narrow ? launch(veb_query_kernel<K, uint32_t>) : launch(veb_query_kernel<K, uint64_t>);
+        const int rc = a.n < kVebPieceEqMin ? launch(veb_query_kernel<K, uint32_t, false>)
+                       : narrow             ? launch(veb_query_kernel<K, uint32_t, true>)
+                                            : launch(veb_query_kernel<K, uint64_t, true>);
         if (rc) return rc;
     }
     TL_CUDA_TRY(cudaGetLastError());
