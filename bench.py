@@ -101,9 +101,10 @@ def query_bytes_model(layout, n, b, kb):
 
 def query_grouped(layout, n, kb, q):
     """Whether the library groups a batch by value in device memory first: BST
-    batches of more than 2^22 queries over 1 GB (2^28 - 1 u32 keys) or more (csrc/query.cu's
-    launch_query)."""
-    return layout == "bst" and (1 << 22) < q < (1 << 32) and n * kb >= (1 << 30) - 1024
+    batches of more than 2^22 queries over 1 GB (2^28 - 1 u32 keys) or more, of 3 * 2^20
+    or more over 4 GB or more (csrc/query.cu's launch_query)."""
+    return layout == "bst" and q < (1 << 32) and (q > 1 << 22 and n * kb >= (1 << 30) - 1024
+                                                  or q >= 3 << 20 and n * kb >= (4 << 30) - 1024)
 
 
 def query_kernel_name(layout, b, kb, n, q):

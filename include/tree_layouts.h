@@ -200,7 +200,7 @@ int tl_query_sorted_u32(const uint32_t *dev_sorted, uint64_t n, const uint32_t *
 int tl_query_sorted_u64(const uint64_t *dev_sorted, uint64_t n, const uint64_t *dev_queries,
                         uint64_t q, uint64_t *dev_answers, void *stream, float *ms);
 /* BST queries: a batch of more than 2^22 queries over a layout of 1 GB or more
- * is first grouped by value, in stream-ordered temporary device memory of about
+ * (of 3 * 2^20 or more over 4 GB or more) is first grouped by value, in stream-ordered temporary device memory of about
  * q * (2 w + 8) bytes plus up to 16 MB (w the key width), so that queries close
  * in value share the deep nodes they fetch; the answers keep the batch's order.
  * If that memory cannot be had, the batch is searched as given.
@@ -404,7 +404,8 @@ int tl_debug_set_schedule(int mode);
  * B-tree one 32-byte load per lane of the group (b * w / 32 lanes); 8 the learned
  * query with 64-bit indices; 9 B-tree top levels in shared memory at any batch
  * size; 19 BST batches never grouped by value in device memory, 20 always (by
- * default only more than 2^22 queries over 1 GB or more); 30 / 31 batched queries
+ * default only more than 2^22 queries over 1 GB or more and 3 * 2^20 over 4 GB or
+ * more); 30 / 31 batched queries
  * always / never ordered by instance. */
 void tl_debug_set_query_variant(int v);
 /* Instances of a batched plan on the ordered-tile schedule and their keys: by

@@ -533,3 +533,21 @@ def test_small_layouts_and_the_largest_key(layout, dtype, last):
             Q[:5] = 0, top, top - 1, keys[0], keys[-1]
             Q[5:40] = top
             assert np.array_equal(gpu_answers(layout, tree, Q), O.search(layout, tree, Q)), (layout, n, q)
+
+
+def test_bst_grouping_line_over_4_gb():
+    """Either side of the batch size from which a 4 GB BST's queries are grouped."""
+    import torch
+    n = 2**30 - 1
+    keys = torch.arange(1, n + 1, device="cuda", dtype=torch.int32) * 2
+    tree = keys.clone()
+    T.permute("bst", tree)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    for q in ((3 << 20) - 1, 3 << 20):
+        Q = torch.randint(0, 2**31 - 1, (q,), generator=g, device="cuda", dtype=torch.int32)
+        ans = torch.full((q,), -7, dtype=torch.int64, device="cuda")
+        T.query("bst", tree, Q, ans)
+        hit = ans != n
+        assert torch.equal(hit, (Q % 2 == 0) & (Q > 0))
+        assert torch.equal(tree[ans[hit]], Q[hit])

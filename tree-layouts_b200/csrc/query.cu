@@ -1592,13 +1592,17 @@ static int launch_query(const QueryArgs &a, cudaStream_t st) {
     // queries 1129 / 1063, 2^27 9617 / 8487; 2^28 - 1 u32 (1 GB) 2^21 230 / 188, 2^22
     // 370 / 355, 2^23 650 / 702, 2^24 1196 / 1371; 2^30 - 1 u32 2^21 297 / 274, 2^22
     // 513 / 553, 2^24 1458 / 2455; u64 of 512 MB 2^24 1265 / 1136, of 2 GB 1442 / 2086.
+    // From 4 GB smaller batches gain too: 2^21 / 3 * 2^20 / 2^22 queries over 2^30 - 1 u32
+    // keys 280 / 386 / 481 grouped, 260 / 395 / 534 in chunks, over 2^30 - 1 u64 333 / 451 /
+    // 577 and 321 / 495 / 676; over 2 GB 239 / 324 / 398 and 214 / 309 / 413.
     // Measurement hooks: variant 19 never groups, 20 always.
     QueryPartition part;
     const uint32_t *perm = nullptr;
     const uint64_t tree_bytes = a.n * sizeof(K);
     const bool large = tree_bytes >= (1ull << 30) - 1024;  // 2^28 - 1 u32 keys included
+    const bool huge = tree_bytes >= (4ull << 30) - 1024;   // 2^30 - 1 u32 keys included
     if (a.layout == Q_BST && g_query_variant != 19 && a.q < (1ull << 32) &&
-        (g_query_variant == 20 || (a.q > (1ull << 22) && large))) {
+        (g_query_variant == 20 || (large && a.q > (1ull << 22)) || (huge && a.q >= (3ull << 20)))) {
         const int rc = partition_queries<K>(Q, a.q, st, part);
         if (rc == TL_SUCCESS) {
             Q = static_cast<const K *>(part.qs);
