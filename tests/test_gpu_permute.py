@@ -207,3 +207,23 @@ def test_btree_stream_ring_of_stages(layout, b, dtype, tiles):
     out = from_dev(buf)
     assert np.array_equal(out[1:1 + n], O.permute(layout, keys, b))
     assert out[0] == 0 and out[-1] == 0
+
+
+@pytest.mark.parametrize("layout,b", [("bst", 1), ("btree", 2), ("btree", 3), ("btree", 8), ("btree", 16), ("btree", 17),
+                                      ("btree", 32)])
+@pytest.mark.parametrize("dtype", [np.uint64, np.uint32])
+def test_edge_sizes_by_tiles(layout, b, dtype):
+    """The edge sizes through the tiled kernels, which arrays of up to 12 MB take
+    when the caller's workspace has no room for a copy of the array."""
+    import torch
+    kb = np.dtype(dtype).itemsize
+    ran = 0
+    for n in EDGE:
+        need = T.workspace_bytes(layout, n, b, kb)
+        if need >= n * kb:
+            continue
+        keys = data.sorted_keys_np(n, 1, 3, 7 + n, dtype)
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+        assert np.array_equal(run(layout, keys, b, workspace=ws), O.permute(layout, keys, b)), (layout, b, n)
+        ran += 1
+    assert ran > len(EDGE) // 2

@@ -145,3 +145,24 @@ def test_veb_forms_round_trip_at_their_line(layout, n, kb):
     T.unpermute(layout, t)
     assert torch.equal(t, keys)
     assert int(buf[0]) == -1 and bool((buf[n + 1:] == -1).all())
+
+
+@pytest.mark.parametrize("b", [1, 2, 3, 8, 16, 17, 32])
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("mb", [13, 200])
+def test_reverse_by_tiles_round_trip_at_tile_edges(b, kb, mb):
+    """B-trees and BSTs just above the sizes that go back key by key (12 MB) and
+    from a copy (192 MB), around whole tiles of 32 KB and off a line."""
+    import torch
+    tile = 32768 // kb
+    for tiles, extra in ((mb * 32, 0), (mb * 32, 1), (mb * 32 + 1, -1), (mb * 32 + 3, 1000)):
+        n = tiles * tile + extra
+        keys = data.sorted_keys_torch(n, 1, 3, 5, kb)
+        buf = torch.full((n + 3,), -1, dtype=keys.dtype, device="cuda")
+        t = buf[3:]
+        t.copy_(keys)
+        layout = "bst" if b == 1 else "btree"
+        T.permute(layout, t, b)
+        T.unpermute(layout, t, b)
+        assert torch.equal(t, keys), (b, kb, n)
+        assert bool((buf[:3] == -1).all())
