@@ -280,11 +280,20 @@ def workload_config(args, layout, b, n, kb, gap_hi, kseed, world):
 
 
 def run_reference(args, rank):
+    """The reference's own code, or a line saying why it cannot run: the oracle's
+    port is no stand-in for it here."""
     layout, b, n, kb, gap_hi, kseed, *_ = WORKLOADS[args.workload]
     if rank != 0:
         return
-    # the single-thread mvEB port runs on a bounded sample (about 2 s a run)
-    n_sample = min(n, args.ref_n) if args.ref_n else (n if layout != "mveb" else min(n, 2**28 - 1))
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle as O
+    why = ("the reference has no CPU code for this layout" if layout == "mveb" else
+           "the reference's CPU code is not built here (oracle/_ref/libref_cpu.so is made from its sources)"
+           if O.ref_cpu() is None else None)
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
+        return
+    n_sample = min(n, args.ref_n) if args.ref_n else n
     steps = []
     keys = sample_keys(n_sample, gap_hi, kseed)
     for _ in range(args.warmup):

@@ -25,3 +25,15 @@ def test_partial_last_level_counts_as_a_level():
     # 17^3 - 1 + 5 keys, b = 16: a perfect 3-level top tree and a last level of 5 keys
     nbytes, l2, levels = bench.query_bytes_model("btree", 17**3 - 1 + 5, 16, 8)
     assert levels == 4 and l2 == 4 and nbytes == 16
+
+
+def test_reference_arm_without_the_reference_prints_no_number(monkeypatch, capsys):
+    import argparse
+    import json
+
+    import oracle as O
+    monkeypatch.setattr(O, "ref_cpu", lambda: None)
+    for workload in ("btree-b16-n500M-u64", "bst-n2^20-1-u64", "mveb-n300M-u32"):
+        bench.run_reference(argparse.Namespace(workload=workload, ref_n=1000, warmup=1, steps=1, gpus=1), 0)
+        line = json.loads(capsys.readouterr().out)
+        assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
