@@ -84,8 +84,11 @@ int tl_permute_workspace_bytes(int layout, uint64_t n, uint64_t b, uint32_t key_
  * kept for the life of the process, each lent to one call at a time; when no
  * cached buffer can be had, a stream-ordered cudaMallocAsync that the call
  * frees before returning).
+ * B-trees and BSTs of up to 12 MB are moved key by key through a copy of the
+ * array, whose size the workspace then has; with a given workspace smaller than
+ * that they are moved by tiles, as larger arrays are.
  * Per-geometry tables: a B-tree or BST of 64 tiles or more (16384 for the BST)
- * takes the ordered-tile schedule, whose tables depend only on (n, b, tile
+ * that is moved by tiles takes the ordered-tile schedule, whose tables depend only on (n, b, tile
  * size).  The first call for a new geometry on a device builds them and copies
  * them into a cudaMalloc'd block that the library keeps for the life of the
  * process (at most 64 geometries, about 12 bytes per 32 KB tile plus the fix
@@ -161,8 +164,10 @@ int tl_permute_algorithm(int layout, int algorithm, void *dev_A, uint64_t n, uin
  * the layouts but implements only sorted -> layout.  Workspace, stream and ms
  * as for tl_permute.  tl_unpermute_workspace_bytes has room for a copy of the
  * array; with dev_workspace NULL the cached buffer is only as large as the
- * layout and size need (large arrays go back in place, through scratch for the
- * keys that took scratch on the way there). */
+ * layout and size need (vEB layouts over 56 MB, B-trees over 192 MB and BSTs of
+ * 16384 tiles or more go back in place, through scratch for the keys that took
+ * scratch on the way there; their first call for a new geometry builds the tables
+ * above if tl_permute has not). */
 int tl_unpermute_workspace_bytes(int layout, uint64_t n, uint64_t b, uint32_t key_bytes, uint64_t *bytes);
 int tl_unpermute(int layout, void *dev_A, uint64_t n, uint64_t b, uint32_t key_bytes, void *dev_workspace,
                  uint64_t workspace_bytes, void *stream, float *ms);
@@ -200,12 +205,15 @@ int tl_query_sorted_u32(const uint32_t *dev_sorted, uint64_t n, const uint32_t *
 int tl_query_sorted_u64(const uint64_t *dev_sorted, uint64_t n, const uint64_t *dev_queries,
                         uint64_t q, uint64_t *dev_answers, void *stream, float *ms);
 /* BST queries: a batch of more than 2^22 queries over a layout of 1 GB or more
- * (of 3 * 2^20 or more over 4 GB or more) is first grouped by value, in stream-ordered temporary device memory of about
- * q * (2 w + 8) bytes plus up to 16 MB (w the key width), so that queries close
- * in value share the deep nodes they fetch; the answers keep the batch's order.
- * If that memory cannot be had, the batch is searched as given.
+ * (of 3 * 2^20 or more over 4 GB or more) is first grouped by value, in
+ * stream-ordered temporary device memory of about q * (2 w + 8) bytes plus up to
+ * 16 MB (w the key width), so that queries close in value share the deep nodes
+ * they fetch; the answers keep the batch's order.  If that memory cannot be had,
+ * the batch is searched as smaller ones are.
  *
- * dev_answers[i] = position of dev_queries[i] in the layout, or n.
+ * dev_answers[i] = position of dev_queries[i] in the layout, or n; of equal keys
+ * the one that a search from the root meets first (of the sorted array, the
+ * first).  Over words that are no such layout the answers mean nothing.
  * searchAll (gpu/src/query-bst.cuh:47-54) behind timeQueryBST (:58-110). */
 int tl_query_bst_u32(const uint32_t *dev_layout, uint64_t n, const uint32_t *dev_queries,
                      uint64_t q, uint64_t *dev_answers, void *stream, float *ms);
@@ -267,9 +275,9 @@ int tl_batch_query(const tl_batch_plan *plan, const void *dev_keys, const void *
                    uint64_t workspace_bytes, void *stream, float *ms);
 /* Tuning per size class c = floor(log2 n_j), 48 entries each: keys per stream
  * tile (a power of two, 256 .. 96 KB / key_bytes); plus the permute block shape
- * (256: eight store warps, 512: four); 0 / NULL keeps a value.  pin_levels and query_chunk are kept and
- * read back, but the queries have nothing to tune.  Changing tile sizes rebuilds
- * the plan from dev_offsets. */
+ * (256: eight store warps, 512: four); 0 / NULL keeps a value.  pin_levels and
+ * query_chunk are kept and read back, but the queries have nothing to tune.
+ * Changing tile sizes rebuilds the plan from dev_offsets. */
 int tl_batch_set_tuning(tl_batch_plan *plan, const uint32_t *tile_keys, const uint32_t *pin_levels,
                         uint32_t query_chunk, uint32_t threads, const int64_t *dev_offsets, void *stream);
 int tl_batch_get_tuning(const tl_batch_plan *plan, uint32_t *tile_keys, uint32_t *pin_levels,
@@ -410,7 +418,8 @@ int tl_debug_set_schedule(int mode);
 void tl_debug_set_query_variant(int v);
 /* Instances of a batched plan on the ordered-tile schedule and their keys: by
  * default those of 64 tiles or more (at the plan's tile size for their size
- * class) whose scratch keys it cuts to 30 % or less. */
+ * class) whose scratch keys it cuts to 90 % or less, above 30 % only in no more
+ * scratch space. */
 int tl_debug_batch_ordered(const tl_batch_plan *plan, uint64_t *instances, uint64_t *keys);
 /* Of the last permutation's bounded waits: how many found their flag unset at
  * the first look, and how many polls those took in total. */
